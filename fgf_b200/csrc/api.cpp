@@ -87,10 +87,10 @@ struct fgfc_plan {
   std::vector<uint32_t> bits_mat, bits_scat, bits_gath;
   uint64_t bits_key = 0;  // hash of bits_mat
   int device;
-  uint32_t* dev;        // device tables, three orientations back to back
-  size_t mat_groups;    // groups per source in the matrix orientation
-  size_t off_mat, off_scat, off_gath;  // word offsets into `dev`
-  size_t scat_groups, gath_groups;
+  uint32_t* dev;        // device images and tables of the three orientations
+  size_t off_img[3];    // word offsets into `dev`: table images (matrix, scatter, gather)
+  size_t off_byte[3];   // compact tables for the byte-table kernel (SIZE_MAX: not its shape)
+  size_t mat_groups, off_mat;  // compact tables of the matrix orientation (batches)
   size_t off_k16 = 0, k16_groups = 0;  // Gf16: byte half-product tables of the matrix orientation (batches)
 };
 
@@ -99,9 +99,9 @@ namespace {
 // Coefficient source for a lowered matrix call: either raw host values
 // (term-major, k x m) or device tables of a plan.
 struct CoeffSrc {
-  const uint64_t* host = nullptr;  // term-major k x m
-  const uint32_t* dev = nullptr;   // compact tables [(t*E+p)*gstride + g][32]
-  size_t gstride = 0;
+  const uint64_t* host = nullptr;      // term-major k x m
+  const uint32_t* img = nullptr;       // table images (build_lut_images), launch by launch of rows
+  const uint32_t* byte_tab = nullptr;  // compact tables [source][32] where the byte-table kernel covers the shape
   const uint32_t* bits = nullptr;  // GF(2) bit matrix (plans), or built from `host` when needed
 };
 
@@ -160,6 +160,14 @@ bool run_gf2mma(int field, const uint8_t* const* srcs, size_t k, uint8_t* const*
   return true;
 }
 
+// Does any row share bytes with any source (an in-place call)?
+bool any_overlap(const uint8_t* const* srcs, size_t k, uint8_t* const* rows, size_t m, size_t len) {
+  for (size_t j = 0; j < m; ++j)
+    for (size_t t = 0; t < k; ++t)
+      if (rows[j] < srcs[t] + len && srcs[t] < rows[j] + len) return true;
+  return false;
+}
+
 fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t* const* rows,
                        size_t m, const CoeffSrc& cs, size_t len, bool overwrite,
                        cudaStream_t stream, const char* name, bool allow_mma) {
@@ -176,69 +184,67 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
     return ok();
   }
   const int E = field_bytes(field);
-  if (E == 8) {
-    cudaError_t e = wide_launch(field, srcs, k, rows, m, cs.host, cs.dev, cs.gstride, len, overwrite, stream);
-    return e == cudaSuccess ? ok() : cuda_fail(e, name);
-  }
-  const int R = 4 / E;
-  const size_t gtot = (m + R - 1) / R;
-  const bool inl = cs.dev == nullptr;
-  const size_t slot_cap = inl ? kInlineSlots : kMaxSlots;
-  size_t gp = std::min<size_t>(gtot, 4);
-  while (gp > 1 && static_cast<size_t>(E) * gp > slot_cap) --gp;
-  size_t kc = std::min<size_t>(k, slot_cap / (E * gp));
-  kc = std::min<size_t>(kc, kMaxSrc);
-  if (kc == 0) return fail(FGFC_ERR_LIMIT, "%s: internal tiling failed", name);
-
-  // Alignment class shared by every source; the kernels store rows at any
-  // offset (columns are spliced in registers when a row's offset differs).
-  uintptr_t al = reinterpret_cast<uintptr_t>(srcs[0]) & 15;
-  bool same = true;
+  // Alignment: every source and row at one offset within 16 bytes, with whole
+  // elements before the first 16-byte boundary, is an aligned job.
+  const uintptr_t al = reinterpret_cast<uintptr_t>(srcs[0]) & 15;
+  bool same = (al % E) == 0;
   for (size_t t = 0; t < k; ++t) same &= (reinterpret_cast<uintptr_t>(srcs[t]) & 15) == al;
-  same &= (al % E) == 0;
-  uint64_t head = len, nvec = 0;
-  bool shift = false;
-  if (same) {
-    head = std::min<uint64_t>((16 - al) & 15, len);
-    nvec = (len - head) / 16;
-    for (size_t j = 0; j < m; ++j) shift |= (reinterpret_cast<uintptr_t>(rows[j]) & 15) != al;
+  const uint64_t head = std::min<uint64_t>((16 - al) & 15, len);
+
+  static thread_local LutArgs a;  // large (inline images): keep off the stack
+  const bool byte_tables = same && len - head >= 16 && choose_kernel(field, k, m, len) == FGFC_KERNEL_BYTE;
+  if (byte_tables) {
+    static thread_local MatrixLaunch f;
+    f.head = head;
+    f.nvec = (len - head) / 16;
+    f.k = static_cast<uint32_t>(k);
+    f.nrows = static_cast<uint32_t>(m);
+    f.shift = 0;
+    for (size_t j = 0; j < m; ++j) f.shift |= (reinterpret_cast<uintptr_t>(rows[j]) & 15) != al;
+    for (size_t t = 0; t < k; ++t) f.src[t] = srcs[t];
+    for (size_t j = 0; j < m; ++j) f.dst[j] = rows[j];
+    f.tables = cs.byte_tab;
+    if (!f.tables) build_compact_tables(field, cs.host, m, 0, k, 0, 1, f.inline_tab);
+    std::lock_guard<std::mutex> lk(g_launch_mu);
+    cudaError_t e = launch_fast_matrix(overwrite, f, stream);
+    if (e != cudaSuccess) return cuda_fail(e, name);
+    if (!head && len % 16 == 0) return ok();
   }
 
-  const bool byte_tables = choose_kernel(field, k, m, len) == FGFC_KERNEL_BYTE;
-  static thread_local MatrixLaunch a;  // large (inline tables): keep off the stack
-  for (size_t g0 = 0; g0 < gtot; g0 += gp) {
-    const size_t G = std::min(gp, gtot - g0);
-    const size_t r0 = g0 * R;
-    const size_t nr = std::min(m - r0, G * R);
+  size_t img_off = 0;
+  for (size_t r0 = 0; r0 < m; r0 += lut_rows(E)) {
+    const size_t nr = std::min(lut_rows(E), m - r0);
+    const size_t kc = lut_sources(E, nr, cs.img == nullptr);
+    const size_t src_words = lut_shape(E, nr).src_words();
+    if (kc == 0) return fail(FGFC_ERR_LIMIT, "%s: internal tiling failed", name);
+    bool unal = !same;
+    for (size_t j = 0; j < nr; ++j) unal |= (reinterpret_cast<uintptr_t>(rows[r0 + j]) & 15) != al;
+    unal &= !byte_tables;  // the byte-table kernel left a head and a tail
+    a.g.len = len;
+    a.g.head = unal ? 0 : head;
+    a.g.ncol = (len - a.g.head) / 16;
+    a.g.bytes = unal && any_overlap(srcs, k, rows + r0, nr, len) ? 1u : 0u;
+    a.g.nrows = static_cast<uint32_t>(nr);
+    for (size_t j = 0; j < nr; ++j) a.dst[j] = rows[r0 + j];
     for (size_t t0 = 0; t0 < k; t0 += kc) {
       const size_t kk = std::min(kc, k - t0);
-      a.len = len;
-      a.head = head;
-      a.nvec = nvec;
-      a.shift = 0;
-      for (size_t j = 0; j < nr; ++j) a.shift |= (reinterpret_cast<uintptr_t>(rows[r0 + j]) & 15) != al;
-      a.shift &= shift ? 1u : 0u;
-      a.k = static_cast<uint32_t>(kk);
-      a.nrows = static_cast<uint32_t>(nr);
+      a.g.k = static_cast<uint32_t>(kk);
+      a.g.ovr = overwrite && t0 == 0 ? 1u : 0u;
       for (size_t t = 0; t < kk; ++t) a.src[t] = srcs[t0 + t];
-      for (size_t j = 0; j < nr; ++j) a.dst[j] = rows[r0 + j];
-      if (inl) {
-        build_compact_tables(field, cs.host, m, t0, kk, g0, G, a.inline_tab);
-        a.tables = nullptr;
-        a.gstride = static_cast<uint32_t>(G);
-        a.g0 = 0;
+      if (cs.img) {
+        a.img = cs.img + img_off + t0 * src_words;
       } else {
-        a.tables = cs.dev + t0 * E * cs.gstride * kCompactWords;
-        a.gstride = static_cast<uint32_t>(cs.gstride);
-        a.g0 = static_cast<uint32_t>(g0);
+        a.img = nullptr;
+        build_lut_images(field, cs.host, m, t0, kk, r0, nr, a.inl);
       }
       cudaError_t e;
       {
         std::lock_guard<std::mutex> lk(g_launch_mu);
-        e = launch_matrix(field, static_cast<int>(G), overwrite && t0 == 0, a, stream, byte_tables);
+        e = lut_launch(field, nr, a, unal, byte_tables, stream);
       }
       if (e != cudaSuccess) return cuda_fail(e, name);
     }
+    img_off += k * src_words;
   }
   return ok();
 }
@@ -252,40 +258,42 @@ bool all_zero(const uint64_t* c, size_t n, uint64_t mask) {
 fgfc_status upload_plan_tables(fgfc_plan* p) {
   const int E = field_bytes(p->field);
   const size_t len = p->values.size();
-  // 4-byte output groups covering n rows of E-byte elements
-  // Per source: E input bytes x (groups) slots of compact tables; the
-  // 8-byte fields keep their half-product tables instead (build_wide_tables:
-  // 12 slots per source and row, "groups" counting rows).
-  const bool wide = E == 8;
-  const auto groups = [E, wide](size_t n) { return wide ? n : (n * E + 3) / 4; };
-  const size_t slots_per_src = wide ? kWideSlotsPerSrcRow : static_cast<size_t>(E);
-  const auto build = [&](const uint64_t* c, size_t m, size_t k, size_t G, uint32_t* out) {
-    if (wide)
-      build_wide_tables(p->field, c, m, 0, k, 0, G, out);
-    else
-      build_compact_tables(p->field, c, m, 0, k, 0, G, out);
+  std::vector<uint32_t> host;
+  // images of k sources x m rows of c, launch by launch; 16-byte aligned
+  const auto add_images = [&](size_t k, size_t m) {
+    const size_t at = (host.size() + 3) / 4 * 4;
+    host.resize(at + lut_image_words(E, k, m));
+    size_t off = at;
+    for (size_t r0 = 0; r0 < m; r0 += lut_rows(E)) {
+      const size_t nr = std::min(lut_rows(E), m - r0);
+      build_lut_images(p->field, p->values.data(), m, 0, k, r0, nr, host.data() + off);
+      off += k * lut_shape(E, nr).src_words();
+    }
+    return at;
   };
-  // matrix orientation: rows = sources, cols = destination rows
-  p->mat_groups = groups(p->cols);
-  const size_t n_mat = p->rows * slots_per_src * p->mat_groups * kCompactWords;
-  p->scat_groups = groups(len);
-  const size_t n_scat = slots_per_src * p->scat_groups * kCompactWords;
-  p->gath_groups = groups(1);
-  const size_t n_gath = len * slots_per_src * p->gath_groups * kCompactWords;
-  // Gf16 batches also run the matrix orientation by byte half-products
+  const auto add_compact = [&](size_t k, size_t m, size_t G) {
+    const size_t at = (host.size() + 3) / 4 * 4;
+    host.resize(at + k * E * G * kCompactWords);
+    build_compact_tables(p->field, p->values.data(), m, 0, k, 0, G, host.data() + at);
+    return at;
+  };
+  // matrix orientation: rows = sources, cols = destination rows; scatter: one
+  // source, each coefficient a row; gather: source i has the single
+  // coefficient values[i]
+  const size_t shape[3][2] = {{p->rows, p->cols}, {1, len}, {len, 1}};
+  for (int o = 0; o < 3; ++o) {
+    const size_t k = shape[o][0], m = shape[o][1];
+    p->off_img[o] = add_images(k, m);
+    p->off_byte[o] = kernel_usable(FGFC_KERNEL_BYTE, p->field, k, m) ? add_compact(k, m, 1) : SIZE_MAX;
+  }
+  // batched work lists
+  p->mat_groups = E == 8 ? 0 : (p->cols * E + 3) / 4;
+  p->off_mat = E == 8 ? 0 : add_compact(p->rows, p->cols, p->mat_groups);
   p->k16_groups = E == 2 ? (p->cols + 3) / 4 : 0;
-  const size_t n_k16 = p->rows * 3 * p->k16_groups * kCompactWords;
-  std::vector<uint32_t> host(n_mat + n_scat + n_gath + n_k16 + 1, 0);
-  p->off_mat = 0;
-  p->off_scat = n_mat;
-  p->off_gath = n_mat + n_scat;
-  p->off_k16 = n_mat + n_scat + n_gath;
-  if (n_k16) build_kara16_tables(p->values.data(), p->cols, p->rows, p->k16_groups, host.data() + p->off_k16);
-  if (n_mat) build(p->values.data(), p->cols, p->rows, p->mat_groups, host.data() + p->off_mat);
-  if (n_scat) build(p->values.data(), len, 1, p->scat_groups, host.data() + p->off_scat);
-  // gather orientation: source i has the single coefficient values[i]
-  if (n_gath) build(p->values.data(), 1, len, p->gath_groups, host.data() + p->off_gath);
-  if (n_mat && gf2mma_shape_ok(p->field, p->rows, p->cols)) {
+  p->off_k16 = host.size();
+  host.resize(host.size() + p->rows * 3 * p->k16_groups * kCompactWords);
+  if (p->k16_groups) build_kara16_tables(p->values.data(), p->cols, p->rows, p->k16_groups, host.data() + p->off_k16);
+  if (p->rows && p->cols && gf2mma_shape_ok(p->field, p->rows, p->cols)) {
     p->bits_mat.resize(kGf2BitWords);
     gf2mma_bits(p->field, p->values.data(), p->rows, p->cols, p->bits_mat.data());
     uint64_t h = 1469598103934665603ull ^ (static_cast<uint64_t>(p->field) << 56);
@@ -302,7 +310,7 @@ fgfc_status upload_plan_tables(fgfc_plan* p) {
   }
   cudaError_t e = cudaGetDevice(&p->device);
   if (e != cudaSuccess) return cuda_fail(e, "Plan::matrix");
-  e = cudaMalloc(&p->dev, host.size() * sizeof(uint32_t));
+  e = cudaMalloc(&p->dev, (host.size() + 1) * sizeof(uint32_t));
   if (e != cudaSuccess) return fail(FGFC_ERR_NOMEM, "Plan::matrix: device allocation failed: %s",
                                     cudaGetErrorString(e));
   e = cudaMemcpy(p->dev, host.data(), host.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
@@ -310,27 +318,16 @@ fgfc_status upload_plan_tables(fgfc_plan* p) {
   return ok();
 }
 
-CoeffSrc plan_mat(const fgfc_plan* p) {
+CoeffSrc plan_src(const fgfc_plan* p, int o, const std::vector<uint32_t>& bits) {
   CoeffSrc c;
-  c.dev = p->dev + p->off_mat;
-  c.gstride = p->mat_groups;
-  c.bits = p->bits_mat.empty() ? nullptr : p->bits_mat.data();
+  c.img = p->dev + p->off_img[o];
+  c.byte_tab = p->off_byte[o] == SIZE_MAX ? nullptr : p->dev + p->off_byte[o];
+  c.bits = bits.empty() ? nullptr : bits.data();
   return c;
 }
-CoeffSrc plan_scat(const fgfc_plan* p) {
-  CoeffSrc c;
-  c.dev = p->dev + p->off_scat;
-  c.gstride = p->scat_groups;
-  c.bits = p->bits_scat.empty() ? nullptr : p->bits_scat.data();
-  return c;
-}
-CoeffSrc plan_gath(const fgfc_plan* p) {
-  CoeffSrc c;
-  c.dev = p->dev + p->off_gath;
-  c.gstride = p->gath_groups;
-  c.bits = p->bits_gath.empty() ? nullptr : p->bits_gath.data();
-  return c;
-}
+CoeffSrc plan_mat(const fgfc_plan* p) { return plan_src(p, 0, p->bits_mat); }
+CoeffSrc plan_scat(const fgfc_plan* p) { return plan_src(p, 1, p->bits_scat); }
+CoeffSrc plan_gath(const fgfc_plan* p) { return plan_src(p, 2, p->bits_gath); }
 
 }  // namespace
 

@@ -16,14 +16,13 @@ namespace fgfc {
 // into several launches by the host (exact: rows are independent, and
 // sources split into an overwrite launch followed by accumulate launches).
 constexpr int kMaxSrc = 64;
-constexpr int kMaxRows = 64;
 // One nibble table slot: 16 rows x 256 bytes. Each row holds 32 lane copies
 // of the lo-nibble word (bytes 0..127) and of the hi-nibble word (128..255),
 // so a warp's 32 lookups hit 32 distinct banks.
 constexpr int kSlotBytes = 4096;
 constexpr int kMaxSlots = 54;            // 216 KiB of tables (+ 6.75 KiB staging) per CTA
-constexpr int kInlineSlots = 48;         // tables carried in launch parameters
 constexpr int kCompactWords = 32;        // 16 lo + 16 hi words per slot
+constexpr size_t kFastMaxSources = 14;   // byte-table kernels: sources per launch
 
 // A compact table slot for (source t, source byte-plane p, row group g):
 // word[n] (n < 16) = products of the lo nibble value n, word[16 + n] =
@@ -31,18 +30,15 @@ constexpr int kCompactWords = 32;        // 16 lo + 16 hi words per slot
 // (g * R + q / E), R = 4 / E rows per group.
 
 struct MatrixLaunch {
-  uint64_t len;            // bytes per row processed by this launch
-  uint64_t head;           // bytes handled by the scalar path before the vector body
+  uint64_t head;           // bytes before the vector body
   uint64_t nvec;           // 16-byte vectors in the body
   uint32_t k;              // sources
-  uint32_t nrows;          // rows written by this launch (<= groups * R)
-  uint32_t gstride;        // groups per (source, plane) in the compact table array
-  uint32_t g0;             // first group of this launch within that array
+  uint32_t nrows;          // rows written by this launch (<= 4)
   uint32_t shift;          // 1: some row is not at the sources' offset within 16 bytes
   const uint32_t* tables;  // device compact tables, or nullptr for `inline_tab`
-  const uint8_t* src[kMaxSrc];
-  uint8_t* dst[kMaxRows];
-  uint32_t inline_tab[kInlineSlots * kCompactWords];
+  const uint8_t* src[kFastMaxSources];
+  uint8_t* dst[4];
+  uint32_t inline_tab[kFastMaxSources * kCompactWords];
 };
 
 // Build compact tables for sources [t0, t0+k) and groups [g0, g0+G) of a
@@ -51,32 +47,68 @@ struct MatrixLaunch {
 void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k,
                           size_t g0, size_t G, uint32_t* out);
 
-// The 8-byte fields multiply a constant c = c0 + c1 w by x = x0 + x1 w
-// (halves over the 4-byte base field: Gf32 for GF(2^64), FP32 for Fan-Paar
-// GF(2^64)) as three half-products A = c0 x0, B = c1 x1, C = (c0 + c1)(x0 + x1)
-// and a fix-up of the sums (Karatsuba): GF(2^64) gives lo = A + beta B,
-// hi = A + C; Fan-Paar gives lo = A + B, hi = A + C + (1 + alpha) B. Tables
-// for sources [t0, t0+k) and rows [j0, j0+M), layout
-// [((t * 3 + P) * 4 + p) * M + j][32]: product P (A, B, C), input byte p of
-// the 4-byte half, 16 words for its low nibble and 16 for its high nibble.
-constexpr size_t kWideSlotsPerSrcRow = 12;
 // The same split for Gf16 = Gf8B[u]/(u^2 + u + 0x20): lo = A + 0x20 B,
 // hi = A + C over byte half-products. Tables for the batched work lists:
 // [(t * 3 + P) * Gq + q][32], nibble tables whose word holds the byte
 // half-product P of rows 4q .. 4q + 3 (zero past m); Gq = ceil(m / 4).
 void build_kara16_tables(const uint64_t* coeffs, size_t m, size_t k, size_t Gq, uint32_t* out);
-void build_wide_tables(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t j0, size_t M,
-                       uint32_t* out);
-// The fix-up map of an 8-byte field as [4 input bytes][32] nibble tables:
-// v -> beta v (GF(2^64)) or v -> (1 + alpha) v (Fan-Paar GF(2^64)).
-void build_wide_fixup(int field, uint32_t* out /* [128] */);
 
-// Kernel entry (kernels.cu). `groups` = G for this launch; `overwrite`
-// selects dot-product (overwrite) or mul_add (accumulate) semantics.
-// `byte_tables`: run the byte-table kernel (Gf8, one group, <= 14 sources)
-// for the vector body instead of the split-nibble kernel.
-cudaError_t launch_matrix(int field, int groups, bool overwrite, const MatrixLaunch& a,
-                          cudaStream_t s, bool byte_tables);
+// ---------------------------------------------------------------- table kernels (lut.cuh)
+
+// One job's geometry. Columns are 16 bytes, column v at head + 16 v. Aligned
+// jobs (every source and row at one offset within 16 bytes, whole elements
+// before the first aligned column) have `head` bytes, then `ncol` whole
+// columns. Unaligned jobs have head = 0 and columns from the row's start.
+// Bytes outside the columns that the vector path covers are "edges".
+struct LutGeom {
+  uint64_t len, head, ncol;
+  uint32_t k, nrows;
+  uint32_t ovr;    // 1 = overwrite
+  uint32_t bytes;  // unaligned in-place job: columns are read and written bytewise
+};
+
+constexpr int kLutRows = 16;               // rows per launch (Gf8; 8 / 4 / 4 for 2, 4 and 8 bytes)
+constexpr int kLutInlineWords = 1536;      // images carried in launch parameters
+constexpr int kLutSmemMax = 110 * 1024;    // tables of one CTA: two CTAs per SM
+struct LutArgs {
+  const uint32_t* img;  // device images, or nullptr: inl
+  LutGeom g;
+  uint32_t fp;          // Fan-Paar fix-ups
+  uint32_t edge_cta;    // 1: the last CTA takes the edges
+  uint64_t ntiles;
+  const uint8_t* src[kMaxSrc];
+  uint8_t* dst[kLutRows];
+  alignas(16) uint32_t inl[kLutInlineWords];
+};
+
+// Tower levels split and output words per leaf product of a launch of nr rows.
+struct LutShape {
+  int lev, w;
+  size_t nv;  // leaf input bytes per element
+  size_t src_words() const { return nv * static_cast<size_t>(w) * 8; }  // image words per source
+  size_t smem3() const { return (nv * w * 640 + 255) / 256 * 256; }     // table bytes of three sources
+};
+inline size_t lut_rows(int E) { return E == 1 ? 16 : E == 2 ? 8 : 4; }
+LutShape lut_shape(int E, size_t nr);
+// Sources per launch: table pages, pointers and (raw forms) inline images fit.
+size_t lut_sources(int E, size_t nr, bool inl);
+// Image words of k sources and m rows, launch by launch of lut_rows(E) rows.
+size_t lut_image_words(int E, size_t k, size_t m);
+// Images of sources [t0, t0 + k) and rows [r0, r0 + nr) of a term-major
+// coefficient matrix with m columns: [source][leaf byte][word][8].
+void build_lut_images(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t r0, size_t nr,
+                      uint32_t* out);
+// Launch one job (rows of one lut_shape); `unal` as LutGeom describes.
+cudaError_t lut_launch(int field, size_t nr, LutArgs& a, bool unal, bool edges_only, cudaStream_t s);
+cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
+cudaError_t lut_launch_e2(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
+cudaError_t lut_launch_e4(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
+cudaError_t lut_launch_e8(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
+
+// The byte-table kernel (kernels.cu; Gf8, at most 4 rows, <= 14 sources) over
+// the vector body of a call; `overwrite` selects dot-product (overwrite) or
+// mul_add (accumulate) semantics.
+cudaError_t launch_fast_matrix(bool overwrite, const MatrixLaunch& a, cudaStream_t s);
 // Fill `n` rows of `len` bytes with zero.
 cudaError_t launch_zero_rows(uint8_t* const* rows, int n, uint64_t len, cudaStream_t s);
 // dst ^= src over `len` bytes.
@@ -88,7 +120,6 @@ cudaError_t launch_elementwise(int field, uint8_t* dst, const uint8_t* a, const 
 int sm_count();
 
 // Kernel families (fgfc_kernel values) and the choice per shape (tune.cpp).
-constexpr size_t kFastMaxSources = 14;  // byte-table kernels: sources per launch
 bool kernel_usable(int kernel, int field, size_t k, size_t m);
 int choose_kernel(int field, size_t k, size_t m, size_t len);
 // Tile shape of the batched nibble work lists (tune.cpp): element-vector
@@ -165,17 +196,6 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
 // shares one offset within 16 bytes) plus table sub-jobs for the rest.
 void lower_matrix_job(const fgfc_plan* plan, const std::vector<uint64_t>& srcs, const std::vector<uint64_t>& dsts,
                       size_t row_len, bool overwrite, std::vector<LoweredJob>& out, std::vector<Gf2Job>& tc);
-
-// The matrix ops for 8-byte fields (wide.cu): coefficients either as raw
-// host values (term-major k x m, tables built into the launch parameters) or
-// as a plan's device tables in the compact layout with `gstride` groups per
-// (source, byte plane).
-// Matrix ops of the 8-byte fields (wide.cu): dev_tables in the
-// build_wide_tables layout with `gstride` rows, or nullptr (tables built
-// per launch from host_coeffs).
-cudaError_t wide_launch(int field, const uint8_t* const* srcs, size_t k, uint8_t* const* rows, size_t m,
-                        const uint64_t* host_coeffs, const uint32_t* dev_tables, size_t gstride, size_t len,
-                        bool overwrite, cudaStream_t stream);
 
 // Error text of the calling thread (api.cpp), for entry points defined in
 // other files.

@@ -1,0 +1,13 @@
+// lut_e2.cu -- the table kernels (lut.cuh) of the 2-byte fields.
+#include "lut_single.cuh"
+
+namespace fgfc {
+
+cudaError_t lut_launch_e2(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only) {
+  if (lev == 0 && w == 1) return lut_launch_lw<2, 0, 1>(a, s, unal, edges_only);
+  if (lev == 1 && w == 1) return lut_launch_lw<2, 1, 1>(a, s, unal, edges_only);
+  if (lev == 1 && w == 2) return lut_launch_lw<2, 1, 2>(a, s, unal, edges_only);
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace fgfc

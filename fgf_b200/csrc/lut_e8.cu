@@ -1,0 +1,13 @@
+// lut_e8.cu -- the table kernels (lut.cuh) of the 8-byte fields.
+#include "lut_single.cuh"
+
+namespace fgfc {
+
+cudaError_t lut_launch_e8(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only) {
+  if (lev == 1 && w == 1) return lut_launch_lw<8, 1, 1>(a, s, unal, edges_only);
+  if (lev == 2 && w == 1) return lut_launch_lw<8, 2, 1>(a, s, unal, edges_only);
+  if (lev == 3 && w == 1) return lut_launch_lw<8, 3, 1>(a, s, unal, edges_only);
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace fgfc

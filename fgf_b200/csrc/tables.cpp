@@ -1,4 +1,5 @@
-// tables.cpp -- host derivation of the compact nibble tables a launch uploads.
+// tables.cpp -- host derivation of the product tables and images a launch uploads.
+#include <algorithm>
 #include <cstring>
 
 #include "internal.hpp"
@@ -56,53 +57,101 @@ void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t t0
   }
 }
 
-namespace {
-
-// c * x over the 4-byte base field of an 8-byte field.
-uint32_t wide_half_mul(int field, uint32_t c, uint32_t x) {
-  return field == kGf64 ? gf32_mul(c, x) : static_cast<uint32_t>(fp_mul(c, x, 32));
+// Tower levels split per launch. A leaf product's table word holds the H-byte
+// products of 4 / H rows, and an element takes 8 H / 5 lookups per leaf product
+// and word, so (lookups per element, source and word set, in input bytes):
+//   2 bytes: direct 2 per 2 rows, halves 3 per 4 rows;
+//   4 bytes: direct 4 per row, 16-bit leaves 6 per 2 rows, byte leaves 9 per 4;
+//   8 bytes: 32-bit leaves 12 per row, 16-bit 18 per 2 rows, byte leaves 27 per 4.
+LutShape lut_shape(int E, size_t nr) {
+  LutShape s{};
+  if (E == 1) {
+    s.w = static_cast<int>((nr + 3) / 4);
+  } else if (E == 2) {
+    s.lev = nr > 2 ? 1 : 0;
+    s.w = nr > 4 ? 2 : 1;
+  } else if (E == 4) {
+    s.lev = nr > 2 ? 2 : nr > 1 ? 1 : 0;
+    s.w = 1;
+  } else {
+    s.lev = nr > 2 ? 3 : nr > 1 ? 2 : 1;
+    s.w = 1;
+  }
+  s.nv = static_cast<size_t>(E >> s.lev);
+  for (int i = 0; i < s.lev; ++i) s.nv *= 3;
+  return s;
 }
 
-// Nibble tables of a GF(2)-linear map on 32-bit words, given the images of
-// its 32 input bits: table p (input byte p) at out + p * 32.
-void linear_tables(const uint32_t img[32], uint32_t* out, size_t stride_slots) {
-  for (int p = 0; p < 4; ++p) {
-    uint32_t* slot = out + p * stride_slots * kCompactWords;
-    for (int half = 0; half < 2; ++half)
-      for (int n = 0; n < 16; ++n) {
-        uint32_t v = 0;
-        for (int b = 0; b < 4; ++b)
-          if ((n >> b) & 1) v ^= img[8 * p + 4 * half + b];
-        slot[half * 16 + n] = v;
-      }
-  }
+size_t lut_sources(int E, size_t nr, bool inl) {
+  const LutShape s = lut_shape(E, nr);
+  const size_t edge = 5 * 16;  // staged edge columns per source
+  size_t kc = std::min<size_t>(kMaxSrc, kLutSmemMax / (s.smem3() + 3 * edge) * 3);
+  if (inl) kc = std::min<size_t>(kc, kLutInlineWords / s.src_words());
+  return kc;
+}
+
+size_t lut_image_words(int E, size_t k, size_t m) {
+  size_t n = 0;
+  for (size_t r0 = 0; r0 < m; r0 += lut_rows(E)) n += k * lut_shape(E, std::min(lut_rows(E), m - r0)).src_words();
+  return n;
+}
+
+namespace {
+
+// The field one level's leaves live in: `field`'s subfield of H bytes.
+int leaf_field(int field, int H) {
+  if (field == kFp8 || field == kFp16 || field == kFp32 || field == kFp64)
+    return H == 1 ? kFp8 : H == 2 ? kFp16 : H == 4 ? kFp32 : kFp64;
+  if (field == kGf8D) return kGf8D;
+  return H == 1 ? kGf8B : H == 2 ? kGf16 : H == 4 ? kGf32 : kGf64;
 }
 
 }  // namespace
 
-void build_wide_tables(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t j0, size_t M,
-                       uint32_t* out) {
-  for (size_t tt = 0; tt < k; ++tt)
-    for (size_t j = 0; j < M; ++j) {
-      const uint64_t c = coeffs[(t0 + tt) * m + j0 + j];
-      const uint32_t c0 = static_cast<uint32_t>(c), c1 = static_cast<uint32_t>(c >> 32);
-      const uint32_t cp[3] = {c0, c1, c0 ^ c1};
-      for (int P = 0; P < 3; ++P) {
-        uint32_t img[32];
-        for (int i = 0; i < 32; ++i) img[i] = wide_half_mul(field, cp[P], 1u << i);
-        // slot of (tt, P, p = 0, j); input byte p is M slots further on
-        linear_tables(img, out + ((tt * 3 + P) * 4 * M + j) * kCompactWords, M);
+void build_lut_images(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t r0, size_t nr,
+                      uint32_t* out) {
+  const int E = field_bytes(field);
+  const LutShape s = lut_shape(E, nr);
+  const int H = E >> s.lev, leaf = leaf_field(field, H);
+  const size_t W = static_cast<size_t>(s.w);
+  std::memset(out, 0, k * s.src_words() * sizeof(uint32_t));
+  for (size_t t = 0; t < k; ++t)
+    for (size_t r = 0; r < nr; ++r) {
+      uint64_t c[27] = {coeffs[(t0 + t) * m + r0 + r] & field_mask(field)};
+      size_t n = 1;
+      for (int w = E / 2; w >= H; w /= 2) {  // split every product: low half, high half, their sum
+        for (size_t i = n; i-- > 0;) {
+          const uint64_t v = c[i], lo = v & ((1ull << (8 * w)) - 1), hi = v >> (8 * w);
+          c[3 * i] = lo;
+          c[3 * i + 1] = hi;
+          c[3 * i + 2] = lo ^ hi;
+        }
+        n *= 3;
       }
+      for (size_t P = 0; P < n; ++P)
+        for (int p = 0; p < H; ++p)
+          for (int b = 0; b < 8; ++b) {
+            const uint64_t v = gf_mul(leaf, c[P], 1ull << (8 * p + b));
+            for (int o = 0; o < H; ++o) {
+              const size_t f = r * H + o;  // output byte: word f / 4
+              out[((t * s.nv + P * H + p) * W + f / 4) * 8 + b] |= static_cast<uint32_t>((v >> (8 * o)) & 0xFF)
+                                                                  << (8 * (f % 4));
+            }
+          }
     }
 }
 
-void build_wide_fixup(int field, uint32_t* out) {
-  uint32_t img[32];
-  for (int i = 0; i < 32; ++i) {
-    const uint32_t v = 1u << i;
-    img[i] = field == kGf64 ? gf32_mul(0x20000000u, v) : v ^ static_cast<uint32_t>(fp_mul_alpha(v, 32));
+cudaError_t lut_launch(int field, size_t nr, LutArgs& a, bool unal, bool edges_only, cudaStream_t s) {
+  const int E = field_bytes(field);
+  const LutShape sh = lut_shape(E, nr);
+  a.fp = field == kFp16 || field == kFp32 || field == kFp64 ? 1u : 0u;
+  switch (E) {
+    case 1: return lut_launch_e1(sh.lev, sh.w, a, s, unal, edges_only);
+    case 2: return lut_launch_e2(sh.lev, sh.w, a, s, unal, edges_only);
+    case 4: return lut_launch_e4(sh.lev, sh.w, a, s, unal, edges_only);
+    case 8: return lut_launch_e8(sh.lev, sh.w, a, s, unal, edges_only);
+    default: return cudaErrorInvalidValue;
   }
-  linear_tables(img, out, 1);
 }
 
 void build_kara16_tables(const uint64_t* coeffs, size_t m, size_t k, size_t Gq, uint32_t* out) {
