@@ -90,8 +90,6 @@ struct fgfc_plan {
   uint32_t* dev;        // device images and tables of the three orientations
   size_t off_img[3];    // word offsets into `dev`: table images (matrix, scatter, gather)
   size_t off_byte[3];   // compact tables for the byte-table kernel (SIZE_MAX: not its shape)
-  size_t mat_groups, off_mat;  // compact tables of the matrix orientation (batches)
-  size_t off_k16 = 0, k16_groups = 0;  // Gf16: byte half-product tables of the matrix orientation (batches)
 };
 
 namespace {
@@ -204,7 +202,7 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
     for (size_t t = 0; t < k; ++t) f.src[t] = srcs[t];
     for (size_t j = 0; j < m; ++j) f.dst[j] = rows[j];
     f.tables = cs.byte_tab;
-    if (!f.tables) build_compact_tables(field, cs.host, m, 0, k, 0, 1, f.inline_tab);
+    if (!f.tables) build_compact_tables(field, cs.host, m, k, f.inline_tab);
     std::lock_guard<std::mutex> lk(g_launch_mu);
     cudaError_t e = launch_fast_matrix(overwrite, f, stream);
     if (e != cudaSuccess) return cuda_fail(e, name);
@@ -271,10 +269,10 @@ fgfc_status upload_plan_tables(fgfc_plan* p) {
     }
     return at;
   };
-  const auto add_compact = [&](size_t k, size_t m, size_t G) {
+  const auto add_compact = [&](size_t k, size_t m) {
     const size_t at = (host.size() + 3) / 4 * 4;
-    host.resize(at + k * E * G * kCompactWords);
-    build_compact_tables(p->field, p->values.data(), m, 0, k, 0, G, host.data() + at);
+    host.resize(at + k * kCompactWords);
+    build_compact_tables(p->field, p->values.data(), m, k, host.data() + at);
     return at;
   };
   // matrix orientation: rows = sources, cols = destination rows; scatter: one
@@ -284,15 +282,8 @@ fgfc_status upload_plan_tables(fgfc_plan* p) {
   for (int o = 0; o < 3; ++o) {
     const size_t k = shape[o][0], m = shape[o][1];
     p->off_img[o] = add_images(k, m);
-    p->off_byte[o] = kernel_usable(FGFC_KERNEL_BYTE, p->field, k, m) ? add_compact(k, m, 1) : SIZE_MAX;
+    p->off_byte[o] = kernel_usable(FGFC_KERNEL_BYTE, p->field, k, m) ? add_compact(k, m) : SIZE_MAX;
   }
-  // batched work lists
-  p->mat_groups = E == 8 ? 0 : (p->cols * E + 3) / 4;
-  p->off_mat = E == 8 ? 0 : add_compact(p->rows, p->cols, p->mat_groups);
-  p->k16_groups = E == 2 ? (p->cols + 3) / 4 : 0;
-  p->off_k16 = host.size();
-  host.resize(host.size() + p->rows * 3 * p->k16_groups * kCompactWords);
-  if (p->k16_groups) build_kara16_tables(p->values.data(), p->cols, p->rows, p->k16_groups, host.data() + p->off_k16);
   if (p->rows && p->cols && gf2mma_shape_ok(p->field, p->rows, p->cols)) {
     p->bits_mat.resize(kGf2BitWords);
     gf2mma_bits(p->field, p->values.data(), p->rows, p->cols, p->bits_mat.data());
@@ -957,75 +948,26 @@ namespace fgfc {
 namespace {
 
 // One stripe (all sources of a plan, rows at the given device addresses) as
-// table sub-jobs of at most 4 groups. The vector body is used when every
-// source has the same offset within 16 bytes (a multiple of the element
-// size), whatever the rows' offsets; otherwise the whole stripe takes the
-// 4-byte-group path.
+// table sub-jobs, one per launch's worth of rows.
 void lower_tables(const fgfc_plan* plan, const std::vector<uint64_t>& srcs, const std::vector<uint64_t>& dsts,
                   size_t row_len, bool overwrite, std::vector<LoweredJob>& out) {
-  const int field = plan->field;
-  const int E = field_bytes(field);
-  const int R = 4 / E;
-  const size_t nrows = dsts.size();
-  const uintptr_t al = srcs.empty() ? 0 : (srcs[0] & 15);
-  bool same = (al % E) == 0;
-  for (uint64_t p : srcs) same = same && (p & 15) == al;
-  uint64_t head = row_len, nvec = 0;
-  if (same) {
-    head = std::min<uint64_t>((16 - al) & 15, row_len);
-    nvec = (row_len - head) / 16;
-  }
-  const size_t gtot = (nrows + R - 1) / R;
-  for (size_t g0 = 0; g0 < gtot; g0 += 4) {
-    const size_t nr = std::min<size_t>(nrows - g0 * R, 4 * R);
-    // FGFC_GF16_HALF=0 in the environment (read once) keeps every Gf16
-    // sub-job on the Gf16 tables, for A/B runs
-    static const bool half_on = [] {
-      const char* v = std::getenv("FGFC_GF16_HALF");
-      return !(v && v[0] == '0');
-    }();
-    if (half_on && E == 2 && plan->k16_groups && (nr % 4 == 0 || nr % 4 == 3)) {
-      // 3, 4, 7 or 8 rows: byte half-products take 6 lookups per element and
-      // 4 rows where the Gf16 tables take 8 (1 or 2 rows: more; 5 or 6: the same)
-      LoweredJob L;
-      L.field = field;
-      L.kara = true;
-      L.tables = plan->dev + plan->off_k16;
-      L.gstride = plan->k16_groups;
-      L.g0 = g0 * R / 4;
-      L.G = (nr + 3) / 4;
-      L.len = row_len;
-      L.head = head;
-      L.nvec = nvec;
-      L.k = srcs.size();
-      L.nrows = nr;
-      L.ovr = overwrite;
-      L.srcs = srcs;
-      L.dsts.assign(dsts.begin() + g0 * R, dsts.begin() + g0 * R + nr);
-      L.shift = false;
-      if (same && nvec)
-        for (uint64_t d : L.dsts) L.shift = L.shift || (d & 15) != al;
-      out.push_back(std::move(L));
-      continue;
-    }
+  const int E = field_bytes(plan->field);
+  const CoeffSrc cs = plan_mat(plan);
+  const uint32_t* img = cs.img;
+  for (size_t r0 = 0; r0 < dsts.size(); r0 += lut_rows(E)) {
+    const size_t nr = std::min(lut_rows(E), dsts.size() - r0);
     LoweredJob L;
-    L.field = field;
-    L.tables = plan->dev + plan->off_mat;
-    L.gstride = plan->mat_groups;
-    L.g0 = g0;
-    L.G = std::min<size_t>(4, gtot - g0);
+    L.field = plan->field;
+    L.img = img;
+    L.byte_tab = cs.byte_tab;
     L.len = row_len;
-    L.head = head;
-    L.nvec = nvec;
     L.k = srcs.size();
-    L.nrows = std::min(nrows - g0 * R, L.G * R);
+    L.nrows = nr;
     L.ovr = overwrite;
     L.srcs = srcs;
-    L.dsts.assign(dsts.begin() + g0 * R, dsts.begin() + g0 * R + L.nrows);
-    L.shift = false;
-    if (same && nvec)
-      for (uint64_t d : L.dsts) L.shift = L.shift || (d & 15) != al;
+    L.dsts.assign(dsts.begin() + r0, dsts.begin() + r0 + nr);
     out.push_back(std::move(L));
+    img += srcs.size() * lut_shape(E, nr).src_words();
   }
 }
 
@@ -1152,19 +1094,6 @@ fgfc_status fgfc_batch_run(fgfc_batch* batch, const fgfc_matrix_job* jobs, size_
               cudaMemsetAsync(J.dst + (J.row_starts ? J.row_starts[j] : j * J.row_len), 0, J.row_len, stream);
           if (e != cudaSuccess) return cuda_fail(e, name);
         }
-      }
-      continue;
-    }
-    if (field_bytes(field) == 8) {  // 8-byte fields have their own kernel: one launch per stripe
-      std::vector<uint8_t*> rp(J.nrows);
-      for (size_t j = 0; j < J.nrows; ++j) rp[j] = J.dst + (J.row_starts ? J.row_starts[j] : j * J.row_len);
-      std::vector<const uint8_t*> sp(J.nsrcs);
-      for (size_t t = 0; t < J.nsrcs; ++t) sp[t] = J.srcs[t].ptr;
-      st = run_matrix(field, sp.data(), J.nsrcs, rp.data(), J.nrows, plan_mat(plan), J.row_len, J.overwrite != 0,
-                      stream, name);
-      if (st != FGFC_OK) {
-        t_err = "batch job " + std::to_string(i) + ": " + t_err;
-        return st;
       }
       continue;
     }

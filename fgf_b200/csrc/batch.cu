@@ -3,23 +3,18 @@
 // work-list.
 //
 // A submission is lowered on the host to sub-jobs (all sources of a stripe,
-// the rows of at most 4 table groups) and grouped in classes:
+// the rows of one table launch) and grouped in classes:
 //   * Gf8 sub-jobs of at most 4 rows and K <= 14 sources use the byte-table
 //     layout (fast_core.cuh), one class per K. When every sub-job of such a
 //     class shares one plan, the CTAs load the tables once and grid-stride
 //     over the flattened columns of all stripes (the stripes travel in the
-//     launch parameters); otherwise they claim work items.
-//   * everything else uses split-nibble tables, one class per (element
-//     width, groups); tables that do not fit at once are processed in source
-//     chunks inside the kernel.
-// Work items are (sub-job, part) pairs: part p of P covers the sub-job's
-// column vectors p*T + tid + j*P*T (T threads per CTA), so CTAs holding
-// consecutive items sweep one window of memory together; the remaining parts
-// cover the 4-byte scalar groups of heads, tails and unaligned stripes.
-// Persistent CTAs claim items from an atomic counter and reload their
-// shared-memory tables only when an item needs a different plan. The
-// descriptor blob (jobs, pointers, items, counters) goes to the device in one
-// copy, and a submission whose structure repeats replays a captured graph.
+//     launch parameters); otherwise each CTA takes one range of the columns.
+//   * everything else runs the table kernels (lut_batch.cuh) on work items
+//     (sub-job, part) claimed from a counter, one class per element width,
+//     tower split, output words and alignment. Items of a stripe interleave,
+//     so CTAs holding consecutive items sweep one window of memory together.
+// The descriptor blob (jobs, pointers, items, counters) goes to the device in
+// one copy, and a submission whose structure repeats replays a captured graph.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,415 +35,9 @@ namespace fgfc {
 
 namespace {
 
-struct BatchJob {
-  const uint32_t* tables;  // plan compact tables (matrix orientation)
-  uint64_t len;            // bytes per row
-  uint64_t head;           // scalar bytes before the vector body
-  uint64_t nvec;           // 16-byte vectors in the body
-  uint32_t gstride, g0;    // plan groups per (source, plane); first group of this sub-job
-  uint32_t k, nrows;       // sources; rows of this sub-job
-  uint32_t ovr;            // 1 = overwrite
-  uint32_t src_idx, dst_idx;
-  uint32_t nv_items;       // vector items; scalar items follow
-};
-
-constexpr int kThreads = 512;
-constexpr uint32_t kVecPerItem = 8 * kThreads;
-constexpr uint32_t kGroupsPerItem = kThreads;
 constexpr uint32_t kFastVecPerItem = 8 * kFastThreads;
 constexpr uint32_t kFastGroupsPerItem = kFastThreads;
-constexpr uint32_t kClaim = 2;  // items claimed per atomic
-
-// ---------------------------------------------------------------- nibble classes
-
-// Expand compact tables of sources [t0, t0 + kk) into the replicated
-// nibble layout (slot = (t * E + p) * G + g, 4 KiB each), via a staging copy.
-template <int E, int G>
-__device__ void fill_chunk(const BatchJob& J, uint32_t t0, uint32_t kk) {
-  const uint32_t nslots = kk * E * G;
-  uint32_t* stage = reinterpret_cast<uint32_t*>(g_smem) + kMaxSlots * 1024u;
-  __syncthreads();  // previous tables no longer read
-  for (uint32_t i = threadIdx.x; i < nslots * kCompactWords; i += blockDim.x) {
-    const uint32_t slot = i >> 5;
-    const uint32_t tp = t0 * E + slot / G;
-    stage[i] = __ldg(J.tables + (tp * J.gstride + J.g0 + slot % G) * kCompactWords + (i & 31u));
-  }
-  __syncthreads();
-  uint4* st4 = reinterpret_cast<uint4*>(g_smem);
-#pragma unroll 4
-  for (uint32_t i = threadIdx.x; i < nslots * 256u; i += blockDim.x) {
-    const uint32_t v = stage[(i >> 8) * kCompactWords + ((i >> 3) & 1u) * 16u + ((i >> 4) & 15u)];
-    st4[i] = make_uint4(v, v, v, v);
-  }
-  __syncthreads();
-}
-
-template <int E, int G>
-struct Ctx {
-  uint32_t pat;
-  uint32_t lr[E];
-  __device__ __forceinline__ Ctx(uint32_t t, uint32_t lane4) {
-    pat = 0;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) pat |= (((t * E + (b % E)) * G) & 15u) << (8 * b + 4);
-#pragma unroll
-    for (int p = 0; p < E; ++p) lr[p] = lane4 | ((((t * E + p) * G) >> 4) << 16);
-  }
-};
-
-template <int E, int G, int NE>
-__device__ __forceinline__ void fold(uint32_t w, const Ctx<E, G>& c, uint32_t (&acc)[G][NE], int e0) {
-  const uint32_t xl = (w & 0x0F0F0F0Fu) | c.pat;
-  const uint32_t xh = ((w >> 4) & 0x0F0F0F0Fu) | c.pat;
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const uint32_t sel = 0x7604u | (static_cast<uint32_t>(b) << 4);
-    const uint32_t al = prmt(xl, c.lr[b % E], sel);
-    const uint32_t ah = prmt(xh, c.lr[b % E], sel);
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-      acc[g][e0 + b / E] ^= lds_at(al + g * kSlotBytes) ^ lds_at(ah + g * kSlotBytes + 128);
-  }
-}
-
-template <int E, int G, int NE>
-__device__ __forceinline__ uint32_t out_word(const uint32_t (&acc)[G][NE], int g, int rr, int q) {
-  if (E == 1) {
-    return row_word4(&acc[g][4 * q], rr);
-  } else if (E == 2) {
-    return prmt(acc[g][2 * q], acc[g][2 * q + 1], rr ? 0x7632u : 0x5410u);
-  } else {
-    return acc[g][q];
-  }
-}
-
-// One vector item of a sub-job, for sources [t0, t0 + kk) whose tables are
-// resident; `ovr` overwrites, otherwise the destination is accumulated.
-// SHIFT: some row is not at the sources' offset within 16 bytes; whole warps
-// then iterate together (the row stores shuffle between lanes) and lanes past
-// the end reload the last column.
-template <int E, int G, bool SHIFT>
-__device__ void vector_item(const BatchJob& J, const uint64_t* ptrs, uint32_t part, uint32_t t0,
-                            uint32_t kk, bool ovr) {
-  constexpr int NE = 16 / E, R = 4 / E;
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t lane4 = lane * 4u;
-  const uint64_t step = static_cast<uint64_t>(J.nv_items) * blockDim.x;
-  for (uint64_t vb = static_cast<uint64_t>(part) * blockDim.x + threadIdx.x - (SHIFT ? lane : 0u); vb < J.nvec;
-       vb += step) {
-    const uint64_t v = SHIFT ? vb + lane : vb;
-    const bool valid = !SHIFT || v < J.nvec;
-    const uint64_t off = J.head + (valid ? v : J.nvec - 1) * 16u;
-    uint32_t acc[G][NE];
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-      for (int e = 0; e < NE; ++e) acc[g][e] = 0;
-    const uint8_t* const* srcs = reinterpret_cast<const uint8_t* const*>(ptrs + J.src_idx + t0);
-    uint4 cur = ldg16(srcs[0] + off);
-    for (uint32_t t = 0; t < kk; ++t) {
-      uint4 nxt = cur;
-      if (t + 1 < kk) nxt = ldg16(srcs[t + 1] + off);
-      const Ctx<E, G> c(t, lane4);
-      fold<E, G, NE>(cur.x, c, acc, 0);
-      fold<E, G, NE>(cur.y, c, acc, 4 / E);
-      fold<E, G, NE>(cur.z, c, acc, 2 * (4 / E));
-      fold<E, G, NE>(cur.w, c, acc, 3 * (4 / E));
-      cur = nxt;
-    }
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-      for (int rr = 0; rr < R; ++rr) {
-        const uint32_t row = g * R + rr;
-        uint4 o;
-        o.x = out_word<E, G, NE>(acc, g, rr, 0);
-        o.y = out_word<E, G, NE>(acc, g, rr, 1);
-        o.z = out_word<E, G, NE>(acc, g, rr, 2);
-        o.w = out_word<E, G, NE>(acc, g, rr, 3);
-        if constexpr (SHIFT) {
-          const bool rv = valid && row < J.nrows;
-          store_vec16(rv ? reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + row]) + off : nullptr, o, rv, ovr);
-        } else {
-          if (row < J.nrows) put16(reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + row]) + off, o, ovr);
-        }
-      }
-  }
-}
-
-// One scalar item: 4-byte groups of the head [0, head) and the tail
-// [head + 16 * nvec, len) of every row, byte loads and stores.
-template <int E, int G>
-__device__ void scalar_item(const BatchJob& J, const uint64_t* ptrs, uint32_t part, uint32_t t0,
-                            uint32_t kk, bool ovr) {
-  constexpr int R = 4 / E;
-  const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
-  const uint64_t tail0 = J.head + J.nvec * 16u;
-  const uint64_t n0 = (J.head + 3) / 4, n1 = (J.len - tail0 + 3) / 4;
-  const uint64_t gi = static_cast<uint64_t>(part) * kGroupsPerItem + threadIdx.x;
-  // every thread runs the lookups (uniform control flow); only threads with
-  // a group in range touch memory
-  const bool live = gi < n0 + n1;
-  const uint64_t off = !live ? 0 : (gi < n0 ? 4 * gi : tail0 + 4 * (gi - n0));
-  const uint64_t end = !live ? 0 : (gi < n0 ? J.head : J.len);
-  const int nb = !live ? 0 : static_cast<int>(end - off < 4 ? end - off : 4);
-  uint32_t acc[G][4 / E];
-#pragma unroll
-  for (int g = 0; g < G; ++g)
-#pragma unroll
-    for (int e = 0; e < 4 / E; ++e) acc[g][e] = 0;
-  for (uint32_t t = 0; t < kk; ++t) {
-    const uint8_t* s = reinterpret_cast<const uint8_t*>(ptrs[J.src_idx + t0 + t]) + off;
-    uint32_t w = 0;
-    for (int b = 0; b < nb; ++b) w |= static_cast<uint32_t>(s[b]) << (8 * b);
-    const Ctx<E, G> c(t, lane4);
-    fold<E, G, 4 / E>(w, c, acc, 0);
-  }
-  if (!live) return;
-#pragma unroll
-  for (int g = 0; g < G; ++g)
-#pragma unroll
-    for (int rr = 0; rr < R; ++rr) {
-      const uint32_t row = g * R + rr;
-      if (row >= J.nrows) continue;
-      uint32_t o;
-      if (E == 1) {
-        o = row_word4(&acc[g][0], rr);
-      } else if (E == 2) {
-        o = prmt(acc[g][0], acc[g][1], rr ? 0x7632u : 0x5410u);
-      } else {
-        o = acc[g][0];
-      }
-      uint8_t* d = reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + row]) + off;
-      for (int b = 0; b < nb; ++b) {
-        const uint8_t v = static_cast<uint8_t>(o >> (8 * b));
-        d[b] = ovr ? v : static_cast<uint8_t>(d[b] ^ v);
-      }
-    }
-}
-
-// Persistent work-list kernel for one nibble (E, G) class.
-template <int E, int G, bool SHIFT>
-__global__ void __launch_bounds__(kThreads, 1)
-    batch_kernel(const BatchJob* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
-                 const uint2* __restrict__ items, uint32_t nitems, uint32_t* counter) {
-  __shared__ uint32_t s_item;
-  __shared__ const uint32_t* s_tab;
-  __shared__ uint32_t s_g0, s_t0;
-  const uint32_t kc = kMaxSlots / (E * G);  // sources whose tables fit at once
-  if (threadIdx.x == 0) {
-    s_tab = nullptr;
-    s_g0 = s_t0 = 0xFFFFFFFFu;
-  }
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) s_item = atomicAdd(counter, kClaim);
-    __syncthreads();
-    const uint32_t first = s_item;
-    if (first >= nitems) break;
-    for (uint32_t it = first; it < first + kClaim && it < nitems; ++it) {
-      const uint2 wi = items[it];
-      const BatchJob J = jobs[wi.x];
-      const uint32_t nchunks = (J.k + kc - 1) / kc;
-      for (uint32_t c = 0; c < nchunks; ++c) {
-        const uint32_t t0 = c * kc, kk = min(kc, J.k - t0);
-        __syncthreads();
-        const bool resident = s_tab == J.tables && s_g0 == J.g0 && s_t0 == t0;
-        if (!resident) {
-          fill_chunk<E, G>(J, t0, kk);
-          if (threadIdx.x == 0) {
-            s_tab = J.tables;
-            s_g0 = J.g0;
-            s_t0 = t0;
-          }
-        }
-        const bool ovr = J.ovr && c == 0;
-        if (wi.y < J.nv_items)
-          vector_item<E, G, SHIFT>(J, ptrs, wi.y, t0, kk, ovr);
-        else
-          scalar_item<E, G>(J, ptrs, wi.y - J.nv_items, t0, kk, ovr);
-        __syncthreads();  // chunk c's writes precede chunk c + 1's reads of the same rows
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------- Gf16 by byte half-products
-
-// Gf16 = Gf8B[u]/(u^2 + u + 0x20) (src/field/gf16.rs:143-153): with
-// c = c0 + c1 u and x = a + b u, A = c0 a, B = c1 b, C = (c0 + c1)(a + b)
-// give c x = (A + 0x20 B) + (A + C) u. Each byte half-product is a Gf8
-// nibble fold whose table word holds 4 rows, so an element costs 3 x 2
-// lookups per 4 rows instead of 2 x 2 per 2 rows. The tables are those of
-// 3 "virtual sources" per source (3t + P, tables.cpp: build_kara16_tables).
-
-// v * 0x20 in every byte of v over Gf8B (x^8 + x^4 + x^3 + x + 1).
-__device__ __forceinline__ uint32_t mul20_4(uint32_t v) {
-#pragma unroll
-  for (int i = 0; i < 5; ++i) v = ((v & 0x7F7F7F7Fu) << 1) ^ (((v >> 7) & 0x01010101u) * 0x1Bu);
-  return v;
-}
-
-// Row word of elements e, e + 1 (lo and hi words: byte r = row 4q + r).
-__device__ __forceinline__ uint32_t k16_word(uint32_t lo0, uint32_t hi0, uint32_t lo1, uint32_t hi1, int r) {
-  const uint32_t sel = static_cast<uint32_t>(r) | ((4u + static_cast<uint32_t>(r)) << 4);
-  return prmt(prmt(lo0, hi0, sel), prmt(lo1, hi1, sel), 0x5410u);
-}
-
-template <int GK, int NE>
-__device__ __forceinline__ void k16_finish(uint32_t (&A)[GK][NE], uint32_t (&B)[GK][NE], uint32_t (&C)[GK][NE]) {
-#pragma unroll
-  for (int q = 0; q < GK; ++q)
-#pragma unroll
-    for (int e = 0; e < NE; ++e) {
-      B[q][e] = A[q][e] ^ mul20_4(B[q][e]);  // lo
-      C[q][e] ^= A[q][e];                    // hi
-    }
-}
-
-template <int GK, bool SHIFT>
-__device__ void vector_item_k16(const BatchJob& J, const uint64_t* ptrs, uint32_t part, uint32_t t0, uint32_t kk,
-                                bool ovr) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t lane4 = lane * 4u;
-  const uint64_t step = static_cast<uint64_t>(J.nv_items) * blockDim.x;
-  for (uint64_t vb = static_cast<uint64_t>(part) * blockDim.x + threadIdx.x - (SHIFT ? lane : 0u); vb < J.nvec;
-       vb += step) {
-    const uint64_t v = SHIFT ? vb + lane : vb;
-    const bool valid = !SHIFT || v < J.nvec;
-    const uint64_t off = J.head + (valid ? v : J.nvec - 1) * 16u;
-    uint32_t A[GK][8], B[GK][8], C[GK][8];
-#pragma unroll
-    for (int q = 0; q < GK; ++q)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) A[q][e] = B[q][e] = C[q][e] = 0;
-    const uint8_t* const* srcs = reinterpret_cast<const uint8_t* const*>(ptrs + J.src_idx + t0);
-    uint4 cur = ldg16(srcs[0] + off);
-    for (uint32_t t = 0; t < kk; ++t) {
-      uint4 nxt = cur;
-      if (t + 1 < kk) nxt = ldg16(srcs[t + 1] + off);
-      // low and high bytes of the 8 elements
-      const uint32_t a0 = prmt(cur.x, cur.y, 0x6420u), a1 = prmt(cur.z, cur.w, 0x6420u);
-      const uint32_t b0 = prmt(cur.x, cur.y, 0x7531u), b1 = prmt(cur.z, cur.w, 0x7531u);
-      const Ctx<1, GK> ca(3u * t, lane4), cb(3u * t + 1u, lane4), cc(3u * t + 2u, lane4);
-      fold<1, GK, 8>(a0, ca, A, 0);
-      fold<1, GK, 8>(a1, ca, A, 4);
-      fold<1, GK, 8>(b0, cb, B, 0);
-      fold<1, GK, 8>(b1, cb, B, 4);
-      fold<1, GK, 8>(a0 ^ b0, cc, C, 0);
-      fold<1, GK, 8>(a1 ^ b1, cc, C, 4);
-      cur = nxt;
-    }
-    k16_finish<GK, 8>(A, B, C);
-#pragma unroll
-    for (int q = 0; q < GK; ++q)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const uint32_t row = 4 * q + r;
-        uint4 o;
-        o.x = k16_word(B[q][0], C[q][0], B[q][1], C[q][1], r);
-        o.y = k16_word(B[q][2], C[q][2], B[q][3], C[q][3], r);
-        o.z = k16_word(B[q][4], C[q][4], B[q][5], C[q][5], r);
-        o.w = k16_word(B[q][6], C[q][6], B[q][7], C[q][7], r);
-        if constexpr (SHIFT) {
-          const bool rv = valid && row < J.nrows;
-          store_vec16(rv ? reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + row]) + off : nullptr, o, rv, ovr);
-        } else {
-          if (row < J.nrows) put16(reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + row]) + off, o, ovr);
-        }
-      }
-  }
-}
-
-// Heads and tails: 4-byte groups (two elements) with byte loads and stores.
-template <int GK>
-__device__ void scalar_item_k16(const BatchJob& J, const uint64_t* ptrs, uint32_t part, uint32_t t0, uint32_t kk,
-                                bool ovr) {
-  const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
-  const uint64_t tail0 = J.head + J.nvec * 16u;
-  const uint64_t n0 = (J.head + 3) / 4, n1 = (J.len - tail0 + 3) / 4;
-  const uint64_t gi = static_cast<uint64_t>(part) * kGroupsPerItem + threadIdx.x;
-  const bool live = gi < n0 + n1;
-  const uint64_t off = !live ? 0 : (gi < n0 ? 4 * gi : tail0 + 4 * (gi - n0));
-  const uint64_t end = !live ? 0 : (gi < n0 ? J.head : J.len);
-  const int nb = !live ? 0 : static_cast<int>(end - off < 4 ? end - off : 4);
-  uint32_t A[GK][4], B[GK][4], C[GK][4];
-#pragma unroll
-  for (int q = 0; q < GK; ++q)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) A[q][e] = B[q][e] = C[q][e] = 0;
-  for (uint32_t t = 0; t < kk; ++t) {
-    const uint8_t* s = reinterpret_cast<const uint8_t*>(ptrs[J.src_idx + t0 + t]) + off;
-    uint32_t w = 0;
-    for (int b = 0; b < nb; ++b) w |= static_cast<uint32_t>(s[b]) << (8 * b);
-    const uint32_t a = prmt(w, 0u, 0x4420u), bb = prmt(w, 0u, 0x4431u);  // [a0 a1 0 0], [b0 b1 0 0]
-    const Ctx<1, GK> ca(3u * t, lane4), cb(3u * t + 1u, lane4), cc(3u * t + 2u, lane4);
-    fold<1, GK, 4>(a, ca, A, 0);
-    fold<1, GK, 4>(bb, cb, B, 0);
-    fold<1, GK, 4>(a ^ bb, cc, C, 0);
-  }
-  if (!live) return;
-  k16_finish<GK, 4>(A, B, C);
-#pragma unroll
-  for (int q = 0; q < GK; ++q)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const uint32_t row = 4 * q + r;
-      if (row >= J.nrows) continue;
-      const uint32_t o = k16_word(B[q][0], C[q][0], B[q][1], C[q][1], r);
-      uint8_t* d = reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + row]) + off;
-      for (int b = 0; b < nb; ++b) {
-        const uint8_t v = static_cast<uint8_t>(o >> (8 * b));
-        d[b] = ovr ? v : static_cast<uint8_t>(d[b] ^ v);
-      }
-    }
-}
-
-// Persistent work-list kernel of a Gf16 half-product class: GK row quads.
-template <int GK, bool SHIFT>
-__global__ void __launch_bounds__(kThreads, 1)
-    batch_kernel_k16(const BatchJob* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
-                     const uint2* __restrict__ items, uint32_t nitems, uint32_t* counter) {
-  __shared__ uint32_t s_item;
-  __shared__ const uint32_t* s_tab;
-  __shared__ uint32_t s_g0, s_t0;
-  const uint32_t kc = kMaxSlots / (3 * GK);  // sources whose tables fit at once
-  if (threadIdx.x == 0) {
-    s_tab = nullptr;
-    s_g0 = s_t0 = 0xFFFFFFFFu;
-  }
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) s_item = atomicAdd(counter, kClaim);
-    __syncthreads();
-    const uint32_t first = s_item;
-    if (first >= nitems) break;
-    for (uint32_t it = first; it < first + kClaim && it < nitems; ++it) {
-      const uint2 wi = items[it];
-      const BatchJob J = jobs[wi.x];
-      const uint32_t nchunks = (J.k + kc - 1) / kc;
-      for (uint32_t c = 0; c < nchunks; ++c) {
-        const uint32_t t0 = c * kc, kk = min(kc, J.k - t0);
-        __syncthreads();
-        const bool resident = s_tab == J.tables && s_g0 == J.g0 && s_t0 == t0;
-        if (!resident) {
-          fill_chunk<1, GK>(J, 3 * t0, 3 * kk);
-          if (threadIdx.x == 0) {
-            s_tab = J.tables;
-            s_g0 = J.g0;
-            s_t0 = t0;
-          }
-        }
-        const bool ovr = J.ovr && c == 0;
-        if (wi.y < J.nv_items)
-          vector_item_k16<GK, SHIFT>(J, ptrs, wi.y, t0, kk, ovr);
-        else
-          scalar_item_k16<GK>(J, ptrs, wi.y - J.nv_items, t0, kk, ovr);
-        __syncthreads();  // chunk c's writes precede chunk c + 1's reads of the same rows
-      }
-    }
-  }
-}
+constexpr uint32_t kClaim = 2;  // byte-table items claimed per atomic
 
 // ---------------------------------------------------------------- byte-table classes
 
@@ -456,16 +45,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 // The plan's tables stay resident across consecutive items of one plan.
 template <int K, bool SHIFT>
 __global__ void __launch_bounds__(kFastThreads, 1)
-    batch_fast_kernel(const BatchJob* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
+    batch_fast_kernel(const BatchDesc* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
                       const uint2* __restrict__ items, uint32_t nitems, uint32_t* counter) {
   __shared__ uint32_t s_item;
   __shared__ const uint32_t* s_tab;
-  __shared__ uint32_t s_g0;
   __shared__ const uint8_t* s_src[K];
   __shared__ uint8_t* s_dst[4];
   if (threadIdx.x == 0) {
     s_tab = nullptr;
-    s_g0 = 0xFFFFFFFFu;
   }
   const FastRegs r;
   for (;;) {
@@ -476,16 +63,15 @@ __global__ void __launch_bounds__(kFastThreads, 1)
     if (first >= nitems) break;
     for (uint32_t it = first; it < first + kClaim && it < nitems; ++it) {
       const uint2 wi = items[it];
-      const BatchJob J = jobs[wi.x];
+      const BatchJob J = jobs[wi.x].byte;
       __syncthreads();  // the previous item is done with tables and pointers
-      const bool resident = s_tab == J.tables && s_g0 == J.g0;
+      const bool resident = s_tab == J.tables;
       if (threadIdx.x < K) s_src[threadIdx.x] = reinterpret_cast<const uint8_t*>(ptrs[J.src_idx + threadIdx.x]);
       if (threadIdx.x < J.nrows) s_dst[threadIdx.x] = reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + threadIdx.x]);
       if (!resident) {
-        fill_fast<K>(J.tables, nullptr, J.gstride, J.g0);
+        fill_fast<K>(J.tables, nullptr);
         if (threadIdx.x == 0) {
           s_tab = J.tables;
-          s_g0 = J.g0;
         }
       }
       __syncthreads();
@@ -566,11 +152,10 @@ __global__ void __launch_bounds__(kFastThreads, 1)
 // tails of the class.
 template <int K, bool SHIFT>
 __global__ void __launch_bounds__(kFastThreads, 1)
-    batch_fast_segment_kernel(const BatchJob* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
+    batch_fast_segment_kernel(const BatchDesc* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
                               const uint32_t* __restrict__ jidx, const uint64_t* __restrict__ vprefix,
                               uint32_t njobs) {
   __shared__ const uint32_t* s_tab;
-  __shared__ uint32_t s_g0;
   __shared__ const uint8_t* s_src[K];
   __shared__ uint8_t* s_dst[4];
   const uint64_t vtotal = vprefix[njobs];
@@ -588,7 +173,6 @@ __global__ void __launch_bounds__(kFastThreads, 1)
   uint32_t q = lo;
   if (threadIdx.x == 0) {
     s_tab = nullptr;
-    s_g0 = 0xFFFFFFFFu;
   }
   const FastRegs r;
   const uint32_t lane = threadIdx.x & 31u;
@@ -596,16 +180,15 @@ __global__ void __launch_bounds__(kFastThreads, 1)
     while (vprefix[q + 1] <= v0) ++q;  // sub-jobs without vectors
     const uint64_t base = vprefix[q];
     const uint64_t vend = vprefix[q + 1] < v1 ? vprefix[q + 1] : v1;
-    const BatchJob J = jobs[jidx[q]];
+    const BatchJob J = jobs[jidx[q]].byte;
     __syncthreads();  // the previous sub-job is done with tables and pointers
-    const bool resident = s_tab == J.tables && s_g0 == J.g0;
+    const bool resident = s_tab == J.tables;
     if (threadIdx.x < K) s_src[threadIdx.x] = reinterpret_cast<const uint8_t*>(ptrs[J.src_idx + threadIdx.x]);
     if (threadIdx.x < J.nrows) s_dst[threadIdx.x] = reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + threadIdx.x]);
     if (!resident) {
-      fill_fast<K>(J.tables, nullptr, J.gstride, J.g0);
+      fill_fast<K>(J.tables, nullptr);
       if (threadIdx.x == 0) {
         s_tab = J.tables;
-        s_g0 = J.g0;
       }
     }
     __syncthreads();
@@ -661,7 +244,7 @@ struct UJob {
 
 struct UniformParams {
   const uint32_t* tables;
-  uint32_t gstride, g0, njobs, pad;
+  uint32_t njobs, pad;
   uint64_t vprefix[kUniformJobs + 1];
   uint64_t gprefix[kUniformJobs + 1];
   UJob jobs[kUniformJobs];
@@ -671,7 +254,7 @@ static_assert(sizeof(UniformParams) <= 32000, "launch parameter block too large"
 template <int K, bool SHIFT>
 __global__ void __launch_bounds__(kFastThreads, 1)
     batch_fast_uniform_kernel(const __grid_constant__ UniformParams P) {
-  fill_fast<K>(P.tables, nullptr, P.gstride, P.g0);
+  fill_fast<K>(P.tables, nullptr);
   const FastRegs r;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -745,36 +328,9 @@ __global__ void __launch_bounds__(kFastThreads, 1)
   }
 }
 
-using KernelFn = void (*)(const BatchJob*, const uint64_t*, const uint2*, uint32_t, uint32_t*);
+using KernelFn = void (*)(const BatchDesc*, const uint64_t*, const uint2*, uint32_t, uint32_t*);
 using UniformFn = void (*)(UniformParams);
-using SegmentFn = void (*)(const BatchJob*, const uint64_t*, const uint32_t*, const uint64_t*, uint32_t);
-
-template <bool S>
-KernelFn kernel_for_s(int E, int G) {
-  switch (E * 8 + G) {
-    case 8 + 1: return batch_kernel<1, 1, S>;
-    case 8 + 2: return batch_kernel<1, 2, S>;
-    case 8 + 3: return batch_kernel<1, 3, S>;
-    case 8 + 4: return batch_kernel<1, 4, S>;
-    case 16 + 1: return batch_kernel<2, 1, S>;
-    case 16 + 2: return batch_kernel<2, 2, S>;
-    case 16 + 3: return batch_kernel<2, 3, S>;
-    case 16 + 4: return batch_kernel<2, 4, S>;
-    case 32 + 1: return batch_kernel<4, 1, S>;
-    case 32 + 2: return batch_kernel<4, 2, S>;
-    case 32 + 3: return batch_kernel<4, 3, S>;
-    case 32 + 4: return batch_kernel<4, 4, S>;
-    default: return nullptr;
-  }
-}
-
-KernelFn kernel_for(int E, int G, bool shift) { return shift ? kernel_for_s<true>(E, G) : kernel_for_s<false>(E, G); }
-
-KernelFn kernel_for_k16(int GK, bool shift) {
-  if (GK == 1) return shift ? batch_kernel_k16<1, true> : batch_kernel_k16<1, false>;
-  if (GK == 2) return shift ? batch_kernel_k16<2, true> : batch_kernel_k16<2, false>;
-  return nullptr;
-}
+using SegmentFn = void (*)(const BatchDesc*, const uint64_t*, const uint32_t*, const uint64_t*, uint32_t);
 
 #define FGFC_K_CASES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14)
 
@@ -818,22 +374,23 @@ uint32_t fast_smem(int K) {
   }
 }
 
-constexpr size_t kBatchSmem = kMaxSlots * (kSlotBytes + kCompactWords * 4);
-
 }  // namespace
 
 // ---------------------------------------------------------------- host side
 
 struct BatchClass {
-  int E, G;
+  int E;
   int K = 0;                   // > 0: byte-table class of Gf8 sub-jobs with K sources
+  LutShape shape{};            // table class
+  LutBatchKernel kern;
+  size_t kc = 0;               // sources per fill
   std::vector<uint32_t> jobs;  // sub-job indices, plan order
   std::vector<uint2> items;
+  std::vector<size_t> cuts;    // first item of each launch after the first
   std::vector<uint32_t> seg_jobs;   // byte-table class with own plans: sub-jobs with vectors, plan order
   std::vector<uint64_t> seg_prefix; // and the prefix of their vector counts (the segmented launch)
   bool uniform = false;        // byte-table class whose sub-jobs share one plan
   bool shift = false;          // its rows are not all at the sources' offset within 16 bytes
-  bool kara = false;           // Gf16 by byte half-products, G = row quads
 };
 
 // Descriptor slots used round robin: a submission waits (on the host) only
@@ -865,7 +422,7 @@ struct BatchState {
   cudaEvent_t fork = nullptr, join[kSideStreams] = {};
   size_t last_launches = 0, last_items = 0;
   int last_replayed = 0;
-  std::vector<std::pair<int, int>> last_classes;  // nibble (E, G) classes of the last submission
+  std::vector<std::pair<int, int>> last_classes;  // table (E, G) classes of the last submission
   mutable std::mutex mu;
 };
 
@@ -935,6 +492,23 @@ void batch_state_stats(const void* p, size_t* launches, size_t* items, int* repl
 
 static size_t align16(size_t x) { return (x + 15) & ~static_cast<size_t>(15); }
 
+// The table sub-job of rows at `a`; parts, pointers to be filled in.
+static LutBatchJob lut_batch_job(int field, const uint32_t* img, const JobAlign& a, uint64_t len, size_t k, size_t nrows,
+                                 bool ovr) {
+  LutBatchJob J;
+  std::memset(&J, 0, sizeof J);
+  J.img = img;
+  J.g.len = len;
+  J.g.head = a.unal ? 0 : a.head;
+  J.g.ncol = (len - J.g.head) / 16;
+  J.g.k = static_cast<uint32_t>(k);
+  J.g.nrows = static_cast<uint32_t>(nrows);
+  J.g.ovr = ovr ? 1u : 0u;
+  J.g.bytes = a.unal && a.overlap ? 1u : 0u;
+  J.fp = field == kFp16 || field == kFp32 || field == kFp64 ? 1u : 0u;
+  return J;
+}
+
 cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const std::vector<Gf2Job>& tc,
                       cudaStream_t stream) {
   BatchState* b = static_cast<BatchState*>(state);
@@ -945,93 +519,110 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   if (jobs.empty() && tc.empty()) return cudaSuccess;
 
   // ---- device descriptors, pointer array, classes (sub-jobs in plan order)
-  std::vector<BatchJob> dj(jobs.size());
+  std::vector<BatchDesc> dj(jobs.size());
+  std::vector<JobAlign> al(jobs.size());
   std::vector<uint64_t> ptrs;
+  std::vector<std::pair<uint32_t, uint32_t>> idx(jobs.size());  // first source and row pointer
   for (size_t i = 0; i < jobs.size(); ++i) {
     const LoweredJob& L = jobs[i];
-    BatchJob& J = dj[i];
-    J.tables = L.tables;
-    J.len = L.len;
-    J.head = L.head;
-    J.nvec = L.nvec;
-    J.gstride = static_cast<uint32_t>(L.gstride);
-    J.g0 = static_cast<uint32_t>(L.g0);
-    J.k = static_cast<uint32_t>(L.k);
-    J.nrows = static_cast<uint32_t>(L.nrows);
-    J.ovr = L.ovr ? 1u : 0u;
-    J.src_idx = static_cast<uint32_t>(ptrs.size());
+    al[i] = job_align(L.field, L.srcs.data(), L.k, L.dsts.data(), L.nrows, L.len);
+    idx[i].first = static_cast<uint32_t>(ptrs.size());
     ptrs.insert(ptrs.end(), L.srcs.begin(), L.srcs.end());
-    J.dst_idx = static_cast<uint32_t>(ptrs.size());
+    idx[i].second = static_cast<uint32_t>(ptrs.size());
     ptrs.insert(ptrs.end(), L.dsts.begin(), L.dsts.end());
-    J.nv_items = 0;
   }
   std::vector<size_t> order(jobs.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t c) {
-    return jobs[a].tables != jobs[c].tables ? jobs[a].tables < jobs[c].tables : jobs[a].g0 < jobs[c].g0;
-  });
-  std::map<int, BatchClass> classes;  // key E * 8 + G, or 100 + K for byte-table classes; + 300 if shifted
+  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t c) { return jobs[a].img < jobs[c].img; });
+  std::map<int, BatchClass> classes;
   for (size_t i : order) {
     const LoweredJob& L = jobs[i];
     const int E = field_bytes(L.field);
-    const bool fast = E == 1 && L.G == 1 && L.k >= 1 && L.k <= static_cast<size_t>(kFastMaxK);
-    const int key = (fast ? 100 + static_cast<int>(L.k) : L.kara ? 200 + static_cast<int>(L.G)
-                                                                  : E * 8 + static_cast<int>(L.G)) +
-                    (L.shift ? 300 : 0);
+    const bool fast = L.byte_tab && al[i].sources;
+    const LutShape shape = lut_shape(E, L.nrows);
+    const int key = fast ? 1000 + 2 * static_cast<int>(L.k) + al[i].unal
+                         : ((E * 4 + shape.lev) * 8 + shape.w) * 2 + al[i].unal;
     BatchClass& c = classes[key];
-    c.shift = L.shift;
-    c.kara = L.kara;
     c.E = E;
-    c.G = static_cast<int>(L.G);
-    c.K = fast ? static_cast<int>(L.k) : 0;
     c.jobs.push_back(static_cast<uint32_t>(i));
+    BatchDesc& D = dj[i];
+    if (fast) {
+      c.shift = al[i].unal;
+      c.K = static_cast<int>(L.k);
+      BatchJob& J = D.byte;
+      J.tables = L.byte_tab;
+      J.len = L.len;
+      J.head = al[i].head;
+      J.nvec = (L.len - J.head) / 16;
+      J.k = static_cast<uint32_t>(L.k);
+      J.nrows = static_cast<uint32_t>(L.nrows);
+      J.ovr = L.ovr ? 1u : 0u;
+      J.src_idx = idx[i].first;
+      J.dst_idx = idx[i].second;
+      J.nv_items = 0;
+    } else {
+      c.shape = shape;
+      c.kern = lut_batch_kernel_for(E, shape, al[i].unal);
+      c.kc = lut_sources(E, L.nrows, false);
+      D.lut = lut_batch_job(L.field, L.img, al[i], L.len, L.k, L.nrows, L.ovr);
+      D.lut.src_idx = idx[i].first;
+      D.lut.dst_idx = idx[i].second;
+    }
   }
   for (auto& kv : classes) {
     BatchClass& c = kv.second;
-    c.uniform = c.K > 0;
-    for (uint32_t i : c.jobs)
-      c.uniform = c.uniform && jobs[i].tables == jobs[c.jobs[0]].tables && jobs[i].g0 == jobs[c.jobs[0]].g0;
-    if (c.uniform) continue;
-    // Columns per item: the class's tile (tune.cpp: tile_cols; 8 per
-    // thread built in) for nibble classes, 8 per thread for byte-table
-    // classes, fewer when the class is too small to give every SM a few
-    // items (a small class runs beside the others on its own stream, see
-    // enqueue).
-    const uint64_t threads = c.K ? kFastThreads : kThreads;
-    const uint64_t tile = c.K ? kFastVecPerItem : threads * static_cast<uint64_t>(tile_cols(c.E, c.G));
-    if (!c.K) b->last_classes.emplace_back(c.E, c.G);
-    uint64_t total = 0;
-    for (uint32_t i : c.jobs) total += jobs[i].nvec;
-    const uint64_t want = (total + 4 * static_cast<uint64_t>(sm_count()) - 1) / (4 * static_cast<uint64_t>(sm_count()));
-    const uint64_t per_vec = std::min<uint64_t>(tile, std::max<uint64_t>(threads, (want + threads - 1) / threads * threads));
-    const uint64_t per_grp = c.K ? kFastGroupsPerItem : kGroupsPerItem;
-    for (uint32_t i : c.jobs) {
-      const LoweredJob& L = jobs[i];
-      const uint64_t nv_items = (L.nvec + per_vec - 1) / per_vec;
-      const uint64_t tail = L.len - L.head - 16 * L.nvec;
-      const uint64_t ngroups = (L.head + 3) / 4 + (tail + 3) / 4;
-      const uint64_t ns_items = (ngroups + per_grp - 1) / per_grp;
-      dj[i].nv_items = static_cast<uint32_t>(nv_items);
-      if (c.K > 0) {
-        // vectors: the segmented launch; scalar heads and tails: work items
-        if (L.nvec) {
-          if (c.seg_prefix.empty()) c.seg_prefix.push_back(0);
-          c.seg_jobs.push_back(i);
-          c.seg_prefix.push_back(c.seg_prefix.back() + L.nvec);
-        }
-        for (uint64_t p = nv_items; p < nv_items + ns_items; ++p)
-          c.items.push_back(make_uint2(i, static_cast<unsigned>(p)));
-      } else {
-        for (uint64_t p = 0; p < nv_items + ns_items; ++p)
-          c.items.push_back(make_uint2(i, static_cast<unsigned>(p)));
+    if (c.K == 0) {
+      // Tiles per item: the class's tile shape (tune.cpp: tile_cols; 8 columns
+      // per thread built in), fewer when the class is too small to give every
+      // resident CTA a few items (a small class runs beside the others on its
+      // own stream, see enqueue).
+      const int G = static_cast<int>((jobs[c.jobs[0]].nrows * c.E + 3) / 4);
+      const uint64_t tile = c.E == 8 ? kTileColsDefault : tile_cols(c.E, G);
+      if (c.E < 8) b->last_classes.emplace_back(c.E, G);
+      const bool unal = kv.first & 1;
+      uint64_t total = 0;
+      for (uint32_t i : c.jobs) total += lut_tiles(dj[i].lut.g, unal, kLutThreads);
+      const uint64_t slots = 4 * static_cast<uint64_t>(sm_count() * c.kern.ctas);
+      const uint64_t per = std::max<uint64_t>(1, std::min<uint64_t>(tile, (total + slots - 1) / slots));
+      // Stripes of one plan and of the byte tables' shape, but with sources at
+      // different offsets: one launch per kUniformJobs stripes, so that such a
+      // submission counts the same launches whatever its alignment.
+      bool one_plan = jobs[c.jobs[0]].byte_tab != nullptr;
+      for (uint32_t i : c.jobs) one_plan = one_plan && jobs[i].byte_tab == jobs[c.jobs[0]].byte_tab;
+      for (size_t q = 0; q < c.jobs.size(); ++q) {
+        const uint32_t i = c.jobs[q];
+        if (one_plan && q && q % kUniformJobs == 0) c.cuts.push_back(c.items.size());
+        LutBatchJob& J = dj[i].lut;
+        J.parts = static_cast<uint32_t>((lut_tiles(J.g, unal, kLutThreads) + per - 1) / per);
+        const uint32_t n = J.parts + (lut_has_edges(J.g, unal) ? 1u : 0u);
+        for (uint32_t p = 0; p < n; ++p) c.items.push_back(make_uint2(i, p));
       }
+      continue;
+    }
+    c.uniform = true;
+    for (uint32_t i : c.jobs) c.uniform = c.uniform && jobs[i].byte_tab == jobs[c.jobs[0]].byte_tab;
+    if (c.uniform) continue;
+    for (uint32_t i : c.jobs) {
+      // vectors: the segmented launch; scalar heads and tails: work items
+      BatchJob& J = dj[i].byte;
+      const uint64_t tail = J.len - J.head - 16 * J.nvec;
+      const uint64_t ngroups = (J.head + 3) / 4 + (tail + 3) / 4;
+      const uint64_t ns_items = (ngroups + kFastGroupsPerItem - 1) / kFastGroupsPerItem;
+      J.nv_items = static_cast<uint32_t>((J.nvec + kFastVecPerItem - 1) / kFastVecPerItem);
+      if (J.nvec) {
+        if (c.seg_prefix.empty()) c.seg_prefix.push_back(0);
+        c.seg_jobs.push_back(i);
+        c.seg_prefix.push_back(c.seg_prefix.back() + J.nvec);
+      }
+      for (uint64_t p = J.nv_items; p < J.nv_items + ns_items; ++p)
+        c.items.push_back(make_uint2(i, static_cast<unsigned>(p)));
     }
   }
 
   // ---- blob: jobs | ptrs | per work-list class: items, counter
   size_t off = 0;
   const size_t off_jobs = off;
-  off = align16(off + dj.size() * sizeof(BatchJob));
+  off = align16(off + dj.size() * sizeof(BatchDesc));
   const size_t off_ptrs = off;
   off = align16(off + ptrs.size() * sizeof(uint64_t));
   std::vector<std::pair<size_t, size_t>> cb;  // (items, counter) offsets
@@ -1042,7 +633,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       x.first = off;
       off = align16(off + kv.second.items.size() * sizeof(uint2));
       x.second = off;
-      off = align16(off + 64);
+      off = align16(off + std::max<size_t>(64, 4 * (kv.second.cuts.size() + 1)));
       if (!kv.second.seg_jobs.empty()) {
         y.first = off;
         off = align16(off + kv.second.seg_jobs.size() * sizeof(uint32_t));
@@ -1094,7 +685,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   }
   e = ensure_slot(s, bytes);
   if (e != cudaSuccess) return e;
-  std::memcpy(s.host + off_jobs, dj.data(), dj.size() * sizeof(BatchJob));
+  std::memcpy(s.host + off_jobs, dj.data(), dj.size() * sizeof(BatchDesc));
   std::memcpy(s.host + off_ptrs, ptrs.data(), ptrs.size() * sizeof(uint64_t));
   {
     size_t ci = 0;
@@ -1103,7 +694,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       const auto& x = cb[ci++];
       if (kv.second.uniform) continue;
       std::memcpy(s.host + x.first, kv.second.items.data(), kv.second.items.size() * sizeof(uint2));
-      std::memset(s.host + x.second, 0, 64);
+      std::memset(s.host + x.second, 0, std::max<size_t>(64, 4 * (kv.second.cuts.size() + 1)));
       if (!kv.second.seg_jobs.empty()) {
         std::memcpy(s.host + y.first, kv.second.seg_jobs.data(), kv.second.seg_jobs.size() * sizeof(uint32_t));
         std::memcpy(s.host + y.second, kv.second.seg_prefix.data(), kv.second.seg_prefix.size() * sizeof(uint64_t));
@@ -1128,6 +719,8 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // ---- launches (their structure is the graph key)
   struct Launch {
     KernelFn fn = nullptr;
+    LutBatchFn lfn = nullptr;
+    uint32_t kc = 0;
     UniformFn ufn = nullptr;
     unsigned grid = 0, threads = 0;
     uint32_t smem = 0;
@@ -1152,17 +745,28 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     const auto& x = cb[ci++];
     const bool fast = c.K > 0;
     Launch L;
-    const int akey = kv.first + (c.uniform ? 100 : 0);
+    const int akey = kv.first + (c.uniform ? 10000 : 0);
     if (c.uniform) {
       L.ufn = uniform_kernel_for(c.K, c.shift);
+    } else if (fast) {
+      L.fn = fast_kernel_for(c.K, c.shift);
     } else {
-      L.fn = fast ? fast_kernel_for(c.K, c.shift) : c.kara ? kernel_for_k16(c.G, c.shift) : kernel_for(c.E, c.G, c.shift);
+      L.lfn = c.kern.fn;
     }
-    if (!L.fn && !L.ufn) return cudaErrorInvalidValue;
-    L.smem = fast ? fast_smem(c.K) : static_cast<uint32_t>(kBatchSmem);
-    L.threads = fast ? static_cast<unsigned>(kFastThreads) : static_cast<unsigned>(kThreads);
-    e = ensure_smem_attr(L.ufn ? reinterpret_cast<const void*>(L.ufn) : reinterpret_cast<const void*>(L.fn),
-                         static_cast<int>(L.smem));
+    if (!L.fn && !L.ufn && !L.lfn) return cudaErrorInvalidValue;
+    if (fast) {
+      L.smem = fast_smem(c.K);
+      L.threads = static_cast<unsigned>(kFastThreads);
+    } else {
+      for (uint32_t i : c.jobs)
+        L.smem = std::max(L.smem, lut_smem(c.shape, std::min<size_t>(jobs[i].k, c.kc)));
+      L.threads = static_cast<unsigned>(kLutThreads);
+      L.kc = static_cast<uint32_t>(c.kc);
+    }
+    e = ensure_smem_attr(L.ufn   ? reinterpret_cast<const void*>(L.ufn)
+                         : L.lfn ? reinterpret_cast<const void*>(L.lfn)
+                                 : reinterpret_cast<const void*>(L.fn),
+                         L.lfn ? kLutSmemMax : static_cast<int>(L.smem));
     if (e != cudaSuccess) return e;
     if (c.uniform) {
       // one launch per block of kUniformJobs stripes
@@ -1171,24 +775,22 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         uparams.emplace_back();
         UniformParams& P = uparams.back();
         std::memset(&P, 0, sizeof P);
-        const BatchJob& J0 = dj[c.jobs[q0]];
-        P.tables = J0.tables;
-        P.gstride = J0.gstride;
-        P.g0 = J0.g0;
+        P.tables = dj[c.jobs[q0]].byte.tables;
         P.njobs = static_cast<uint32_t>(nq);
         for (size_t q = 0; q < nq; ++q) {
           const LoweredJob& LJ = jobs[c.jobs[q0 + q]];
+          const BatchJob& J = dj[c.jobs[q0 + q]].byte;
           UJob& U = P.jobs[q];
           for (size_t t = 0; t < LJ.k; ++t) U.src[t] = reinterpret_cast<const uint8_t*>(LJ.srcs[t]);
           for (size_t rr = 0; rr < 4; ++rr) U.dst[rr] = reinterpret_cast<uint8_t*>(LJ.dsts[rr < LJ.nrows ? rr : 0]);
-          U.len = LJ.len;
-          U.head = LJ.head;
-          U.nvec = LJ.nvec;
+          U.len = J.len;
+          U.head = J.head;
+          U.nvec = J.nvec;
           U.nrows = static_cast<uint32_t>(LJ.nrows);
           U.ovr = LJ.ovr ? 1u : 0u;
-          const uint64_t tail = LJ.len - LJ.head - 16 * LJ.nvec;
-          P.vprefix[q + 1] = P.vprefix[q] + LJ.nvec;
-          P.gprefix[q + 1] = P.gprefix[q] + (LJ.head + 3) / 4 + (tail + 3) / 4;
+          const uint64_t tail = J.len - J.head - 16 * J.nvec;
+          P.vprefix[q + 1] = P.vprefix[q] + J.nvec;
+          P.gprefix[q + 1] = P.gprefix[q] + (J.head + 3) / 4 + (tail + 3) / 4;
         }
         Launch U = L;
         const uint64_t want = (std::max(P.vprefix[nq], P.gprefix[nq]) + L.threads - 1) / L.threads;
@@ -1220,13 +822,18 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         launches.push_back(S);
       }
       if (!c.items.empty()) {
-        L.n = static_cast<uint32_t>(c.items.size());
-        L.grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((L.n + kClaim - 1) / kClaim, sms)));
-        L.items = reinterpret_cast<const uint2*>(s.dev + x.first);
-        L.counter = reinterpret_cast<uint32_t*>(s.dev + x.second);
+        for (size_t q = 0; q <= c.cuts.size(); ++q) {
+          const size_t i0 = q ? c.cuts[q - 1] : 0, i1 = q < c.cuts.size() ? c.cuts[q] : c.items.size();
+          L.n = static_cast<uint32_t>(i1 - i0);
+          L.grid = L.lfn ? static_cast<unsigned>(std::min<uint64_t>(L.n, static_cast<uint64_t>(sms) * c.kern.ctas))
+                         : static_cast<unsigned>(std::min<uint64_t>((L.n + kClaim - 1) / kClaim, sms));
+          L.items = reinterpret_cast<const uint2*>(s.dev + x.first) + i0;
+          L.counter = reinterpret_cast<uint32_t*>(s.dev + x.second) + q;
+          key += "|" + std::to_string(akey) + "," + std::to_string(L.n) + "," + std::to_string(L.grid) + "," +
+                 std::to_string(L.smem);
+          launches.push_back(L);
+        }
         b->last_items += c.items.size();
-        key += "|" + std::to_string(akey) + "," + std::to_string(L.n) + "," + std::to_string(L.grid);
-        launches.push_back(L);
       }
     }
   }
@@ -1242,7 +849,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
            std::to_string(tcg[g].nblk);
     launches.push_back(L);
   }
-  const BatchJob* djobs = reinterpret_cast<const BatchJob*>(s.dev + off_jobs);
+  const BatchDesc* djobs = reinterpret_cast<const BatchDesc*>(s.dev + off_jobs);
   const uint64_t* dptrs = reinterpret_cast<const uint64_t*>(s.dev + off_ptrs);
 
   const int nside = launches.size() > 1 ? static_cast<int>(std::min<size_t>(launches.size(), kSideStreams)) : 0;
@@ -1281,6 +888,9 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         err = cudaGetLastError();
       } else if (L.sfn) {
         L.sfn<<<L.grid, L.threads, L.smem, ls>>>(djobs, dptrs, L.seg_jobs, L.seg_prefix, L.n);
+        err = cudaGetLastError();
+      } else if (L.lfn) {
+        L.lfn<<<L.grid, L.threads, L.smem, ls>>>(djobs, dptrs, L.items, L.n, L.counter, L.kc);
         err = cudaGetLastError();
       } else {
         L.fn<<<L.grid, L.threads, L.smem, ls>>>(djobs, dptrs, L.items, L.n, L.counter);
@@ -1350,10 +960,13 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
 // call would first have to wait on an event recorded after the previous copy.)
 //
 // Stripes are grouped in classes as in fgfc_batch_run: Gf8 stripes of at most
-// 4 rows and at most 14 sources run the byte-table kernel for their source
-// count; the rest run the split-nibble kernel for their own number of table
-// groups, so a wide stripe does not widen the others. One launch per class,
-// in order, on the caller's stream.
+// 4 rows and at most 14 sources at one offset run the byte-table kernel for
+// their source count; the rest run the table kernel of their element width,
+// tower split, output words and alignment. One launch per class, in order, on
+// the caller's stream. The scratch limit counts a stripe's tables and items at
+// 128 bytes per (source byte, 4 output bytes) and 4096 columns or 2 KiB of
+// head and tail per item; what is stored (32-byte images, fewer items) fits in
+// that.
 
 static __device__ __align__(256) uint8_t g_noalloc_scratch[FGFC_NOALLOC_SCRATCH_BYTES];
 alignas(256) static uint8_t g_noalloc_host[FGFC_NOALLOC_SCRATCH_BYTES];
@@ -1363,14 +976,16 @@ static uint8_t* g_noalloc_dev[kNoallocMaxDevices];  // device address of the arr
 
 namespace {
 
-// Class of a stripe in fgfc_batch_run_noalloc: 1..14 = byte-table kernel
-// with that many sources, 100 + G = nibble kernel with G table groups.
+// Class of a stripe for the scratch limit: 1..14 = byte-table kernel with that
+// many sources, 100 + G = G groups of 4 output bytes.
 int noalloc_class(int E, size_t nsrcs, size_t nrows) {
   const int R = 4 / E;
   const size_t G = (nrows + R - 1) / R;
   if (E == 1 && G == 1 && nsrcs >= 1 && nsrcs <= static_cast<size_t>(kFastMaxK)) return static_cast<int>(nsrcs);
   return 100 + static_cast<int>(G);
 }
+constexpr uint32_t kNoallocCols = 4096;   // columns per item
+constexpr uint32_t kNoallocGroups = 512;  // 4-byte groups per item of the limit
 
 }  // namespace
 
@@ -1430,12 +1045,12 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
     nptr += J.nsrcs + J.nrows;
     ntab += J.nsrcs * E * G * kCompactWords;
     const uint64_t nvec = J.row_len / 16 + 1;  // upper bound before alignment is known
-    const uint64_t per_vec = fast ? kFastVecPerItem : kVecPerItem;
-    const uint64_t per_grp = fast ? kFastGroupsPerItem : kGroupsPerItem;
+    const uint64_t per_vec = fast ? kFastVecPerItem : kNoallocCols;
+    const uint64_t per_grp = fast ? kFastGroupsPerItem : kNoallocGroups;
     class_items[cls] += (nvec + per_vec - 1) / per_vec + (J.row_len / 4 + 2 + per_grp - 1) / per_grp + 1;
   }
   const size_t off_jobs = 0;
-  const size_t off_ptrs = align16(off_jobs + nlive * sizeof(BatchJob));
+  const size_t off_ptrs = align16(off_jobs + nlive * sizeof(BatchDesc));
   const size_t off_tabs = align16(off_ptrs + nptr * sizeof(uint64_t));
   size_t class_off[kClasses] = {0};
   size_t off = align16(off_tabs + ntab * sizeof(uint32_t));
@@ -1452,11 +1067,15 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
   }
 
   // ---- blob in the host array
-  BatchJob* hj = reinterpret_cast<BatchJob*>(g_noalloc_host + off_jobs);
+  BatchDesc* hj = reinterpret_cast<BatchDesc*>(g_noalloc_host + off_jobs);
   uint64_t* hp = reinterpret_cast<uint64_t*>(g_noalloc_host + off_ptrs);
   uint32_t* ht = reinterpret_cast<uint32_t*>(g_noalloc_host + off_tabs);
   size_t jn = 0, pn = 0, tn = 0;
-  size_t class_n[kClasses] = {0};
+  // Launches of a class: [0] stripes at one offset (byte-table kernel where the
+  // class has it), [1] the others, whose items fill the class's list from its end.
+  size_t class_n[kClasses][2] = {{0}};
+  uint32_t class_smem[kClasses][2] = {{0}};
+  size_t class_rows[kClasses] = {0};
   for (size_t i = 0; i < njobs; ++i) {
     const fgfc_noalloc_job& S = jobs[i];
     if (S.nrows == 0 || S.row_len == 0) continue;
@@ -1474,48 +1093,55 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
     }
     const size_t G = (S.nrows + R - 1) / R;
     const int cls = noalloc_class(E, S.nsrcs, S.nrows);
-    const bool fast = cls < 100;
-    BatchJob& J = hj[jn];
-    const uintptr_t al = reinterpret_cast<uintptr_t>(S.srcs[0].ptr) & 15;
-    bool same = (al % E) == 0;
-    J.src_idx = static_cast<uint32_t>(pn);
-    for (size_t t = 0; t < S.nsrcs; ++t) {
-      hp[pn] = reinterpret_cast<uint64_t>(S.srcs[t].ptr);
-      same = same && (hp[pn] & 15) == al;
-      ++pn;
-    }
-    J.dst_idx = static_cast<uint32_t>(pn);
-    for (size_t j = 0; j < S.nrows; ++j) {
-      hp[pn] = reinterpret_cast<uint64_t>(S.dst + (S.row_starts ? S.row_starts[j] : j * S.row_len));
-      same = same && (hp[pn] & 15) == al;
-      ++pn;
-    }
-    J.len = S.row_len;
-    J.head = S.row_len;
-    J.nvec = 0;
-    if (same) {
-      J.head = std::min<uint64_t>((16 - al) & 15, S.row_len);
-      J.nvec = (S.row_len - J.head) / 16;
-    }
+    const uint32_t src_idx = static_cast<uint32_t>(pn);
+    for (size_t t = 0; t < S.nsrcs; ++t) hp[pn++] = reinterpret_cast<uint64_t>(S.srcs[t].ptr);
+    const uint32_t dst_idx = static_cast<uint32_t>(pn);
+    for (size_t j = 0; j < S.nrows; ++j)
+      hp[pn++] = reinterpret_cast<uint64_t>(S.dst + (S.row_starts ? S.row_starts[j] : j * S.row_len));
+    const JobAlign al = job_align(field, hp + src_idx, S.nsrcs, hp + dst_idx, S.nrows, S.row_len);
+    const int var = al.unal ? 1 : 0;
+    const bool fast = cls < 100 && !al.unal;
     uint64_t cm[kMaxSrc * 16];  // coefficients reduced to the field's width, as Plan::matrix does
     for (size_t q = 0; q < S.nsrcs * S.nrows; ++q) cm[q] = S.coeffs[q] & field_mask(field);
-    build_compact_tables(field, cm, S.nrows, 0, S.nsrcs, 0, G, ht + tn);
-    J.tables = reinterpret_cast<const uint32_t*>(dbase + off_tabs) + tn;
+    const uint32_t* tables = reinterpret_cast<const uint32_t*>(dbase + off_tabs) + tn;
+    uint64_t nitems;
+    if (fast) {
+      build_compact_tables(field, cm, S.nrows, S.nsrcs, ht + tn);
+      BatchJob& J = hj[jn].byte;
+      J.tables = tables;
+      J.len = S.row_len;
+      J.head = al.head;
+      J.nvec = (S.row_len - al.head) / 16;
+      J.k = static_cast<uint32_t>(S.nsrcs);
+      J.nrows = static_cast<uint32_t>(S.nrows);
+      J.ovr = S.overwrite ? 1u : 0u;
+      J.src_idx = src_idx;
+      J.dst_idx = dst_idx;
+      const uint64_t tail = J.len - J.head - 16 * J.nvec;
+      J.nv_items = static_cast<uint32_t>((J.nvec + kFastVecPerItem - 1) / kFastVecPerItem);
+      nitems = J.nv_items + ((J.head + 3) / 4 + (tail + 3) / 4 + kFastGroupsPerItem - 1) / kFastGroupsPerItem;
+      class_smem[cls][var] = fast_smem(cls);
+    } else {
+      build_lut_images(field, cm, S.nrows, 0, S.nsrcs, 0, S.nrows, ht + tn);
+      LutBatchJob& J = hj[jn].lut;
+      J = lut_batch_job(field, tables, al, S.row_len, S.nsrcs, S.nrows, S.overwrite != 0);
+      J.src_idx = src_idx;
+      J.dst_idx = dst_idx;
+      const uint64_t per = kNoallocCols / kLutThreads;
+      J.parts = static_cast<uint32_t>((lut_tiles(J.g, al.unal, kLutThreads) + per - 1) / per);
+      nitems = J.parts + (lut_has_edges(J.g, al.unal) ? 1 : 0);
+      class_smem[cls][var] = std::max(class_smem[cls][var],
+                                      lut_smem(lut_shape(E, S.nrows),
+                                               std::min(S.nsrcs, lut_sources(E, S.nrows, false))));
+    }
     tn += S.nsrcs * E * G * kCompactWords;
-    J.gstride = static_cast<uint32_t>(G);
-    J.g0 = 0;
-    J.k = static_cast<uint32_t>(S.nsrcs);
-    J.nrows = static_cast<uint32_t>(S.nrows);
-    J.ovr = S.overwrite ? 1u : 0u;
-    const uint64_t per_vec = fast ? kFastVecPerItem : kVecPerItem;
-    const uint64_t per_grp = fast ? kFastGroupsPerItem : kGroupsPerItem;
-    const uint64_t nv_items = (J.nvec + per_vec - 1) / per_vec;
-    const uint64_t tail = J.len - J.head - 16 * J.nvec;
-    const uint64_t ns_items = ((J.head + 3) / 4 + (tail + 3) / 4 + per_grp - 1) / per_grp;
-    J.nv_items = static_cast<uint32_t>(nv_items);
-    uint2* hi = reinterpret_cast<uint2*>(g_noalloc_host + class_off[cls]);
-    for (uint64_t q = 0; q < nv_items + ns_items; ++q)
-      hi[class_n[cls]++] = make_uint2(static_cast<unsigned>(jn), static_cast<unsigned>(q));
+    uint2* list = reinterpret_cast<uint2*>(g_noalloc_host + class_off[cls]);
+    for (uint64_t q = 0; q < nitems; ++q) {
+      const size_t at = var ? class_items[cls] - 1 - class_n[cls][1] : class_n[cls][0];
+      list[at] = make_uint2(static_cast<unsigned>(jn), static_cast<unsigned>(q));
+      ++class_n[cls][var];
+    }
+    class_rows[cls] = S.nrows;  // any of the class: they share a table shape
     ++jn;
   }
   if (jn == 0) return 0;
@@ -1525,27 +1151,35 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
   // ---- one copy, then one launch of the work-list kernel per class
   e = cudaMemcpyAsync(dbase, g_noalloc_host, bytes, cudaMemcpyHostToDevice, stream);
   for (int c = 0; c < kClasses && e == cudaSuccess; ++c) {
-    if (!class_n[c]) continue;
-    const bool fast = c < 100;
-    // rows share the sources' alignment here (otherwise the whole stripe is scalar)
-    KernelFn fn = fast ? fast_kernel_for(c, false) : kernel_for(E, c - 100, false);
-    const int smem = fast ? static_cast<int>(fast_smem(c)) : static_cast<int>(kBatchSmem);
-    const unsigned threads = fast ? static_cast<unsigned>(kFastThreads) : static_cast<unsigned>(kThreads);
-    if (!fn) {
-      e = cudaErrorInvalidValue;
-      break;
+    for (int var = 0; var < 2 && e == cudaSuccess; ++var) {
+      const size_t n = class_n[c][var];
+      if (!n) continue;
+      const bool fast = c < 100 && var == 0;
+      const KernelFn fn = fast ? fast_kernel_for(c, false) : nullptr;
+      const LutBatchKernel lut = fast ? LutBatchKernel{} : lut_batch_kernel_for(E, lut_shape(E, class_rows[c]), var != 0);
+      if (!fn && !lut.fn) {
+        e = cudaErrorInvalidValue;
+        break;
+      }
+      const uint32_t smem = class_smem[c][var];
+      e = ensure_smem_attr(fast ? reinterpret_cast<const void*>(fn) : reinterpret_cast<const void*>(lut.fn),
+                           fast ? static_cast<int>(smem) : kLutSmemMax);
+      if (e != cudaSuccess) break;
+      const BatchDesc* descs = reinterpret_cast<const BatchDesc*>(dbase + off_jobs);
+      const uint64_t* ptrs = reinterpret_cast<const uint64_t*>(dbase + off_ptrs);
+      const uint2* list = reinterpret_cast<const uint2*>(dbase + class_off[c]) + (var ? class_items[c] - n : 0);
+      uint32_t* counter =
+          reinterpret_cast<uint32_t*>(dbase + align16(class_off[c] + class_items[c] * sizeof(uint2))) + var;
+      const uint64_t sms = static_cast<uint64_t>(sm_count());
+      if (fast)
+        fn<<<static_cast<unsigned>(std::min<uint64_t>((n + kClaim - 1) / kClaim, sms)), kFastThreads, smem, stream>>>(
+            descs, ptrs, list, static_cast<uint32_t>(n), counter);
+      else
+        lut.fn<<<static_cast<unsigned>(std::min<uint64_t>(n, sms * lut.ctas)), kLutThreads, smem, stream>>>(
+            descs, ptrs, list, static_cast<uint32_t>(n), counter,
+            static_cast<uint32_t>(lut_sources(E, class_rows[c], false)));
+      e = cudaGetLastError();
     }
-    e = ensure_smem_attr(reinterpret_cast<const void*>(fn), smem);
-    if (e != cudaSuccess) break;
-    const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((class_n[c] + kClaim - 1) / kClaim, sm_count()));
-    const size_t items_off = class_off[c];
-    const size_t counter_off = align16(class_off[c] + class_items[c] * sizeof(uint2));
-    fn<<<grid, threads, smem, stream>>>(reinterpret_cast<const BatchJob*>(dbase + off_jobs),
-                                        reinterpret_cast<const uint64_t*>(dbase + off_ptrs),
-                                        reinterpret_cast<const uint2*>(dbase + items_off),
-                                        static_cast<uint32_t>(class_n[c]),
-                                        reinterpret_cast<uint32_t*>(dbase + counter_off));
-    e = cudaGetLastError();
   }
   if (e != cudaSuccess) {
     snprintf(msg, msglen, "batch_run_noalloc: CUDA error: %s", cudaGetErrorString(e));

@@ -55,19 +55,17 @@ struct FastLayout {
   static constexpr uint32_t smem = tables + K * kCompactWords * 4u;  // + compact staging
 };
 
-// Expand the compact tables of K sources (plan layout: source t at
-// ((t * gstride + g0) * 32)) into the byte-table layout. `tables` is a device
+// Expand the compact tables of K sources (32 words each) into the byte-table
+// layout. `tables` is a device
 // pointer, or null to read `inl` (launch parameters). The compact words are
 // staged in shared memory first (one independent load per thread) and every
 // entry's 32 lane copies are written as 8 identical 16-byte stores.
 template <int K>
-__device__ __forceinline__ void fill_fast(const uint32_t* tables, const uint32_t* inl, uint32_t gstride,
-                                          uint32_t g0) {
+__device__ __forceinline__ void fill_fast(const uint32_t* tables, const uint32_t* inl) {
   using L = FastLayout<K>;
   uint32_t* stage = reinterpret_cast<uint32_t*>(g_smem) + L::tables / 4;
   for (uint32_t i = threadIdx.x; i < K * kCompactWords; i += blockDim.x) {
-    const uint32_t src = ((i >> 5) * gstride + g0) * kCompactWords + (i & 31u);
-    stage[i] = tables ? __ldg(tables + src) : inl[src];
+    stage[i] = tables ? __ldg(tables + i) : inl[i];
   }
   __syncthreads();
   // byte tables: word index = page * 16384 + x * 64 + half * 32 + lane

@@ -16,18 +16,14 @@ namespace fgfc {
 // into several launches by the host (exact: rows are independent, and
 // sources split into an overwrite launch followed by accumulate launches).
 constexpr int kMaxSrc = 64;
-// One nibble table slot: 16 rows x 256 bytes. Each row holds 32 lane copies
-// of the lo-nibble word (bytes 0..127) and of the hi-nibble word (128..255),
-// so a warp's 32 lookups hit 32 distinct banks.
+// One nibble table slot of the byte-table kernels: 16 rows x 256 bytes. Each
+// row holds 32 lane copies of the lo-nibble word (bytes 0..127) and of the
+// hi-nibble word (128..255).
 constexpr int kSlotBytes = 4096;
-constexpr int kMaxSlots = 54;            // 216 KiB of tables (+ 6.75 KiB staging) per CTA
-constexpr int kCompactWords = 32;        // 16 lo + 16 hi words per slot
 constexpr size_t kFastMaxSources = 14;   // byte-table kernels: sources per launch
-
-// A compact table slot for (source t, source byte-plane p, row group g):
-// word[n] (n < 16) = products of the lo nibble value n, word[16 + n] =
-// products of (n << 4); byte q of each word is output byte (q % E) of row
-// (g * R + q / E), R = 4 / E rows per group.
+// Their compact tables, per source: word[n] (n < 16) = products of the low
+// nibble value n, word[16 + n] = products of n << 4; byte q is row q.
+constexpr int kCompactWords = 32;
 
 struct MatrixLaunch {
   uint64_t head;           // bytes before the vector body
@@ -41,17 +37,8 @@ struct MatrixLaunch {
   uint32_t inline_tab[kFastMaxSources * kCompactWords];
 };
 
-// Build compact tables for sources [t0, t0+k) and groups [g0, g0+G) of a
-// coefficient matrix (term-major: coeffs[t * m + j]). Output layout
-// [(t * E + p) * G + g][32].
-void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k,
-                          size_t g0, size_t G, uint32_t* out);
-
-// The same split for Gf16 = Gf8B[u]/(u^2 + u + 0x20): lo = A + 0x20 B,
-// hi = A + C over byte half-products. Tables for the batched work lists:
-// [(t * 3 + P) * Gq + q][32], nibble tables whose word holds the byte
-// half-product P of rows 4q .. 4q + 3 (zero past m); Gq = ceil(m / 4).
-void build_kara16_tables(const uint64_t* coeffs, size_t m, size_t k, size_t Gq, uint32_t* out);
+// Compact tables of a term-major k x m (m <= 4) matrix over a 1-byte field.
+void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t k, uint32_t* out);
 
 // ---------------------------------------------------------------- table kernels (lut.cuh)
 
@@ -67,6 +54,36 @@ struct LutGeom {
   uint32_t bytes;  // unaligned in-place job: columns are read and written bytewise
 };
 
+constexpr uint32_t kEdges = 5;  // edge columns of a job
+// First block an unaligned job's vector path writes: columns 0 and 1 and the
+// last two whole ones are edges (a source's granules may reach past them).
+constexpr uint64_t kUnalFirst = 2;
+// A warp of an unaligned job takes 32 columns and writes 30 blocks: lane 0's
+// column only supplies the bytes before lane 1's, and lane 31's 16 source
+// bytes only complete lane 30's.
+constexpr uint32_t kUnalStep = 30;
+#ifdef __CUDACC__
+#define FGFC_HD __host__ __device__
+#else
+#define FGFC_HD
+#endif
+// Blocks of an unaligned job's vector path: v = kUnalFirst .. ncol - 2.
+FGFC_HD inline uint64_t lut_unal_blocks(uint64_t ncol) { return ncol >= 4 ? ncol - 3 : 0; }
+// Does the job leave bytes to the edge pass?
+FGFC_HD inline bool lut_has_edges(const LutGeom& g, bool unal) {
+  if (unal) return !g.bytes;
+  return g.head != 0 || g.head + 16 * g.ncol != g.len;
+}
+// Tiles of a job for CTAs of `threads`: a column per thread, 30 blocks per
+// warp of an unaligned job.
+FGFC_HD inline uint64_t lut_tiles(const LutGeom& g, bool unal, uint32_t threads) {
+  if (!unal) return (g.ncol + threads - 1) / threads;
+  if (g.bytes) return (g.len + 16 * threads - 1) / (16 * threads);
+  const uint32_t step = threads / 32 * kUnalStep;
+  return (lut_unal_blocks(g.ncol) + step - 1) / step;
+}
+
+constexpr int kLutThreads = 256;
 constexpr int kLutRows = 16;               // rows per launch (Gf8; 8 / 4 / 4 for 2, 4 and 8 bytes)
 constexpr int kLutInlineWords = 1536;      // images carried in launch parameters
 constexpr int kLutSmemMax = 110 * 1024;    // tables of one CTA: two CTAs per SM
@@ -87,7 +104,12 @@ struct LutShape {
   size_t nv;  // leaf input bytes per element
   size_t src_words() const { return nv * static_cast<size_t>(w) * 8; }  // image words per source
   size_t smem3() const { return (nv * w * 640 + 255) / 256 * 256; }     // table bytes of three sources
+  size_t smem1() const { return (nv * w * 128 + 255) / 256 * 256; }     // and of one left over
 };
+// Shared memory of one CTA: tables of k sources and the staged edge columns.
+inline uint32_t lut_smem(const LutShape& s, size_t k) {
+  return static_cast<uint32_t>(k / 3 * s.smem3() + k % 3 * s.smem1() + k * kEdges * 16);
+}
 inline size_t lut_rows(int E) { return E == 1 ? 16 : E == 2 ? 8 : 4; }
 LutShape lut_shape(int E, size_t nr);
 // Sources per launch: table pages, pointers and (raw forms) inline images fit.
@@ -100,6 +122,40 @@ void build_lut_images(int field, const uint64_t* coeffs, size_t m, size_t t0, si
                       uint32_t* out);
 // Launch one job (rows of one lut_shape); `unal` as LutGeom describes.
 cudaError_t lut_launch(int field, size_t nr, LutArgs& a, bool unal, bool edges_only, cudaStream_t s);
+// One descriptor of a batched submission: a byte-table sub-job (batch.cu) or a
+// table sub-job (lut_batch.cuh).
+struct BatchJob {
+  const uint32_t* tables;  // compact tables [source][32]
+  uint64_t len;            // bytes per row
+  uint64_t head;           // scalar bytes before the vector body
+  uint64_t nvec;           // 16-byte vectors in the body
+  uint32_t k, nrows;       // sources; rows of this sub-job
+  uint32_t ovr;            // 1 = overwrite
+  uint32_t src_idx, dst_idx;
+  uint32_t nv_items;       // vector items; scalar items follow
+};
+struct LutBatchJob {
+  const uint32_t* img;
+  LutGeom g;
+  uint32_t src_idx, dst_idx;
+  uint32_t parts;  // items over the tiles; one item of edges follows
+  uint32_t fp;
+};
+union BatchDesc {
+  BatchJob byte;
+  LutBatchJob lut;
+};
+static_assert(sizeof(BatchDesc) == 64, "the no-allocation scratch limit counts 64 bytes per stripe");
+using LutBatchFn = void (*)(const BatchDesc*, const uint64_t*, const uint2*, uint32_t, uint32_t*, uint32_t);
+struct LutBatchKernel {
+  LutBatchFn fn = nullptr;
+  int ctas = 1;  // resident per SM
+};
+LutBatchKernel lut_batch_kernel_for(int E, LutShape s, bool unal);
+LutBatchKernel lut_batch_e1(int lev, int w, bool unal);
+LutBatchKernel lut_batch_e2(int lev, int w, bool unal);
+LutBatchKernel lut_batch_e4(int lev, int w, bool unal);
+LutBatchKernel lut_batch_e8(int lev, int w, bool unal);
 cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
 cudaError_t lut_launch_e2(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
 cudaError_t lut_launch_e4(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
@@ -154,20 +210,24 @@ int gf2mma_error(bool clear);
 cudaError_t ensure_smem_attr(const void* fn, int bytes);
 
 // One lowered sub-job of a batched submission: all sources of a stripe and
-// the rows of at most 4 table groups, with its alignment split resolved.
+// the rows of one table launch.
 struct LoweredJob {
   int field;
-  const uint32_t* tables;  // plan compact tables, matrix orientation
-  size_t gstride;          // plan groups per (source, plane)
-  size_t g0;               // first group of this sub-job
-  size_t G;                // groups in this sub-job (1..4)
-  uint64_t len, head, nvec;
+  const uint32_t* img;       // plan images of these rows
+  const uint32_t* byte_tab;  // plan byte-table tables, or nullptr (not their shape)
+  uint64_t len;
   size_t k, nrows;
   bool ovr;
-  bool shift;              // some row is not at the sources' offset within 16 bytes
-  bool kara = false;       // Gf16 by byte half-products (tables: build_kara16_tables; G = row quads)
   std::vector<uint64_t> srcs, dsts;
 };
+// How the sub-job's pointers sit within 16 bytes.
+struct JobAlign {
+  bool sources;   // every source at one offset, whole elements before the boundary
+  bool unal;      // a source or row is elsewhere
+  bool overlap;   // a row shares bytes with a source
+  uint64_t head;  // bytes before the sources' first boundary
+};
+JobAlign job_align(int field, const uint64_t* srcs, size_t k, const uint64_t* dsts, size_t m, uint64_t len);
 
 // One stripe's 16-byte-aligned body for the tensor-core kernel in a batch:
 // its k sources and m rows already offset to the body start, nblk blocks of

@@ -26,7 +26,7 @@ namespace {
 
 template <int K, bool OVR, bool SHIFT>
 __global__ void __launch_bounds__(kFastThreads, 1) matrix_fast_kernel(const __grid_constant__ MatrixLaunch a) {
-  fill_fast<K>(a.tables, a.inline_tab, 1, 0);
+  fill_fast<K>(a.tables, a.inline_tab);
   const FastRegs r;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   const uint32_t lane = threadIdx.x & 31u;

@@ -29,6 +29,8 @@
 // index masks). Measured on B200 against the kernels it replaced, with 32
 // table copies per lane (or unreplicated nibbles for 8-byte elements):
 //   GF(2^64) RS(10,4), 16 MiB shards     308 -> 206 us (lookups per element 992 -> 483)
+//   256 stripes of Gf8D and Gf16, k 4..32, m 1..8, 4 KiB .. 4 MiB, one batch
+//                                        3260 -> 1711 us (more CTAs resident, no 216 KiB refills)
 //   Gf8D RS(12,4), 1000003-byte shards at any offset, 18 -> 4 us on the device
 //   (whole-element bytes one at a time before, 16-byte granules spliced now)
 #pragma once
@@ -363,24 +365,6 @@ __device__ __forceinline__ uint4 lut_row(const uint32_t (&f)[L::NF], int r) {
 }
 
 // ---------------------------------------------------------------- one job
-
-constexpr uint32_t kEdges = 5;  // edge columns of a job
-// First block an unaligned job's vector path writes: columns 0 and 1 and the
-// last two whole ones are edges (a source's granules may reach past them).
-constexpr uint64_t kUnalFirst = 2;
-// A warp of an unaligned job takes 32 columns and writes 30 blocks: lane 0's
-// column only supplies the bytes before lane 1's, and lane 31's 16 source
-// bytes only complete lane 30's.
-constexpr uint32_t kUnalStep = 30;
-
-// Blocks of an unaligned job's vector path: v = kUnalFirst .. ncol - 2.
-__host__ __device__ inline uint64_t lut_unal_blocks(uint64_t ncol) { return ncol >= 4 ? ncol - 3 : 0; }
-
-// Does the job leave bytes to the edge pass?
-__host__ __device__ inline bool lut_has_edges(const LutGeom& g, bool unal) {
-  if (unal) return !g.bytes;
-  return g.head != 0 || g.head + 16 * g.ncol != g.len;
-}
 
 struct LutShared {
   const uint8_t* src[kMaxSrc];

@@ -1,5 +1,5 @@
 // lut_e1.cu -- the table kernels (lut.cuh) of the 1-byte fields.
-#include "lut_single.cuh"
+#include "lut_batch.cuh"
 
 namespace fgfc {
 
@@ -9,6 +9,14 @@ cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, bool unal,
   if (lev == 0 && w == 3) return lut_launch_lw<1, 0, 3>(a, s, unal, edges_only);
   if (lev == 0 && w == 4) return lut_launch_lw<1, 0, 4>(a, s, unal, edges_only);
   return cudaErrorInvalidValue;
+}
+
+LutBatchKernel lut_batch_e1(int lev, int w, bool unal) {
+  if (lev == 0 && w == 1) return lut_batch_lw<1, 0, 1>(unal);
+  if (lev == 0 && w == 2) return lut_batch_lw<1, 0, 2>(unal);
+  if (lev == 0 && w == 3) return lut_batch_lw<1, 0, 3>(unal);
+  if (lev == 0 && w == 4) return lut_batch_lw<1, 0, 4>(unal);
+  return LutBatchKernel{};
 }
 
 }  // namespace fgfc

@@ -1,5 +1,5 @@
 // lut_e2.cu -- the table kernels (lut.cuh) of the 2-byte fields.
-#include "lut_single.cuh"
+#include "lut_batch.cuh"
 
 namespace fgfc {
 
@@ -8,6 +8,13 @@ cudaError_t lut_launch_e2(int lev, int w, LutArgs& a, cudaStream_t s, bool unal,
   if (lev == 1 && w == 1) return lut_launch_lw<2, 1, 1>(a, s, unal, edges_only);
   if (lev == 1 && w == 2) return lut_launch_lw<2, 1, 2>(a, s, unal, edges_only);
   return cudaErrorInvalidValue;
+}
+
+LutBatchKernel lut_batch_e2(int lev, int w, bool unal) {
+  if (lev == 0 && w == 1) return lut_batch_lw<2, 0, 1>(unal);
+  if (lev == 1 && w == 1) return lut_batch_lw<2, 1, 1>(unal);
+  if (lev == 1 && w == 2) return lut_batch_lw<2, 1, 2>(unal);
+  return LutBatchKernel{};
 }
 
 }  // namespace fgfc

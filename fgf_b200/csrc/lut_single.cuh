@@ -6,8 +6,6 @@
 
 namespace fgfc {
 
-constexpr int kLutThreads = 256;
-
 // CTAs per SM the register budget is set for: accumulators (3^LEV leaf
 // products x W words x 16 / E elements) plus three sources and their packed words.
 template <int E, int LEV, int W, bool UNAL>
@@ -51,14 +49,7 @@ cudaError_t lut_launch_one(LutArgs& a, cudaStream_t s, bool edges_only) {
   const uint64_t cols = edges_only ? 0 : UNAL && !a.g.bytes ? lut_unal_blocks(a.g.ncol) * 32 / kUnalStep : a.g.len / 16;
   while (threads > 64 && cols < sms * threads) threads /= 2;
   a.edge_cta = edges ? 1u : 0u;
-  if (edges_only)
-    a.ntiles = 0;
-  else if (!UNAL)
-    a.ntiles = (a.g.ncol + threads - 1) / threads;
-  else if (a.g.bytes)
-    a.ntiles = (a.g.len + 16 * threads - 1) / (16 * threads);
-  else
-    a.ntiles = (lut_unal_blocks(a.g.ncol) + threads / 32 * kUnalStep - 1) / (threads / 32 * kUnalStep);
+  a.ntiles = edges_only ? 0 : lut_tiles(a.g, UNAL, threads);
   const uint64_t cap = sms * lut_min_ctas<E, LEV, W, UNAL>();
   const unsigned grid = static_cast<unsigned>(a.ntiles < cap ? a.ntiles : cap) + a.edge_cta;
   if (!grid) return cudaSuccess;

@@ -15,46 +15,15 @@ const Gf8Log& gf8d_tab() {
   return t;
 }
 
-void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k,
-                          size_t g0, size_t G, uint32_t* out) {
-  const int E = field_bytes(field);
-  for (size_t tt = 0; tt < k; ++tt) {
-    const size_t t = t0 + tt;
-    for (size_t g = 0; g < G; ++g) {
-      // The group's 4 output bytes are the flat output bytes
-      // f = 4 (g0 + g) + q of the m * E (row f / E, byte f % E); rows past m
-      // contribute zero products. Images per row this group touches.
-      uint64_t img[4][8][8];
-      size_t row[4];
-      int ri[4], ob[4];
-      int nr = 0;
-      for (int q = 0; q < 4; ++q) {
-        const size_t f = 4 * (g0 + g) + q;
-        const size_t j = f / E;
-        ob[q] = static_cast<int>(f % E);
-        ri[q] = -1;
-        if (j >= m) continue;
-        for (int r = 0; r < nr; ++r)
-          if (row[r] == j) ri[q] = r;
-        if (ri[q] < 0) {
-          row[nr] = j;
-          coeff_images(field, coeffs[t * m + j], img[nr]);
-          ri[q] = nr++;
-        }
+void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t k, uint32_t* out) {
+  for (size_t t = 0; t < k; ++t)
+    for (int half = 0; half < 2; ++half)
+      for (uint32_t n = 0; n < 16; ++n) {
+        uint32_t word = 0;
+        for (size_t j = 0; j < m; ++j)
+          word |= static_cast<uint32_t>(gf_mul(field, coeffs[t * m + j] & 0xFF, half ? n << 4 : n)) << (8 * j);
+        out[t * kCompactWords + half * 16 + n] = word;
       }
-      for (int p = 0; p < E; ++p) {
-        uint32_t* slot = out + ((tt * E + p) * G + g) * kCompactWords;
-        for (int half = 0; half < 2; ++half)
-          for (int n = 0; n < 16; ++n) {
-            const uint8_t x = static_cast<uint8_t>(half ? (n << 4) : n);
-            uint32_t word = 0;
-            for (int q = 0; q < 4; ++q)
-              if (ri[q] >= 0) word |= static_cast<uint32_t>(image_byte(img[ri[q]], p, x, ob[q])) << (8 * q);
-            slot[half * 16 + n] = word;
-          }
-      }
-    }
-  }
 }
 
 // Tower levels split per launch. A leaf product's table word holds the H-byte
@@ -154,26 +123,28 @@ cudaError_t lut_launch(int field, size_t nr, LutArgs& a, bool unal, bool edges_o
   }
 }
 
-void build_kara16_tables(const uint64_t* coeffs, size_t m, size_t k, size_t Gq, uint32_t* out) {
-  for (size_t t = 0; t < k; ++t)
-    for (int P = 0; P < 3; ++P)
-      for (size_t q = 0; q < Gq; ++q) {
-        uint8_t cp[4];
-        for (int r = 0; r < 4; ++r) {
-          const size_t j = 4 * q + r;
-          const uint64_t c = j < m ? coeffs[t * m + j] : 0;
-          const uint8_t c0 = static_cast<uint8_t>(c), c1 = static_cast<uint8_t>(c >> 8);
-          cp[r] = P == 0 ? c0 : P == 1 ? c1 : static_cast<uint8_t>(c0 ^ c1);
-        }
-        uint32_t* slot = out + ((t * 3 + P) * Gq + q) * kCompactWords;
-        for (int half = 0; half < 2; ++half)
-          for (int n = 0; n < 16; ++n) {
-            const uint8_t x = static_cast<uint8_t>(half ? (n << 4) : n);
-            uint32_t w = 0;
-            for (int r = 0; r < 4; ++r) w |= static_cast<uint32_t>(gf8b_mul(cp[r], x)) << (8 * r);
-            slot[half * 16 + n] = w;
-          }
-      }
+LutBatchKernel lut_batch_kernel_for(int E, LutShape s, bool unal) {
+  switch (E) {
+    case 1: return lut_batch_e1(s.lev, s.w, unal);
+    case 2: return lut_batch_e2(s.lev, s.w, unal);
+    case 4: return lut_batch_e4(s.lev, s.w, unal);
+    case 8: return lut_batch_e8(s.lev, s.w, unal);
+    default: return LutBatchKernel{};
+  }
+}
+
+JobAlign job_align(int field, const uint64_t* srcs, size_t k, const uint64_t* dsts, size_t m, uint64_t len) {
+  JobAlign r{true, false, false, 0};
+  const uint64_t al = k ? srcs[0] & 15 : 0;
+  for (size_t t = 0; t < k; ++t) r.sources = r.sources && (srcs[t] & 15) == al;
+  r.sources = r.sources && al % static_cast<uint64_t>(field_bytes(field)) == 0;
+  r.unal = !r.sources;
+  for (size_t j = 0; j < m; ++j) r.unal = r.unal || (dsts[j] & 15) != al;
+  if (r.unal)
+    for (size_t j = 0; j < m; ++j)
+      for (size_t t = 0; t < k; ++t) r.overlap = r.overlap || (dsts[j] < srcs[t] + len && srcs[t] < dsts[j] + len);
+  if (r.sources) r.head = std::min<uint64_t>((16 - al) & 15, len);
+  return r;
 }
 
 }  // namespace fgfc

@@ -367,7 +367,7 @@ fgfc_status fgfc_batch_run_noalloc(fgfc_field field, const fgfc_noalloc_job *job
  * can run; every family gives the same bytes. */
 typedef enum fgfc_kernel {
   FGFC_KERNEL_AUTO = 0,   /* the tuned or built-in choice */
-  FGFC_KERNEL_NIBBLE = 1, /* split-nibble product tables in shared memory (every shape) */
+  FGFC_KERNEL_NIBBLE = 1, /* small product tables in shared memory (every shape) */
   FGFC_KERNEL_BYTE = 2,   /* 256-entry byte tables: Gf8, at most 4 rows and 14 sources */
   FGFC_KERNEL_GF2MMA = 3  /* bit-sliced GF(2) contraction on the tensor cores (tcgen05) */
 } fgfc_kernel;
@@ -387,7 +387,7 @@ fgfc_status fgfc_tune_shape(fgfc_field field, size_t nsrcs, size_t nrows, size_t
 fgfc_status fgfc_device_check(int clear);
 /* Tile shape of the batched work lists (fgfc_batch_run and the serving
  * loop): the 16-byte element vectors each thread takes per work item, for a
- * split-nibble work-list class (element bytes 1, 2 or 4; table groups 1..4 =
+ * table work-list class (element bytes 1, 2 or 4; table groups 1..4 =
  * rows per 4-byte group times groups). cols is 1, 2, 4, 8 or 16; 0 restores
  * the built-in 8. The environment variable FGFC_TILE_COLS (read once)
  * overrides every class for A/B runs. Tiles change only how work is split,

@@ -70,7 +70,7 @@ def _run(field, k, m, rl, src_offs, base, row_offs, ovr, raw, batched, rng):
     assert bad.size == 0, (field.__name__, k, m, rl, src_offs, base, row_offs, ovr, raw, batched, bad[:8], starts)
 
 
-@pytest.mark.parametrize("batched", [False], ids=["single"])
+@pytest.mark.parametrize("batched", [False, True], ids=["single", "batch"])
 @pytest.mark.parametrize("offsets", ["aligned", "common", "rows", "sources", "any"])
 @pytest.mark.parametrize("field", ALL, ids=lambda f: f.__name__)
 def test_matrix_shapes(cuda, field, offsets, batched):
