@@ -2,8 +2,8 @@
 //
 // The reference routes each call by shape once its CPU backend is known
 // (blocked vs AXPY paths, src/kernel/gf16.rs:419-460; backend detection,
-// src/kernel/mod.rs:147-184). Here the families are the split-nibble table
-// kernels (every shape), the byte-table kernels (Gf8, one 4-row group, at most
+// src/kernel/mod.rs:147-184). Here the families are the table
+// kernels (every shape, lut.cuh), the byte-table kernels (Gf8, one 4-row group, at most
 // 14 sources) and the bit-sliced GF(2) contraction on the tensor cores
 // (gf2mma.cu). The choice for a (field, sources, rows, row-length bucket)
 // comes from, in order: a process-wide override for A/B runs
@@ -99,19 +99,17 @@ int forced_locked() {
   return g_force;
 }
 
-// Built-in rules (B200 measurements of dot_product_matrix over 1 and 4 MiB
-// rows, every field, k * E in {4 .. 64} bytes, m * E in {1 .. 16} bytes):
-// byte tables reach the HBM roofline for their shapes once a row is long
-// enough to amortise the 1.5 us table fill; the tensor-core contraction
-// wins where a column carries the most output it takes (m * E = 16 bytes)
-// from at least 32 input bytes (Gf8 RS(64,16), Gf16 RS(16..32,8), Gf32
-// RS(8..16,4): 1.1 - 1.6x the split-nibble kernel, whose lookups per output
-// bit cost the most there).
+// Built-in rules. Byte tables for their shapes once a row is long enough to
+// amortise their 1.5 us fill. The tensor-core contraction is not chosen: at
+// the shapes that suit it best (16 output bytes per column, 64 input bytes)
+// the 32-word tables take, on B200 and device time,
+//   Gf16 RS(32,8), 16 MiB rows   361 us against 522
+//   Gf32 RS(16,4),  8 MiB rows    91 us against 149
+//   Gf8B RS(64,16), 4 MiB rows   249 us against 321
+// and the gap widens as columns carry fewer bytes (Gf8D RS(20,8): 46 against
+// 176). It stays for callers that force it or measure their own shapes.
 int builtin_choice(int field, size_t k, size_t m, size_t len) {
-  const size_t E = static_cast<size_t>(field_bytes(field));
   if (kernel_usable(FGFC_KERNEL_BYTE, field, k, m) && len >= (4u << 20)) return FGFC_KERNEL_BYTE;
-  if (kernel_usable(FGFC_KERNEL_GF2MMA, field, k, m) && len >= (1u << 20) && E * m >= 16 && E * k >= 32)
-    return FGFC_KERNEL_GF2MMA;
   return FGFC_KERNEL_NIBBLE;
 }
 
