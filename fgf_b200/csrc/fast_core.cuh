@@ -19,6 +19,20 @@ __device__ __forceinline__ uint32_t lds_at(uint32_t off) {
   return *reinterpret_cast<const uint32_t*>(g_smem + off);
 }
 
+// Shifts by constants, MUL: on the multiply pipe. The bit-plane and tower-table
+// kernels are bound by the ALU pipe (shifts, logic, permutes) with the FMA pipe
+// nearly idle, and the compiler leaves right shifts and part of the left ones on
+// the former. A multiplier it cannot see to be a power of two (grids are one
+// CTA high, so gridDim.y is 1) makes x << s a product and x >> s the high half
+// of one.
+template <bool MUL>
+struct Shift {
+  uint32_t one;
+  __device__ __forceinline__ Shift() : one(MUL ? gridDim.y : 1u) {}
+  __device__ __forceinline__ uint32_t shl(uint32_t x, int s) const { return MUL ? x * (one << s) : x << s; }
+  __device__ __forceinline__ uint32_t shr(uint32_t x, int s) const { return MUL ? __umulhi(x, one << (32 - s)) : x >> s; }
+};
+
 // Source loads: read-only path without L1 allocation (sources are read once).
 __device__ __forceinline__ uint4 ldg16(const uint8_t* p) {
   uint4 v;

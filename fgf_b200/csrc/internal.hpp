@@ -172,6 +172,11 @@ cudaError_t launch_xor(uint8_t* dst, const uint8_t* src, uint64_t len, cudaStrea
 // Elementwise product dst[i] = a[i] * b[i].
 cudaError_t launch_elementwise(int field, uint8_t* dst, const uint8_t* a, const uint8_t* b,
                                uint64_t len, cudaStream_t s);
+// The same for vectors that share their offset within 16 bytes
+// (elementwise.cu): `head` bytes of whole elements, then nvec vectors of 16
+// bytes, then a tail of less.
+cudaError_t launch_elementwise_planes(int field, uint8_t* dst, const uint8_t* a, const uint8_t* b, uint64_t len,
+                                      uint32_t head, uint64_t nvec, cudaStream_t s);
 
 int sm_count();
 

@@ -5,6 +5,7 @@
 // two vectors.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <map>
@@ -124,7 +125,8 @@ __global__ void xor_kernel(uint8_t* __restrict__ dst, const uint8_t* __restrict_
 // Per-device caches (SM count) are arrays indexed by device ordinal.
 constexpr int kMaxDevices = 64;
 
-// ---- mul_elementwise: products of two vectors, without tables.
+// ---- mul_elementwise where the three vectors do not share their offset
+// within 16 bytes (the others run elementwise.cu).
 //
 // GF(2^8) products of 4 byte lanes of a 32-bit word at once by shifts and
 // XORs: x * y = XOR over the set bits b of y of x * 2^b, where x * 2 is the
@@ -134,8 +136,7 @@ constexpr int kMaxDevices = 64;
 // Gf16 and Gf32 use their tower identities over these byte products:
 //   (a + b u)(c + d u) = (ac + 0x20 bd) + ((a + b)(c + d) + ac) u      (Gf16)
 //   (A + B v)(C + D v) = (AC + 0x2000 BD) + ((A + B)(C + D) + AC) v   (Gf32)
-// (src/field/gf16.rs:54-60, src/field/gf32.rs:36-42). No lookups means no
-// shared-memory bank conflicts; the kernel is bound by HBM for Gf8.
+// (src/field/gf16.rs:54-60, src/field/gf32.rs:36-42).
 
 __device__ __forceinline__ uint32_t prmt_sign(uint32_t a, uint32_t sel) {
   uint32_t d;
@@ -219,36 +220,23 @@ __device__ __forceinline__ uint32_t emul_word(uint32_t x, uint32_t y) {
   return gmul32(x, y);
 }
 
-// Vector path: dst, a and b share their offset within 16 bytes and the first
-// `head` bytes (a whole number of elements) run through the scalar path, so
-// the body is 16-byte loads and stores; `nvec` 16-byte vectors follow.
-// Scalar path (head, tail, or every element when the offsets differ): one
-// element per thread step, its bytes gathered into the low lanes of a word.
+// One element per thread step, its bytes gathered into the low lanes of a word
+// (whole elements where they are aligned): vectors that do not share their
+// offset within 16 bytes, and short ones.
 template <int F>
 __global__ void elementwise_kernel(uint8_t* __restrict__ dst, const uint8_t* __restrict__ a,
-                                   const uint8_t* __restrict__ b, uint64_t len, uint64_t head, uint64_t nvec) {
+                                   const uint8_t* __restrict__ b, uint64_t nelem) {
   constexpr int E = (F == kGf16) ? 2 : (F == kGf32 ? 4 : 1);
+  const bool words = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(a) |
+                       reinterpret_cast<uintptr_t>(b)) & 3u) == 0;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  for (uint64_t v = tid; v < nvec; v += stride) {
-    const uint64_t o = head + 16 * v;
-    const uint4 x = ldg16(a + o), y = ldg16(b + o);
-    uint4 r;
-    if (F == kGf16) {  // pairs of words share their cross-product pass
-      gmul16x2_pair(x.x, y.x, x.y, y.y, r.x, r.y);
-      gmul16x2_pair(x.z, y.z, x.w, y.w, r.z, r.w);
-    } else {
-      r.x = emul_word<F>(x.x, y.x);
-      r.y = emul_word<F>(x.y, y.y);
-      r.z = emul_word<F>(x.z, y.z);
-      r.w = emul_word<F>(x.w, y.w);
+  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nelem; i += stride) {
+    const uint64_t o = i * E;
+    if (E == 4 && words) {
+      *reinterpret_cast<uint32_t*>(dst + o) = emul_word<F>(*reinterpret_cast<const uint32_t*>(a + o),
+                                                           *reinterpret_cast<const uint32_t*>(b + o));
+      continue;
     }
-    *reinterpret_cast<uint4*>(dst + o) = r;
-  }
-  const uint64_t tail0 = head + 16 * nvec;
-  const uint64_t nscalar = (head + (len - tail0)) / E;
-  for (uint64_t i = tid; i < nscalar; i += stride) {
-    const uint64_t o = i * E < head ? i * E : tail0 + (i * E - head);
     uint32_t x = 0, y = 0;
 #pragma unroll
     for (int k = 0; k < E; ++k) {
@@ -467,36 +455,42 @@ static cudaError_t launch_elementwise_fp(int field, uint8_t* dst, const uint8_t*
   return cudaGetLastError();
 }
 
+// Vectors shorter than this run one element per thread: a planes warp takes
+// 1 KiB times the element width through 1400 (4 bytes) to 3500 (8 bytes)
+// instructions, which a short vector does not amortise. us on B200, element
+// kernel / planes: Gf32 64 KiB 3.2 / 4.6, 1 MiB 4.9 / 4.6; FP32 64 KiB 3.5 / 4.8,
+// 1 MiB 10.5 / 4.8; Gf64 1 MiB 7.4 / 10.5, 64 MiB 322 / 107; FP64 1 MiB 9.8 /
+// 11.0, 64 MiB 246 / 108. 1- and 2-byte fields are level at 64 KiB.
+static uint64_t planes_min_bytes(int field) {
+  switch (field) {
+    case kGf32: return 1u << 20;
+    case kFp32: return 1u << 18;
+    case kGf64:
+    case kFp64: return 2u << 20;
+    default: return 0;
+  }
+}
+
 cudaError_t launch_elementwise(int field, uint8_t* dst, const uint8_t* a, const uint8_t* b,
                                uint64_t len, cudaStream_t s) {
   if (!len) return cudaSuccess;
   const int E = field_bytes(field);
   if (E <= 0 || len % E) return cudaErrorInvalidValue;
+  const uint64_t al = reinterpret_cast<uintptr_t>(dst) & 15, head = std::min<uint64_t>((16 - al) & 15, len);
+  if (al == (reinterpret_cast<uintptr_t>(a) & 15) && al == (reinterpret_cast<uintptr_t>(b) & 15) && head % E == 0 &&
+      len >= planes_min_bytes(field))
+    return launch_elementwise_planes(field, dst, a, b, len, static_cast<uint32_t>(head), (len - head) / 16, s);
   if (field == kFp8 || field == kFp16 || field == kFp32 || field == kFp64)
     return launch_elementwise_fp(field, dst, a, b, len, s);
-  if (field == kGf64) {
-    const uint64_t nelem = len / 8;
-    uint64_t want = (nelem + 255) / 256, cap = static_cast<uint64_t>(sm_count()) * 8;
-    elementwise_gf64_kernel<<<static_cast<unsigned>(want < cap ? want : cap), 256, 0, s>>>(dst, a, b, nelem);
-    return cudaGetLastError();
-  }
-  const uint64_t ad = reinterpret_cast<uintptr_t>(dst) & 15;
-  uint64_t head = len, nvec = 0;
-  if (ad == (reinterpret_cast<uintptr_t>(a) & 15) && ad == (reinterpret_cast<uintptr_t>(b) & 15)) {
-    const uint64_t h = (16 - ad) & 15;
-    if (h % E == 0 && h <= len) {
-      head = h;
-      nvec = (len - h) / 16;
-    }
-  }
-  const uint64_t work = nvec + (len - 16 * nvec) / E;
-  uint64_t want = (work + 255) / 256, cap = static_cast<uint64_t>(sm_count()) * 8;
+  const uint64_t nelem = len / E;
+  const uint64_t want = (nelem + 255) / 256, cap = static_cast<uint64_t>(sm_count()) * 8;
   const unsigned blocks = static_cast<unsigned>(want < cap ? want : cap);
   switch (field) {
-    case kGf8B: elementwise_kernel<kGf8B><<<blocks, 256, 0, s>>>(dst, a, b, len, head, nvec); break;
-    case kGf8D: elementwise_kernel<kGf8D><<<blocks, 256, 0, s>>>(dst, a, b, len, head, nvec); break;
-    case kGf16: elementwise_kernel<kGf16><<<blocks, 256, 0, s>>>(dst, a, b, len, head, nvec); break;
-    case kGf32: elementwise_kernel<kGf32><<<blocks, 256, 0, s>>>(dst, a, b, len, head, nvec); break;
+    case kGf8B: elementwise_kernel<kGf8B><<<blocks, 256, 0, s>>>(dst, a, b, nelem); break;
+    case kGf8D: elementwise_kernel<kGf8D><<<blocks, 256, 0, s>>>(dst, a, b, nelem); break;
+    case kGf16: elementwise_kernel<kGf16><<<blocks, 256, 0, s>>>(dst, a, b, nelem); break;
+    case kGf32: elementwise_kernel<kGf32><<<blocks, 256, 0, s>>>(dst, a, b, nelem); break;
+    case kGf64: elementwise_gf64_kernel<<<blocks, 256, 0, s>>>(dst, a, b, nelem); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
