@@ -378,8 +378,21 @@ struct LutShared {
   uint8_t* dst[kLutRows];
 };
 
-// Fold all sources of one column: load(t) fetches source t's 16 bytes, fix(t,
-// x) puts them in place once they are needed. The fetches of the next three
+// Three sources' 16-byte columns on their way from memory.
+struct LutAhead {
+  uint4 c[3];
+};
+
+// Does a shape's aligned path fetch the next column's first sources during the
+// last lookups of this one? Where the accumulators leave 16 warps an SM it hides the fetch (us,
+// without -> with: Gf16 RS(32,8) 16 MiB 355 -> 339, Gf32 RS(16,4) 8 MiB 91 -> 86,
+// Gf8D RS(32,12) 4 MiB 103 -> 99); smaller shapes have the warps to hide it and
+// pay for the registers (Gf8D RS(10,4) 4 MiB 17.6 -> 18.4).
+template <class L, int W>
+constexpr bool kLutAhead = L::NP * W * L::NE >= 32;
+
+// Fold all sources of one column. load(t) fetches source t's 16 bytes, fix(t, x)
+// puts a fetch in place once it is needed. The fetches of the next three
 // sources are in flight during the lookups.
 template <class L, int W, class Load, class Fix>
 __device__ __forceinline__ void lut_column(LutAcc<L, W>& A, uint32_t k, Load load, Fix fix) {
@@ -406,6 +419,42 @@ __device__ __forceinline__ void lut_column(LutAcc<L, W>& A, uint32_t k, Load loa
     lut_fold1<L, W>(fix(3u * nt + r, c0), base, A);
     c0 = c1;
     base += S::block1;
+  }
+}
+
+// The same for shapes that look ahead: on entry h holds this column's first
+// three sources, on return the next column's, which next(t) fetches.
+template <class L, int W, class Load, class Next, class Fix>
+__device__ __forceinline__ void lut_column_ahead(LutAcc<L, W>& A, uint32_t k, LutAhead& h, Load load, Next next,
+                                                 Fix fix) {
+  using S = LutSmem<L::NV, W>;
+  A.zero();
+  const uint32_t nt = k / 3u, rest = k - 3u * nt;
+  uint32_t base = 0;
+  for (uint32_t i = 0; i < nt; ++i) {
+    const uint32_t t = 3u * i;
+    const uint4 x0 = fix(t, h.c[0]), x1 = fix(t + 1u, h.c[1]), x2 = fix(t + 2u, h.c[2]);
+    if (t + 3u < k) {
+#pragma unroll
+      for (uint32_t j = 0; j < 3; ++j)
+        if (t + 3u + j < k) h.c[j] = load(t + 3u + j);
+    } else {
+#pragma unroll
+      for (uint32_t j = 0; j < 3; ++j) h.c[j] = next(j);
+    }
+    lut_fold3<L, W>(x0, x1, x2, base, A);
+    base += S::block3;
+  }
+  if (rest) {
+    const uint32_t t = 3u * nt;
+    const uint4 x0 = fix(t, h.c[0]);
+    uint4 x1 = x0;
+    if (rest > 1) x1 = fix(t + 1u, h.c[1]);
+#pragma unroll
+    for (uint32_t j = 0; j < 3; ++j)
+      if (j < k) h.c[j] = next(j);
+    lut_fold1<L, W>(x0, base, A);
+    if (rest > 1) lut_fold1<L, W>(x1, base + S::block1, A);
   }
 }
 
@@ -445,71 +494,95 @@ __device__ __forceinline__ uint4 load_bytes16(const uint8_t* p, uint64_t off, ui
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Tile `tile` of a job: blockDim.x columns of an aligned job, 30 blocks per
-// warp of an unaligned one.
+// Tiles first, first + step, ... of a job's ntiles: blockDim.x columns each, 30
+// blocks per warp of an unaligned job.
 template <class L, int LEV, int W, bool UNAL>
-__device__ __forceinline__ void lut_tile(const LutGeom& g, const LutShared& sh, uint64_t tile, bool ovr, bool fp) {
+__device__ __forceinline__ void lut_run(const LutGeom& g, const LutShared& sh, uint64_t first, uint64_t step, bool ovr,
+                                        bool fp) {
+  constexpr int R = 4 / L::H;
+  const uint32_t k = g.k;
   LutAcc<L, W> A;
   uint32_t f[W][L::NF];
-  constexpr int R = 4 / L::H;
   if constexpr (!UNAL) {
-    const uint64_t v = tile * blockDim.x + threadIdx.x;
-    if (v >= g.ncol) return;
-    const uint64_t off = g.head + 16 * v;
-    lut_column<L, W>(A, g.k, [&](uint32_t t) { return ldg16(sh.src[t] + off); }, LutAsIs());
-    lut_finish<L, W, LEV>(A, f, fp);
-    lut_store<L, W>(f, sh, g.nrows, off, ovr);
-  } else {
-    if (g.bytes) {  // each thread reads and writes only its own column
-      const uint64_t v = tile * blockDim.x + threadIdx.x;
-      if (16 * v >= g.len) return;
-      lut_column<L, W>(A, g.k, [&](uint32_t t) { return load_bytes16(sh.src[t], 16 * v, g.len); }, LutAsIs());
+    if constexpr (kLutAhead<L, W>) {
+      const uint64_t end = g.head + 16 * g.ncol, stride = 16 * step * blockDim.x;
+      uint64_t off = g.head + 16 * (first * blockDim.x + threadIdx.x);
+      if (off >= end) return;
+      LutAhead h;
+#pragma unroll
+      for (uint32_t j = 0; j < 3; ++j) h.c[j] = j < k ? ldg16(sh.src[j] + off) : make_uint4(0, 0, 0, 0);
+      for (;;) {
+        const uint64_t noff = off + stride;
+        const bool more = noff < end;
+        lut_column_ahead<L, W>(
+            A, k, h, [&](uint32_t t) { return ldg16(sh.src[t] + off); },
+            [&](uint32_t t) { return more ? ldg16(sh.src[t] + noff) : make_uint4(0, 0, 0, 0); }, LutAsIs());
+        lut_finish<L, W, LEV>(A, f, fp);
+        lut_store<L, W>(f, sh, g.nrows, off, ovr);
+        if (!more) return;
+        off = noff;
+      }
+    } else {
+      const uint64_t ntiles = lut_tiles(g, false, blockDim.x);
+      for (uint64_t tile = first; tile < ntiles; tile += step) {
+        const uint64_t v = tile * blockDim.x + threadIdx.x;
+        if (v >= g.ncol) return;
+        const uint64_t o = g.head + 16 * v;
+        lut_column<L, W>(A, g.k, [&](uint32_t t) { return ldg16(sh.src[t] + o); }, LutAsIs());
+        lut_finish<L, W, LEV>(A, f, fp);
+        lut_store<L, W>(f, sh, g.nrows, o, ovr);
+      }
+    }
+  } else if (g.bytes) {  // each thread reads and writes only its own column
+    for (uint64_t off = 16 * (first * blockDim.x + threadIdx.x); off < g.len; off += 16 * step * blockDim.x) {
+      lut_column<L, W>(A, k, [&](uint32_t t) { return load_bytes16(sh.src[t], off, g.len); }, LutAsIs());
       lut_finish<L, W, LEV>(A, f, fp);
-      const uint32_t nb = g.len - 16 * v < 16 ? static_cast<uint32_t>(g.len - 16 * v) : 16u;
+      const uint32_t nb = g.len - off < 16 ? static_cast<uint32_t>(g.len - off) : 16u;
 #pragma unroll
       for (int q = 0; q < W; ++q)
 #pragma unroll
         for (int r = 0; r < R; ++r)
           if (static_cast<uint32_t>(q * R + r) < g.nrows)
-            put_bytes(sh.dst[q * R + r] + 16 * v, lut_row<L>(f[q], r), 0, nb, ovr);
-      return;
+            put_bytes(sh.dst[q * R + r] + off, lut_row<L>(f[q], r), 0, nb, ovr);
     }
+  } else {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint64_t first = kUnalFirst + (tile * (blockDim.x >> 5) + warp) * kUnalStep;  // lane 1's column
-    const uint64_t end = g.ncol - 1;                                                   // blocks end before it
-    if (first >= end) return;  // the whole warp
-    const uint64_t c = first - 1 + lane;
-    // A granule past the last whole one belongs to no column that is written.
-    lut_column<L, W>(
-        A, g.k,
-        [&](uint32_t t) {
-          const uint64_t a = reinterpret_cast<uint64_t>(sh.src[t]);
-          const uint32_t s = static_cast<uint32_t>(a) & 15u;
-          uint4 x = make_uint4(0, 0, 0, 0);
-          if (16 * c + 16 - s <= g.len) x = ldg16(reinterpret_cast<const uint8_t*>(a - s) + 16 * c);
-          return x;
-        },
-        [&](uint32_t t, const uint4& x) {
-          const uint32_t s = static_cast<uint32_t>(reinterpret_cast<uint64_t>(sh.src[t])) & 15u;  // one value for the warp
-          return s == 0 ? x : splice16(x, shfl_down4(x), s);
-        });
-    lut_finish<L, W, LEV>(A, f, fp);
-    const bool valid = lane >= 1 && lane <= kUnalStep && c < end;
+    // lane l's column is v - 1 + l, blocks end before column ncol - 1
+    const uint64_t end = g.ncol - 1, stride = step * (blockDim.x >> 5) * kUnalStep;
+    for (uint64_t v = kUnalFirst + (first * (blockDim.x >> 5) + warp) * kUnalStep; v < end; v += stride) {
+      const uint64_t c = v - 1 + lane;
+      // A granule past the last whole one belongs to no column that is written.
+      lut_column<L, W>(
+          A, k,
+          [&](uint32_t t) {
+            const uint64_t a = reinterpret_cast<uint64_t>(sh.src[t]);
+            const uint32_t s = static_cast<uint32_t>(a) & 15u;
+            uint4 x = make_uint4(0, 0, 0, 0);
+            if (16 * c + 16 - s <= g.len) x = ldg16(reinterpret_cast<const uint8_t*>(a - s) + 16 * c);
+            return x;
+          },
+          [&](uint32_t t, const uint4& x) {
+            const uint32_t s = static_cast<uint32_t>(reinterpret_cast<uint64_t>(sh.src[t])) & 15u;  // one for the warp
+            return s == 0 ? x : splice16(x, shfl_down4(x), s);
+          });
+      lut_finish<L, W, LEV>(A, f, fp);
+      const bool valid = lane >= 1 && lane <= kUnalStep && c < end;
 #pragma unroll
-    for (int q = 0; q < W; ++q)
+      for (int q = 0; q < W; ++q)
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const uint32_t row = q * R + r;
-        if (row >= g.nrows) continue;
-        const uint4 o = lut_row<L>(f[q], r);
-        const uint32_t dl = static_cast<uint32_t>(reinterpret_cast<uint64_t>(sh.dst[row])) & 15u;
-        if (dl == 0) {
-          if (valid) put16(sh.dst[row] + 16 * c, o, ovr);
-        } else {
-          const uint4 b = splice16(shfl_up4(o), o, 16u - dl);
-          if (valid) put16(sh.dst[row] + 16 * c - dl, b, ovr);
+        for (int r = 0; r < R; ++r) {
+          const uint32_t row = q * R + r;
+          if (row >= g.nrows) continue;
+          const uint4 o = lut_row<L>(f[q], r);
+          const uint32_t dl = static_cast<uint32_t>(reinterpret_cast<uint64_t>(sh.dst[row])) & 15u;
+          if (dl == 0) {
+            if (valid) put16(sh.dst[row] + 16 * c, o, ovr);
+          } else {
+            const uint4 b = splice16(shfl_up4(o), o, 16u - dl);
+            if (valid) put16(sh.dst[row] + 16 * c - dl, b, ovr);
+          }
         }
-      }
+    }
   }
 }
 
@@ -554,8 +627,8 @@ __device__ __forceinline__ void lut_edges(const LutGeom& g, const LutShared& sh,
     if (nb) {
       LutAcc<L, W> A;
       uint32_t f[W][L::NF];
-      lut_column<L, W>(A, g.k, [&](uint32_t t) { return reinterpret_cast<const uint4*>(stage)[t * kEdges + j]; },
-                       LutAsIs());
+      const auto load = [&](uint32_t t) { return reinterpret_cast<const uint4*>(stage)[t * kEdges + j]; };
+      lut_column<L, W>(A, g.k, load, LutAsIs());
       lut_finish<L, W, LEV>(A, f, fp);
 #pragma unroll
       for (int q = 0; q < W; ++q)

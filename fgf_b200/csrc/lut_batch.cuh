@@ -51,9 +51,7 @@ __global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, UNAL>())
       __syncthreads();
       const bool ovr = s_job.g.ovr != 0, fp = s_job.fp != 0;
       if (wi.y < s_job.parts) {
-        const uint64_t ntiles = lut_tiles(s_job.g, UNAL, blockDim.x);
-        for (uint64_t tile = wi.y; tile < ntiles; tile += s_job.parts)
-          lut_tile<L, LEV, W, UNAL>(s_job.g, sh, tile, ovr, fp);
+        lut_run<L, LEV, W, UNAL>(s_job.g, sh, wi.y, s_job.parts, ovr, fp);
       } else {
         uint8_t* stage = g_smem + kk / 3u * S::block3 + kk % 3u * S::block1;
         lut_edges<L, LEV, W, UNAL>(s_job.g, sh, stage, ovr, fp);

@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, UNAL>())
     lut_edges<L, LEV, W, UNAL>(a.g, sh, stage, ovr, fp);
     return;
   }
-  for (uint64_t tile = blockIdx.x; tile < a.ntiles; tile += nwork) lut_tile<L, LEV, W, UNAL>(a.g, sh, tile, ovr, fp);
+  if (a.ntiles) lut_run<L, LEV, W, UNAL>(a.g, sh, blockIdx.x, nwork, ovr, fp);
 }
 
 // Launch one job of this (LEV, W); `a` is complete but for its tiling.
