@@ -52,28 +52,31 @@ __device__ __forceinline__ void prefetch_l2(const uint8_t* p) { asm volatile("pr
 // Gf8 fields with at most 4 rows (one table group) and a compile-time number
 // of sources K. Sources t < kByteSrc get a full 256-entry product table (one
 // lookup per source byte, 32 KiB with the 32 lane copies; two tables share
-// each 64 KiB page, at byte offsets 0 and 128 of every 256-byte row), the
-// rest keep split-nibble tables in 4 KiB slots after the three byte-table
-// pages. With K fixed every table address is a PRMT of the data byte plus an
-// immediate.
+// each 64 KiB page, at byte offsets 0 and 128 of every 256-byte row). The rest
+// use single-copy 32-word tables after those pages, as lut.cuh does: five
+// lookups for three sources, two for one (nibble tables with lane copies took
+// two each). With K fixed every table address is a PRMT of the data byte plus
+// an immediate. 16 MiB rows, 4 rows out, us before -> after: K = 8 41.2 -> 39.2,
+// K = 10 51.3 -> 48.2, K = 12 62.2 -> 57.4, K = 14 73.9 -> 72.0.
 constexpr int kByteSrc = 6;
 constexpr int kFastMaxK = 14;
 constexpr int kFastThreads = 1024;
-constexpr uint32_t kNibbleBase = 3u * 65536u;
 
 template <int K>
 struct FastLayout {
   static constexpr int NB = K < kByteSrc ? K : kByteSrc;  // byte-table sources
-  static constexpr int NN = K - NB;                       // nibble-table sources
-  static constexpr uint32_t tables = NN ? kNibbleBase + NN * kSlotBytes : ((NB + 1) / 2) * 65536u;
+  static constexpr int NN = K - NB;                       // small-table sources
+  static constexpr int N3 = NN / 3, N1 = NN % 3;          // threes, then single ones
+  static constexpr uint32_t small = ((NB + 1) / 2) * 65536u;
+  static constexpr uint32_t tables = small + N3 * 640u + N1 * 128u;
   static constexpr uint32_t smem = tables + K * kCompactWords * 4u;  // + compact staging
 };
 
 // Expand the compact tables of K sources (32 words each) into the byte-table
-// layout. `tables` is a device
-// pointer, or null to read `inl` (launch parameters). The compact words are
-// staged in shared memory first (one independent load per thread) and every
-// entry's 32 lane copies are written as 8 identical 16-byte stores.
+// layout. `tables` is a device pointer, or null to read `inl` (launch
+// parameters). The compact words are staged in shared memory first (one
+// independent load per thread) and every byte-table entry's 32 lane copies are
+// written as 8 identical 16-byte stores.
 template <int K>
 __device__ __forceinline__ void fill_fast(const uint32_t* tables, const uint32_t* inl) {
   using L = FastLayout<K>;
@@ -91,11 +94,24 @@ __device__ __forceinline__ void fill_fast(const uint32_t* tables, const uint32_t
     st4[(t >> 1) * 4096u + x * 16u + (t & 1u) * 8u + q] = make_uint4(v, v, v, v);
   }
   if constexpr (L::NN > 0) {
-#pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < L::NN * 256u; i += blockDim.x) {
-      const uint32_t v =
-          stage[(L::NB + (i >> 8)) * kCompactWords + ((i >> 3) & 1u) * 16u + ((i >> 4) & 15u)];
-      st4[kNibbleBase / 16 + i] = make_uint4(v, v, v, v);
+    // small tables: the words of one table are its 5- (or 4-) bit index
+    uint32_t* out = reinterpret_cast<uint32_t*>(g_smem + L::small);
+    for (uint32_t i = threadIdx.x; i < L::N3 * 160u + L::N1 * 32u; i += blockDim.x) {
+      const uint32_t n = i & 31u;
+      if (i < L::N3 * 160u) {
+        const uint32_t q = i / 32u % 5u;
+        const uint32_t* a = stage + (L::NB + 3u * (i / 160u)) * kCompactWords;  // source 0; 1 and 2 follow
+        uint32_t v;
+        if (q < 3)  // low 5 bits of source q
+          v = a[q * kCompactWords + (n & 15u)] ^ a[q * kCompactWords + 16u + (n >> 4)];
+        else if (q == 3)  // bits 5..7 of source 0, 5 and 6 of source 1
+          v = a[16u + 2u * (n & 7u)] ^ a[kCompactWords + 16u + 2u * (n >> 3)];
+        else  // bits 5..7 of source 2, 7 of source 1
+          v = a[2u * kCompactWords + 16u + 2u * (n & 7u)] ^ a[kCompactWords + 16u + (n & 8u)];
+        out[i] = v;
+      } else {
+        out[i] = stage[(L::NB + 3u * L::N3 + (i - L::N3 * 160u) / 32u) * kCompactWords + n];
+      }
     }
   }
   __syncthreads();
@@ -104,12 +120,10 @@ __device__ __forceinline__ void fill_fast(const uint32_t* tables, const uint32_t
 // Lane / page registers of the byte-table layout.
 struct FastRegs {
   uint32_t lrp[3];  // byte-table pages 0..2
-  uint32_t lrn;     // nibble slots (page 3)
   __device__ __forceinline__ FastRegs() {
     const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
 #pragma unroll
     for (int p = 0; p < 3; ++p) lrp[p] = lane4 | (static_cast<uint32_t>(p) << 16);
-    lrn = lane4 | (3u << 16);
   }
 };
 
@@ -141,16 +155,35 @@ __device__ __forceinline__ void fast_fold(const uint32_t (&w)[K][NW], uint32_t (
     }
   }
 #pragma unroll
-  for (int i = 0; i < L::NN; ++i) {
-    const uint32_t pat = ((static_cast<uint32_t>(48 + i) & 15u) << 4) * 0x01010101u;
+  for (int i = 0; i < L::N3; ++i) {
+    constexpr uint32_t base = L::small;
+    const int t = L::NB + 3 * i;
 #pragma unroll
     for (int q = 0; q < NW; ++q) {
-      const uint32_t xl = (w[L::NB + i][q] & 0x0F0F0F0Fu) | pat;
-      const uint32_t xh = ((w[L::NB + i][q] >> 4) & 0x0F0F0F0Fu) | pat;
+      const uint32_t i0 = (w[t][q] << 2) & 0x7C7C7C7Cu, i1 = (w[t + 1][q] << 2) & 0x7C7C7C7Cu,
+                     i2 = (w[t + 2][q] << 2) & 0x7C7C7C7Cu;
+      const uint32_t i3 = ((w[t][q] >> 3) & 0x1C1C1C1Cu) | (w[t + 1][q] & 0x60606060u);
+      const uint32_t i4 = ((w[t + 2][q] >> 3) & 0x1C1C1C1Cu) | ((w[t + 1][q] >> 2) & 0x20202020u);
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const uint32_t sel = 0x7604u | (static_cast<uint32_t>(b) << 4);
-        acc[4 * q + b] ^= lds_at(prmt(xl, r.lrn, sel)) ^ lds_at(prmt(xh, r.lrn, sel) + 128u);
+        const uint32_t sel = 0x7650u | static_cast<uint32_t>(b), o = i * 640u;
+        acc[4 * q + b] ^= lds_at(prmt(i0, base, sel) + o) ^ lds_at(prmt(i1, base, sel) + o + 128u);
+        acc[4 * q + b] ^= lds_at(prmt(i2, base, sel) + o + 256u) ^ lds_at(prmt(i3, base, sel) + o + 384u);
+        acc[4 * q + b] ^= lds_at(prmt(i4, base, sel) + o + 512u);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < L::N1; ++i) {
+    constexpr uint32_t base = L::small;
+    const int t = L::NB + 3 * L::N3 + i;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) {
+      const uint32_t i0 = (w[t][q] << 2) & 0x3C3C3C3Cu, i1 = (w[t][q] >> 2) & 0x3C3C3C3Cu;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const uint32_t sel = 0x7650u | static_cast<uint32_t>(b), o = L::N3 * 640u + i * 128u;
+        acc[4 * q + b] ^= lds_at(prmt(i0, base, sel) + o) ^ lds_at(prmt(i1, base, sel) + o + 64u);
       }
     }
   }

@@ -16,10 +16,6 @@ namespace fgfc {
 // into several launches by the host (exact: rows are independent, and
 // sources split into an overwrite launch followed by accumulate launches).
 constexpr int kMaxSrc = 64;
-// One nibble table slot of the byte-table kernels: 16 rows x 256 bytes. Each
-// row holds 32 lane copies of the lo-nibble word (bytes 0..127) and of the
-// hi-nibble word (128..255).
-constexpr int kSlotBytes = 4096;
 constexpr size_t kFastMaxSources = 14;   // byte-table kernels: sources per launch
 // Their compact tables, per source: word[n] (n < 16) = products of the low
 // nibble value n, word[16 + n] = products of n << 4; byte q is row q.
