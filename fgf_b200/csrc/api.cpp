@@ -215,13 +215,15 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
     const size_t kc = lut_sources(E, nr, cs.img == nullptr);
     const size_t src_words = lut_shape(E, nr).src_words();
     if (kc == 0) return fail(FGFC_ERR_LIMIT, "%s: internal tiling failed", name);
-    bool unal = !same;
-    for (size_t j = 0; j < nr; ++j) unal |= (reinterpret_cast<uintptr_t>(rows[r0 + j]) & 15) != al;
-    unal &= !byte_tables;  // the byte-table kernel left a head and a tail
+    bool off = !same;
+    for (size_t j = 0; j < nr; ++j) off |= (reinterpret_cast<uintptr_t>(rows[r0 + j]) & 15) != al;
+    off &= !byte_tables;  // the byte-table kernel left a head and a tail
+    const bool overlap = off && any_overlap(srcs, k, rows + r0, nr, len);
+    const LutMode mode = !off ? kAligned : same && !overlap ? kRowsOff : kAnyOff;
     a.g.len = len;
-    a.g.head = unal ? 0 : head;
+    a.g.head = mode == kAnyOff ? 0 : head;
     a.g.ncol = (len - a.g.head) / 16;
-    a.g.bytes = unal && any_overlap(srcs, k, rows + r0, nr, len) ? 1u : 0u;
+    a.g.bytes = mode == kAnyOff && overlap ? 1u : 0u;
     a.g.nrows = static_cast<uint32_t>(nr);
     for (size_t j = 0; j < nr; ++j) a.dst[j] = rows[r0 + j];
     for (size_t t0 = 0; t0 < k; t0 += kc) {
@@ -238,7 +240,7 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
       cudaError_t e;
       {
         std::lock_guard<std::mutex> lk(g_launch_mu);
-        e = lut_launch(field, nr, a, unal, byte_tables, stream);
+        e = lut_launch(field, nr, a, mode, byte_tables, stream);
       }
       if (e != cudaSuccess) return cuda_fail(e, name);
     }

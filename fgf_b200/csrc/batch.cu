@@ -499,12 +499,12 @@ static LutBatchJob lut_batch_job(int field, const uint32_t* img, const JobAlign&
   std::memset(&J, 0, sizeof J);
   J.img = img;
   J.g.len = len;
-  J.g.head = a.unal ? 0 : a.head;
+  J.g.head = a.mode == kAnyOff ? 0 : a.head;
   J.g.ncol = (len - J.g.head) / 16;
   J.g.k = static_cast<uint32_t>(k);
   J.g.nrows = static_cast<uint32_t>(nrows);
   J.g.ovr = ovr ? 1u : 0u;
-  J.g.bytes = a.unal && a.overlap ? 1u : 0u;
+  J.g.bytes = a.mode == kAnyOff && a.overlap ? 1u : 0u;
   J.fp = field == kFp16 || field == kFp32 || field == kFp64 ? 1u : 0u;
   return J;
 }
@@ -541,7 +541,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     const bool fast = L.byte_tab && al[i].sources;
     const LutShape shape = lut_shape(E, L.nrows);
     const int key = fast ? 1000 + 2 * static_cast<int>(L.k) + al[i].unal
-                         : ((E * 4 + shape.lev) * 8 + shape.w) * 2 + al[i].unal;
+                         : ((E * 4 + shape.lev) * 8 + shape.w) * 3 + al[i].mode;
     BatchClass& c = classes[key];
     c.E = E;
     c.jobs.push_back(static_cast<uint32_t>(i));
@@ -562,7 +562,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       J.nv_items = 0;
     } else {
       c.shape = shape;
-      c.kern = lut_batch_kernel_for(E, shape, al[i].unal);
+      c.kern = lut_batch_kernel_for(E, shape, al[i].mode);
       c.kc = lut_sources(E, L.nrows, false);
       D.lut = lut_batch_job(L.field, L.img, al[i], L.len, L.k, L.nrows, L.ovr);
       D.lut.src_idx = idx[i].first;
@@ -579,9 +579,9 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       const int G = static_cast<int>((jobs[c.jobs[0]].nrows * c.E + 3) / 4);
       const uint64_t tile = c.E == 8 ? kTileColsDefault : tile_cols(c.E, G);
       if (c.E < 8) b->last_classes.emplace_back(c.E, G);
-      const bool unal = kv.first & 1;
+      const int mode = kv.first % 3;
       uint64_t total = 0;
-      for (uint32_t i : c.jobs) total += lut_tiles(dj[i].lut.g, unal, kLutThreads);
+      for (uint32_t i : c.jobs) total += lut_tiles(dj[i].lut.g, mode, kLutThreads);
       const uint64_t slots = 4 * static_cast<uint64_t>(sm_count() * c.kern.ctas);
       const uint64_t per = std::max<uint64_t>(1, std::min<uint64_t>(tile, (total + slots - 1) / slots));
       // Stripes of one plan and of the byte tables' shape, but with sources at
@@ -593,8 +593,8 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         const uint32_t i = c.jobs[q];
         if (one_plan && q && q % kUniformJobs == 0) c.cuts.push_back(c.items.size());
         LutBatchJob& J = dj[i].lut;
-        J.parts = static_cast<uint32_t>((lut_tiles(J.g, unal, kLutThreads) + per - 1) / per);
-        const uint32_t n = J.parts + (lut_has_edges(J.g, unal) ? 1u : 0u);
+        J.parts = static_cast<uint32_t>((lut_tiles(J.g, mode, kLutThreads) + per - 1) / per);
+        const uint32_t n = J.parts + (lut_has_edges(J.g, mode) ? 1u : 0u);
         for (uint32_t p = 0; p < n; ++p) c.items.push_back(make_uint2(i, p));
       }
       continue;
@@ -1098,8 +1098,9 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
     const uint32_t dst_idx = static_cast<uint32_t>(pn);
     for (size_t j = 0; j < S.nrows; ++j)
       hp[pn++] = reinterpret_cast<uint64_t>(S.dst + (S.row_starts ? S.row_starts[j] : j * S.row_len));
-    const JobAlign al = job_align(field, hp + src_idx, S.nsrcs, hp + dst_idx, S.nrows, S.row_len);
-    const int var = al.unal ? 1 : 0;
+    JobAlign al = job_align(field, hp + src_idx, S.nsrcs, hp + dst_idx, S.nrows, S.row_len);
+    if (al.mode == kRowsOff) al.mode = kAnyOff;  // two launches per class at most
+    const int var = al.mode == kAligned ? 0 : 1;
     const bool fast = cls < 100 && !al.unal;
     uint64_t cm[kMaxSrc * 16];  // coefficients reduced to the field's width, as Plan::matrix does
     for (size_t q = 0; q < S.nsrcs * S.nrows; ++q) cm[q] = S.coeffs[q] & field_mask(field);
@@ -1128,8 +1129,8 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
       J.src_idx = src_idx;
       J.dst_idx = dst_idx;
       const uint64_t per = kNoallocCols / kLutThreads;
-      J.parts = static_cast<uint32_t>((lut_tiles(J.g, al.unal, kLutThreads) + per - 1) / per);
-      nitems = J.parts + (lut_has_edges(J.g, al.unal) ? 1 : 0);
+      J.parts = static_cast<uint32_t>((lut_tiles(J.g, al.mode, kLutThreads) + per - 1) / per);
+      nitems = J.parts + (lut_has_edges(J.g, al.mode) ? 1 : 0);
       class_smem[cls][var] = std::max(class_smem[cls][var],
                                       lut_smem(lut_shape(E, S.nrows),
                                                std::min(S.nsrcs, lut_sources(E, S.nrows, false))));
@@ -1156,7 +1157,7 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
       if (!n) continue;
       const bool fast = c < 100 && var == 0;
       const KernelFn fn = fast ? fast_kernel_for(c, false) : nullptr;
-      const LutBatchKernel lut = fast ? LutBatchKernel{} : lut_batch_kernel_for(E, lut_shape(E, class_rows[c]), var != 0);
+      const LutBatchKernel lut = fast ? LutBatchKernel{} : lut_batch_kernel_for(E, lut_shape(E, class_rows[c]), var ? kAnyOff : kAligned);
       if (!fn && !lut.fn) {
         e = cudaErrorInvalidValue;
         break;

@@ -38,45 +38,53 @@ void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t k,
 
 // ---------------------------------------------------------------- table kernels (lut.cuh)
 
-// One job's geometry. Columns are 16 bytes, column v at head + 16 v. Aligned
-// jobs (every source and row at one offset within 16 bytes, whole elements
-// before the first aligned column) have `head` bytes, then `ncol` whole
-// columns. Unaligned jobs have head = 0 and columns from the row's start.
-// Bytes outside the columns that the vector path covers are "edges".
+// How a job's pointers sit within 16 bytes.
+enum LutMode : int {
+  kAligned = 0,  // every source and row at one offset, whole elements before the boundary
+  kRowsOff = 1,  // the sources so, rows anywhere (contiguous rows of a ragged length)
+  kAnyOff = 2,   // sources anywhere, or an in-place call off the boundaries
+};
+
+// One job's geometry. Columns are 16 bytes, column v at head + 16 v: the first
+// boundary of the sources, or the row's start (kAnyOff). Bytes outside the
+// columns that the vector path writes are "edges".
 struct LutGeom {
   uint64_t len, head, ncol;
   uint32_t k, nrows;
   uint32_t ovr;    // 1 = overwrite
-  uint32_t bytes;  // unaligned in-place job: columns are read and written bytewise
+  uint32_t bytes;  // kAnyOff, in place: columns are read and written bytewise
 };
 
-constexpr uint32_t kEdges = 5;  // edge columns of a job
-// First block an unaligned job's vector path writes: columns 0 and 1 and the
-// last two whole ones are edges (a source's granules may reach past them).
-constexpr uint64_t kUnalFirst = 2;
-// A warp of an unaligned job takes 32 columns and writes 30 blocks: lane 0's
-// column only supplies the bytes before lane 1's, and lane 31's 16 source
-// bytes only complete lane 30's.
-constexpr uint32_t kUnalStep = 30;
+constexpr uint32_t kEdges = 5;  // edge columns of a job, at most
 #ifdef __CUDACC__
 #define FGFC_HD __host__ __device__
 #else
 #define FGFC_HD
 #endif
-// Blocks of an unaligned job's vector path: v = kUnalFirst .. ncol - 2.
-FGFC_HD inline uint64_t lut_unal_blocks(uint64_t ncol) { return ncol >= 4 ? ncol - 3 : 0; }
+// Blocks of 16 row bytes that the vector path of an unaligned job writes: block
+// v ends inside column v and starts inside column v - 1, as far as the row's
+// offset goes back. kRowsOff: v = 1 .. ncol - 1. kAnyOff: v = 2 .. ncol - 2 (a
+// source's 16-byte granules may reach past the columns around those).
+FGFC_HD constexpr uint64_t lut_first_block(int mode) { return mode == kAnyOff ? 2 : 1; }
+FGFC_HD constexpr uint64_t lut_end_block(int mode, uint64_t ncol) { return mode == kAnyOff ? ncol - 1 : ncol; }
+FGFC_HD constexpr uint64_t lut_blocks(int mode, uint64_t ncol) {
+  return mode == kAnyOff ? (ncol >= 4 ? ncol - 3 : 0) : ncol >= 2 ? ncol - 1 : 0;
+}
+// Of a warp's 32 columns, lane 0's only supplies the bytes before lane 1's;
+// with unaligned sources lane 31's 16 bytes only complete lane 30's.
+FGFC_HD constexpr uint32_t lut_warp_blocks(int mode) { return mode == kAnyOff ? 30 : 31; }
 // Does the job leave bytes to the edge pass?
-FGFC_HD inline bool lut_has_edges(const LutGeom& g, bool unal) {
-  if (unal) return !g.bytes;
+FGFC_HD inline bool lut_has_edges(const LutGeom& g, int mode) {
+  if (mode != kAligned) return !g.bytes;
   return g.head != 0 || g.head + 16 * g.ncol != g.len;
 }
-// Tiles of a job for CTAs of `threads`: a column per thread, 30 blocks per
-// warp of an unaligned job.
-FGFC_HD inline uint64_t lut_tiles(const LutGeom& g, bool unal, uint32_t threads) {
-  if (!unal) return (g.ncol + threads - 1) / threads;
+// Tiles of a job for CTAs of `threads`: a column per thread, or the blocks of
+// its warps.
+FGFC_HD inline uint64_t lut_tiles(const LutGeom& g, int mode, uint32_t threads) {
+  if (mode == kAligned) return (g.ncol + threads - 1) / threads;
   if (g.bytes) return (g.len + 16 * threads - 1) / (16 * threads);
-  const uint32_t step = threads / 32 * kUnalStep;
-  return (lut_unal_blocks(g.ncol) + step - 1) / step;
+  const uint32_t step = threads / 32 * lut_warp_blocks(mode);
+  return (lut_blocks(mode, g.ncol) + step - 1) / step;
 }
 
 constexpr int kLutThreads = 256;
@@ -102,9 +110,10 @@ struct LutShape {
   size_t smem3() const { return (nv * w * 640 + 255) / 256 * 256; }     // table bytes of three sources
   size_t smem1() const { return (nv * w * 128 + 255) / 256 * 256; }     // and of one left over
 };
-// Shared memory of one CTA: tables of k sources and the staged edge columns.
+// Shared memory of one CTA: tables of k sources, the staged edge columns of
+// the sources and of the rows.
 inline uint32_t lut_smem(const LutShape& s, size_t k) {
-  return static_cast<uint32_t>(k / 3 * s.smem3() + k % 3 * s.smem1() + k * kEdges * 16);
+  return static_cast<uint32_t>(k / 3 * s.smem3() + k % 3 * s.smem1() + (k + kLutRows) * kEdges * 16);
 }
 inline size_t lut_rows(int E) { return E == 1 ? 16 : E == 2 ? 8 : 4; }
 LutShape lut_shape(int E, size_t nr);
@@ -116,8 +125,8 @@ size_t lut_image_words(int E, size_t k, size_t m);
 // coefficient matrix with m columns: [source][leaf byte][word][8].
 void build_lut_images(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t r0, size_t nr,
                       uint32_t* out);
-// Launch one job (rows of one lut_shape); `unal` as LutGeom describes.
-cudaError_t lut_launch(int field, size_t nr, LutArgs& a, bool unal, bool edges_only, cudaStream_t s);
+// Launch one job (rows of one lut_shape).
+cudaError_t lut_launch(int field, size_t nr, LutArgs& a, int mode, bool edges_only, cudaStream_t s);
 // One descriptor of a batched submission: a byte-table sub-job (batch.cu) or a
 // table sub-job (lut_batch.cuh).
 struct BatchJob {
@@ -147,15 +156,15 @@ struct LutBatchKernel {
   LutBatchFn fn = nullptr;
   int ctas = 1;  // resident per SM
 };
-LutBatchKernel lut_batch_kernel_for(int E, LutShape s, bool unal);
-LutBatchKernel lut_batch_e1(int lev, int w, bool unal);
-LutBatchKernel lut_batch_e2(int lev, int w, bool unal);
-LutBatchKernel lut_batch_e4(int lev, int w, bool unal);
-LutBatchKernel lut_batch_e8(int lev, int w, bool unal);
-cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
-cudaError_t lut_launch_e2(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
-cudaError_t lut_launch_e4(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
-cudaError_t lut_launch_e8(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only);
+LutBatchKernel lut_batch_kernel_for(int E, LutShape s, int mode);
+LutBatchKernel lut_batch_e1(int lev, int w, int mode);
+LutBatchKernel lut_batch_e2(int lev, int w, int mode);
+LutBatchKernel lut_batch_e4(int lev, int w, int mode);
+LutBatchKernel lut_batch_e8(int lev, int w, int mode);
+cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only);
+cudaError_t lut_launch_e2(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only);
+cudaError_t lut_launch_e4(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only);
+cudaError_t lut_launch_e8(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only);
 
 // The byte-table kernel (kernels.cu; Gf8, at most 4 rows, <= 14 sources) over
 // the vector body of a call; `overwrite` selects dot-product (overwrite) or
@@ -227,6 +236,7 @@ struct JobAlign {
   bool unal;      // a source or row is elsewhere
   bool overlap;   // a row shares bytes with a source
   uint64_t head;  // bytes before the sources' first boundary
+  LutMode mode;
 };
 JobAlign job_align(int field, const uint64_t* srcs, size_t k, const uint64_t* dsts, size_t m, uint64_t len);
 

@@ -494,16 +494,41 @@ __device__ __forceinline__ uint4 load_bytes16(const uint8_t* p, uint64_t off, ui
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Tiles first, first + step, ... of a job's ntiles: blockDim.x columns each, 30
-// blocks per warp of an unaligned job.
-template <class L, int LEV, int W, bool UNAL>
+// Tiles first, first + step, ... of a job: blockDim.x columns each, or the
+// blocks of an unaligned job's warps. Rows off the sources' boundaries (ragged
+// row lengths) have their own mode beside unaligned sources: no granules to
+// splice on the way in, one lane less lost, the aligned shapes' look-ahead and
+// occupancy. Over rows of the next aligned length, 4 MiB (unaligned sources'
+// path -> rows' own): Gf8D RS(20,8) +21 -> +7 %, Gf16 RS(18,8) +16 -> +6 %,
+// Gf16 RS(18,4) +19 -> +12 %; 256 mixed stripes, most of them ragged, 1685 ->
+// 1540 us.
+template <class L, int LEV, int W, int MODE>
 __device__ __forceinline__ void lut_run(const LutGeom& g, const LutShared& sh, uint64_t first, uint64_t step, bool ovr,
                                         bool fp) {
   constexpr int R = 4 / L::H;
-  const uint32_t k = g.k;
+  const uint32_t k = g.k, lane = threadIdx.x & 31u;
   LutAcc<L, W> A;
   uint32_t f[W][L::NF];
-  if constexpr (!UNAL) {
+  // rows of an unaligned job: lane l holds column c, lanes 1 .. write block c
+  const auto store_blocks = [&](uint64_t off, bool valid) {
+#pragma unroll
+    for (int q = 0; q < W; ++q)
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint32_t row = q * R + r;
+        if (row >= g.nrows) continue;
+        const uint4 o = lut_row<L>(f[q], r);
+        uint8_t* const d = sh.dst[row] + off;
+        const uint32_t dl = static_cast<uint32_t>(reinterpret_cast<uint64_t>(d)) & 15u;  // one for the warp
+        if (dl == 0) {
+          if (valid) put16(d, o, ovr);
+        } else {
+          const uint4 b = splice16(shfl_up4(o), o, 16u - dl);
+          if (valid) put16(d - dl, b, ovr);
+        }
+      }
+  };
+  if constexpr (MODE == kAligned) {
     if constexpr (kLutAhead<L, W>) {
       const uint64_t end = g.head + 16 * g.ncol, stride = 16 * step * blockDim.x;
       uint64_t off = g.head + 16 * (first * blockDim.x + threadIdx.x);
@@ -523,7 +548,7 @@ __device__ __forceinline__ void lut_run(const LutGeom& g, const LutShared& sh, u
         off = noff;
       }
     } else {
-      const uint64_t ntiles = lut_tiles(g, false, blockDim.x);
+      const uint64_t ntiles = lut_tiles(g, MODE, blockDim.x);
       for (uint64_t tile = first; tile < ntiles; tile += step) {
         const uint64_t v = tile * blockDim.x + threadIdx.x;
         if (v >= g.ncol) return;
@@ -531,6 +556,38 @@ __device__ __forceinline__ void lut_run(const LutGeom& g, const LutShared& sh, u
         lut_column<L, W>(A, g.k, [&](uint32_t t) { return ldg16(sh.src[t] + o); }, LutAsIs());
         lut_finish<L, W, LEV>(A, f, fp);
         lut_store<L, W>(f, sh, g.nrows, o, ovr);
+      }
+    }
+  } else if constexpr (MODE == kRowsOff) {
+    const uint32_t warps = blockDim.x >> 5;
+    const uint64_t stride = step * warps * lut_warp_blocks(MODE);
+    uint64_t v = lut_first_block(MODE) + (first * warps + (threadIdx.x >> 5)) * lut_warp_blocks(MODE);  // lane 1's
+    // lanes past the last column read it again
+    const auto column = [&](uint64_t c) { return g.head + 16 * (c < g.ncol ? c : g.ncol - 1); };
+    if constexpr (kLutAhead<L, W>) {
+      if (v >= g.ncol) return;
+      LutAhead h;
+      uint64_t off = column(v - 1 + lane);
+#pragma unroll
+      for (uint32_t j = 0; j < 3; ++j) h.c[j] = j < k ? ldg16(sh.src[j] + off) : make_uint4(0, 0, 0, 0);
+      for (;;) {
+        const uint64_t nv = v + stride, noff = column(nv - 1 + lane);
+        const bool more = nv < g.ncol;
+        lut_column_ahead<L, W>(
+            A, k, h, [&](uint32_t t) { return ldg16(sh.src[t] + off); },
+            [&](uint32_t t) { return more ? ldg16(sh.src[t] + noff) : make_uint4(0, 0, 0, 0); }, LutAsIs());
+        lut_finish<L, W, LEV>(A, f, fp);
+        store_blocks(off, lane >= 1 && v - 1 + lane < g.ncol);
+        if (!more) return;
+        v = nv;
+        off = noff;
+      }
+    } else {
+      for (; v < g.ncol; v += stride) {
+        const uint64_t off = column(v - 1 + lane);
+        lut_column<L, W>(A, k, [&](uint32_t t) { return ldg16(sh.src[t] + off); }, LutAsIs());
+        lut_finish<L, W, LEV>(A, f, fp);
+        store_blocks(off, lane >= 1 && v - 1 + lane < g.ncol);
       }
     }
   } else if (g.bytes) {  // each thread reads and writes only its own column
@@ -546,10 +603,10 @@ __device__ __forceinline__ void lut_run(const LutGeom& g, const LutShared& sh, u
             put_bytes(sh.dst[q * R + r] + off, lut_row<L>(f[q], r), 0, nb, ovr);
     }
   } else {
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    // lane l's column is v - 1 + l, blocks end before column ncol - 1
-    const uint64_t end = g.ncol - 1, stride = step * (blockDim.x >> 5) * kUnalStep;
-    for (uint64_t v = kUnalFirst + (first * (blockDim.x >> 5) + warp) * kUnalStep; v < end; v += stride) {
+    const uint32_t warps = blockDim.x >> 5;
+    const uint64_t end = lut_end_block(MODE, g.ncol), stride = step * warps * lut_warp_blocks(MODE);
+    uint64_t v = lut_first_block(MODE) + (first * warps + (threadIdx.x >> 5)) * lut_warp_blocks(MODE);
+    for (; v < end; v += stride) {
       const uint64_t c = v - 1 + lane;
       // A granule past the last whole one belongs to no column that is written.
       lut_column<L, W>(
@@ -566,93 +623,86 @@ __device__ __forceinline__ void lut_run(const LutGeom& g, const LutShared& sh, u
             return s == 0 ? x : splice16(x, shfl_down4(x), s);
           });
       lut_finish<L, W, LEV>(A, f, fp);
-      const bool valid = lane >= 1 && lane <= kUnalStep && c < end;
-#pragma unroll
-      for (int q = 0; q < W; ++q)
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const uint32_t row = q * R + r;
-          if (row >= g.nrows) continue;
-          const uint4 o = lut_row<L>(f[q], r);
-          const uint32_t dl = static_cast<uint32_t>(reinterpret_cast<uint64_t>(sh.dst[row])) & 15u;
-          if (dl == 0) {
-            if (valid) put16(sh.dst[row] + 16 * c, o, ovr);
-          } else {
-            const uint4 b = splice16(shfl_up4(o), o, 16u - dl);
-            if (valid) put16(sh.dst[row] + 16 * c - dl, b, ovr);
-          }
-        }
+      store_blocks(16 * c, lane >= 1 && lane <= lut_warp_blocks(MODE) && c < end);
     }
   }
 }
 
 // Start of edge column j of a job, its bytes (0 = none).
-__device__ __forceinline__ uint64_t lut_edge(const LutGeom& g, bool unal, uint32_t j, uint32_t* nb) {
+__device__ __forceinline__ uint64_t lut_edge(const LutGeom& g, int mode, uint32_t j, uint32_t* nb) {
+  const uint64_t tail = g.head + 16 * g.ncol;
   uint64_t st = 0, n = 0;
-  if (!unal) {
-    if (j == 0) {
-      n = g.head;
-    } else if (j == 1) {
-      st = g.head + 16 * g.ncol;
-      n = g.len - st;
-    }
-  } else {
+  if (mode == kAnyOff) {
     // columns 0, 1 and ncol - 2, ncol - 1, ncol, each once
     const uint64_t lo = g.ncol >= 4 ? g.ncol - 2 : 2;
     st = 16 * (j < 2 ? j : lo + (j - 2));
     n = st < g.len ? g.len - st : 0;
     if (n > 16) n = 16;
+  } else if (j == 0) {
+    n = g.head;
+  } else if (j == 1) {
+    st = tail;
+    n = g.len - tail;
+  } else if (mode == kRowsOff && g.ncol >= j - 1 && j < 4) {  // the first and the last column
+    st = j == 2 ? g.head : tail - 16;
+    n = 16;
   }
   *nb = static_cast<uint32_t>(n);
   return st;
 }
 
-// The edge columns of a job, by one CTA: all bytes are staged in shared
-// memory with independent byte loads, one thread folds a column and writes
-// its bytes. `stage` holds kMaxSrc * kEdges * 16 bytes.
-template <class L, int LEV, int W, bool UNAL>
+// The edge columns of a job, by one CTA: a thread stages a source's column with
+// 16 independent byte loads, one thread folds a column, a thread writes a
+// row's column. `stage` holds (kMaxSrc + kLutRows) * kEdges * 16 bytes.
+template <class L, int LEV, int W, int MODE>
 __device__ __forceinline__ void lut_edges(const LutGeom& g, const LutShared& sh, uint8_t* stage, bool ovr, bool fp) {
   constexpr int R = 4 / L::H;
-  for (uint32_t i = threadIdx.x; i < g.k * kEdges * 16u; i += blockDim.x) {
-    const uint32_t t = i / (kEdges * 16u), j = (i / 16u) % kEdges, b = i & 15u;
+  for (uint32_t i = threadIdx.x; i < g.k * kEdges; i += blockDim.x) {
     uint32_t nb;
-    const uint64_t st = lut_edge(g, UNAL, j, &nb);
-    stage[i] = b < nb ? sh.src[t][st + b] : 0;
+    const uint64_t st = lut_edge(g, MODE, i % kEdges, &nb);
+    reinterpret_cast<uint4*>(stage)[i] = load_bytes16(sh.src[i / kEdges] + st, 0, nb);
   }
   __syncthreads();
+  uint8_t* const out = stage + g.k * kEdges * 16u;  // [row][edge][16]
   if (threadIdx.x < kEdges) {
     const uint32_t j = threadIdx.x;
     uint32_t nb;
-    const uint64_t st = lut_edge(g, UNAL, j, &nb);
+    lut_edge(g, MODE, j, &nb);
     if (nb) {
       LutAcc<L, W> A;
       uint32_t f[W][L::NF];
-      const auto load = [&](uint32_t t) { return reinterpret_cast<const uint4*>(stage)[t * kEdges + j]; };
-      lut_column<L, W>(A, g.k, load, LutAsIs());
+      lut_column<L, W>(A, g.k, [&](uint32_t t) { return reinterpret_cast<const uint4*>(stage)[t * kEdges + j]; },
+                       LutAsIs());
       lut_finish<L, W, LEV>(A, f, fp);
 #pragma unroll
       for (int q = 0; q < W; ++q)
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const uint32_t row = q * R + r;
-          if (row >= g.nrows) continue;
-          const uint4 o = lut_row<L>(f[q], r);
-          uint8_t* const d = sh.dst[row];
-          uint32_t b0 = 0, b1 = nb;
-          if (UNAL && lut_unal_blocks(g.ncol)) {
-            // the vector path wrote [16 kUnalFirst - dl, 16 (ncol - 1) - dl)
-            const uint32_t dl = static_cast<uint32_t>(reinterpret_cast<uint64_t>(d)) & 15u;
-            const uint64_t w0 = 16 * kUnalFirst - dl, w1 = 16 * (g.ncol - 1) - dl;
-            if (st < w1) {  // ahead of the written range, or straddling one of its ends
-              if (st >= w0)
-                b0 = w1 - st < nb ? static_cast<uint32_t>(w1 - st) : nb;
-              else if (w0 - st < nb)
-                b1 = static_cast<uint32_t>(w0 - st);
-            }
-          }
-          if (b0 < b1) put_bytes(d + st + b0, o, b0, b1, ovr);
-        }
+        for (int r = 0; r < R; ++r)
+          if (static_cast<uint32_t>(q * R + r) < g.nrows)
+            reinterpret_cast<uint4*>(out)[(q * R + r) * kEdges + j] = lut_row<L>(f[q], r);
     }
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < g.nrows * kEdges; i += blockDim.x) {
+    uint32_t nb;
+    const uint64_t st = lut_edge(g, MODE, i % kEdges, &nb);
+    uint8_t* const d = sh.dst[i / kEdges];
+    uint32_t b0 = 0, b1 = nb;
+    if (MODE != kAligned && lut_blocks(MODE, g.ncol)) {
+      // the vector path wrote [w0, w1): no column reaches past both ends
+      const uint32_t dl = static_cast<uint32_t>(reinterpret_cast<uint64_t>(d) + g.head) & 15u;
+      const uint64_t w0 = g.head + 16 * lut_first_block(MODE) - dl, w1 = g.head + 16 * lut_end_block(MODE, g.ncol) - dl;
+      if (st >= w0 && st < w1)
+        b0 = w1 - st < nb ? static_cast<uint32_t>(w1 - st) : nb;
+      else if (st < w0 && w0 - st < nb)
+        b1 = static_cast<uint32_t>(w0 - st);
+    }
+    uint4 o = reinterpret_cast<const uint4*>(out)[i];
+    if (!ovr && b0 < b1) {
+      const uint4 x = load_bytes16(d + st, 0, nb);
+      o.x ^= x.x, o.y ^= x.y, o.z ^= x.z, o.w ^= x.w;
+    }
+    if (b0 < b1) put_bytes(d + st + b0, o, b0, b1, true);
   }
 }
 

@@ -10,8 +10,8 @@ namespace fgfc {
 // item is claimed before the current one is worked on, and the tables are
 // refilled (a few KiB) only where the plan changes. Sources past kc (one fill's
 // limit) accumulate in further rounds over the same tiles.
-template <int E, int LEV, int W, bool UNAL>
-__global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, UNAL>())
+template <int E, int LEV, int W, int MODE>
+__global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, MODE>())
     lut_batch_kernel(const BatchDesc* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
                      const uint2* __restrict__ items, uint32_t nitems, uint32_t* counter, uint32_t kc) {
   using L = Lut<E, LEV>;
@@ -51,10 +51,10 @@ __global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, UNAL>())
       __syncthreads();
       const bool ovr = s_job.g.ovr != 0, fp = s_job.fp != 0;
       if (wi.y < s_job.parts) {
-        lut_run<L, LEV, W, UNAL>(s_job.g, sh, wi.y, s_job.parts, ovr, fp);
+        lut_run<L, LEV, W, MODE>(s_job.g, sh, wi.y, s_job.parts, ovr, fp);
       } else {
         uint8_t* stage = g_smem + kk / 3u * S::block3 + kk % 3u * S::block1;
-        lut_edges<L, LEV, W, UNAL>(s_job.g, sh, stage, ovr, fp);
+        lut_edges<L, LEV, W, MODE>(s_job.g, sh, stage, ovr, fp);
       }
     }
     __syncthreads();  // done with tables, pointers and s_item
@@ -62,10 +62,14 @@ __global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, UNAL>())
 }
 
 template <int E, int LEV, int W>
-LutBatchKernel lut_batch_lw(bool unal) {
+LutBatchKernel lut_batch_lw(int mode) {
   LutBatchKernel b;
-  b.fn = unal ? lut_batch_kernel<E, LEV, W, true> : lut_batch_kernel<E, LEV, W, false>;
-  b.ctas = unal ? lut_min_ctas<E, LEV, W, true>() : lut_min_ctas<E, LEV, W, false>();
+  b.fn = mode == kAligned   ? lut_batch_kernel<E, LEV, W, kAligned>
+         : mode == kRowsOff ? lut_batch_kernel<E, LEV, W, kRowsOff>
+                            : lut_batch_kernel<E, LEV, W, kAnyOff>;
+  b.ctas = mode == kAligned   ? lut_min_ctas<E, LEV, W, kAligned>()
+           : mode == kRowsOff ? lut_min_ctas<E, LEV, W, kRowsOff>()
+                              : lut_min_ctas<E, LEV, W, kAnyOff>();
   return b;
 }
 

@@ -3,19 +3,19 @@
 
 namespace fgfc {
 
-cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, bool unal, bool edges_only) {
-  if (lev == 0 && w == 1) return lut_launch_lw<1, 0, 1>(a, s, unal, edges_only);
-  if (lev == 0 && w == 2) return lut_launch_lw<1, 0, 2>(a, s, unal, edges_only);
-  if (lev == 0 && w == 3) return lut_launch_lw<1, 0, 3>(a, s, unal, edges_only);
-  if (lev == 0 && w == 4) return lut_launch_lw<1, 0, 4>(a, s, unal, edges_only);
+cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only) {
+  if (lev == 0 && w == 1) return lut_launch_lw<1, 0, 1>(a, s, mode, edges_only);
+  if (lev == 0 && w == 2) return lut_launch_lw<1, 0, 2>(a, s, mode, edges_only);
+  if (lev == 0 && w == 3) return lut_launch_lw<1, 0, 3>(a, s, mode, edges_only);
+  if (lev == 0 && w == 4) return lut_launch_lw<1, 0, 4>(a, s, mode, edges_only);
   return cudaErrorInvalidValue;
 }
 
-LutBatchKernel lut_batch_e1(int lev, int w, bool unal) {
-  if (lev == 0 && w == 1) return lut_batch_lw<1, 0, 1>(unal);
-  if (lev == 0 && w == 2) return lut_batch_lw<1, 0, 2>(unal);
-  if (lev == 0 && w == 3) return lut_batch_lw<1, 0, 3>(unal);
-  if (lev == 0 && w == 4) return lut_batch_lw<1, 0, 4>(unal);
+LutBatchKernel lut_batch_e1(int lev, int w, int mode) {
+  if (lev == 0 && w == 1) return lut_batch_lw<1, 0, 1>(mode);
+  if (lev == 0 && w == 2) return lut_batch_lw<1, 0, 2>(mode);
+  if (lev == 0 && w == 3) return lut_batch_lw<1, 0, 3>(mode);
+  if (lev == 0 && w == 4) return lut_batch_lw<1, 0, 4>(mode);
   return LutBatchKernel{};
 }
 

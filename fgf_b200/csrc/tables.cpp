@@ -53,8 +53,8 @@ LutShape lut_shape(int E, size_t nr) {
 
 size_t lut_sources(int E, size_t nr, bool inl) {
   const LutShape s = lut_shape(E, nr);
-  const size_t edge = 5 * 16;  // staged edge columns per source
-  size_t kc = std::min<size_t>(kMaxSrc, kLutSmemMax / (s.smem3() + 3 * edge) * 3);
+  const size_t edge = kEdges * 16;  // staged edge columns per source and row
+  size_t kc = std::min<size_t>(kMaxSrc, (kLutSmemMax - kLutRows * edge) / (s.smem3() + 3 * edge) * 3);
   if (inl) kc = std::min<size_t>(kc, kLutInlineWords / s.src_words());
   return kc;
 }
@@ -110,31 +110,31 @@ void build_lut_images(int field, const uint64_t* coeffs, size_t m, size_t t0, si
     }
 }
 
-cudaError_t lut_launch(int field, size_t nr, LutArgs& a, bool unal, bool edges_only, cudaStream_t s) {
+cudaError_t lut_launch(int field, size_t nr, LutArgs& a, int mode, bool edges_only, cudaStream_t s) {
   const int E = field_bytes(field);
   const LutShape sh = lut_shape(E, nr);
   a.fp = field == kFp16 || field == kFp32 || field == kFp64 ? 1u : 0u;
   switch (E) {
-    case 1: return lut_launch_e1(sh.lev, sh.w, a, s, unal, edges_only);
-    case 2: return lut_launch_e2(sh.lev, sh.w, a, s, unal, edges_only);
-    case 4: return lut_launch_e4(sh.lev, sh.w, a, s, unal, edges_only);
-    case 8: return lut_launch_e8(sh.lev, sh.w, a, s, unal, edges_only);
+    case 1: return lut_launch_e1(sh.lev, sh.w, a, s, mode, edges_only);
+    case 2: return lut_launch_e2(sh.lev, sh.w, a, s, mode, edges_only);
+    case 4: return lut_launch_e4(sh.lev, sh.w, a, s, mode, edges_only);
+    case 8: return lut_launch_e8(sh.lev, sh.w, a, s, mode, edges_only);
     default: return cudaErrorInvalidValue;
   }
 }
 
-LutBatchKernel lut_batch_kernel_for(int E, LutShape s, bool unal) {
+LutBatchKernel lut_batch_kernel_for(int E, LutShape s, int mode) {
   switch (E) {
-    case 1: return lut_batch_e1(s.lev, s.w, unal);
-    case 2: return lut_batch_e2(s.lev, s.w, unal);
-    case 4: return lut_batch_e4(s.lev, s.w, unal);
-    case 8: return lut_batch_e8(s.lev, s.w, unal);
+    case 1: return lut_batch_e1(s.lev, s.w, mode);
+    case 2: return lut_batch_e2(s.lev, s.w, mode);
+    case 4: return lut_batch_e4(s.lev, s.w, mode);
+    case 8: return lut_batch_e8(s.lev, s.w, mode);
     default: return LutBatchKernel{};
   }
 }
 
 JobAlign job_align(int field, const uint64_t* srcs, size_t k, const uint64_t* dsts, size_t m, uint64_t len) {
-  JobAlign r{true, false, false, 0};
+  JobAlign r{true, false, false, 0, kAligned};
   const uint64_t al = k ? srcs[0] & 15 : 0;
   for (size_t t = 0; t < k; ++t) r.sources = r.sources && (srcs[t] & 15) == al;
   r.sources = r.sources && al % static_cast<uint64_t>(field_bytes(field)) == 0;
@@ -144,6 +144,7 @@ JobAlign job_align(int field, const uint64_t* srcs, size_t k, const uint64_t* ds
     for (size_t j = 0; j < m; ++j)
       for (size_t t = 0; t < k; ++t) r.overlap = r.overlap || (dsts[j] < srcs[t] + len && srcs[t] < dsts[j] + len);
   if (r.sources) r.head = std::min<uint64_t>((16 - al) & 15, len);
+  r.mode = !r.unal ? kAligned : r.sources && !r.overlap ? kRowsOff : kAnyOff;
   return r;
 }
 
