@@ -17,6 +17,7 @@
 // vectors coalesce: vector j of lane l is base + 32 j + l.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "fast_core.cuh"
@@ -295,9 +296,14 @@ cudaError_t launch(uint8_t* dst, const uint8_t* a, const uint8_t* b, uint64_t le
   const uint64_t sms = static_cast<uint64_t>(sm_count());
   // Short vectors take one-warp CTAs, so that every SM gets one.
   const unsigned threads = nblocks < 4 * sms ? 32 : 128;
-  int occ = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, elementwise_planes_kernel<E, F>, threads, 0);
-  if (e != cudaSuccess) return e;
+  // Resident CTAs, asked for once: every device here is the same chip.
+  static std::atomic<int> resident[2];
+  int occ = resident[threads == 32].load(std::memory_order_relaxed);
+  if (occ == 0) {
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, elementwise_planes_kernel<E, F>, threads, 0);
+    if (e != cudaSuccess) return e;
+    resident[threads == 32].store(occ, std::memory_order_relaxed);
+  }
   const uint64_t want = (nblocks + threads / 32 - 1) / (threads / 32), cap = sms * static_cast<uint64_t>(occ < 1 ? 1 : occ);
   elementwise_planes_kernel<E, F>
       <<<static_cast<unsigned>(want < cap ? want : cap), threads, 0, s>>>(dst, a, b, len, head, nvec);

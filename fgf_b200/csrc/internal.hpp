@@ -89,7 +89,7 @@ FGFC_HD inline uint64_t lut_tiles(const LutGeom& g, int mode, uint32_t threads) 
 
 constexpr int kLutThreads = 256;
 constexpr int kLutRows = 16;               // rows per launch (Gf8; 8 / 4 / 4 for 2, 4 and 8 bytes)
-constexpr int kLutInlineWords = 1536;      // images carried in launch parameters
+constexpr int kLutInlineWords = 768;       // images carried in launch parameters: 3 of their 4 KiB
 constexpr int kLutSmemMax = 110 * 1024;    // tables of one CTA: two CTAs per SM
 struct LutArgs {
   const uint32_t* img;  // device images, or nullptr: inl
@@ -101,6 +101,7 @@ struct LutArgs {
   uint8_t* dst[kLutRows];
   alignas(16) uint32_t inl[kLutInlineWords];
 };
+static_assert(sizeof(LutArgs) <= 4096, "launches with more than 4 KiB of parameters cost more");
 
 // Tower levels split and output words per leaf product of a launch of nr rows.
 struct LutShape {

@@ -15,6 +15,8 @@ arguments through the C ABI (include/fgf_cuda.h).
 from __future__ import annotations
 
 import ctypes as C
+import sys
+from array import array
 from typing import Iterable, Sequence
 
 from ._lib import FgfError, Slice, Term, check, lib
@@ -50,14 +52,11 @@ def _buf(x) -> tuple[int, int]:
 
 def _stream(stream) -> int:
     if stream is None:
-        try:
-            import torch
-
-            if torch.cuda.is_available() and torch.cuda.is_initialized():
-                return int(torch.cuda.current_stream().cuda_stream)
-        except ImportError:
-            pass
-        return 0
+        torch = sys.modules.get("torch")
+        if torch is None or not torch.cuda.is_initialized():
+            return 0
+        # the handle of torch.cuda.current_stream(), without building a Stream object
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     if hasattr(stream, "cuda_stream"):
         return int(stream.cuda_stream)
     return int(stream)
@@ -80,21 +79,20 @@ def _wide(field) -> bool:
     return FIELDS[_fid(field)].BYTES == 8
 
 
-_SLICE_WORDS: dict = {}
+_SLICE_TYPES: dict = {}
 
 
 def _slices(srcs: Sequence):
-    """fgfc_slice array of the sources: built as one flat array of (pointer,
-    length) words (one ctypes object instead of one per source) and viewed
-    as the struct array, which keeps the words alive."""
-    flat = []
+    """fgfc_slice array of the sources: a flat array of (pointer, length)
+    words viewed as the struct array, which keeps the words alive."""
+    flat: list[int] = []
     for s in srcs:
-        flat.extend(_buf(s))
+        flat += _buf(s)
     n = len(flat) // 2
-    typ = _SLICE_WORDS.get(n)
+    typ = _SLICE_TYPES.get(n)
     if typ is None:
-        typ = _SLICE_WORDS[n] = C.c_uint64 * max(2, 2 * n)
-    return C.cast(typ(*flat), C.POINTER(Slice)), n
+        typ = _SLICE_TYPES[n] = Slice * max(1, n)
+    return typ.from_buffer(array("Q", flat or (0, 0))), n
 
 
 def _terms(terms: Sequence) -> tuple[C.Array, int, list]:
