@@ -25,12 +25,12 @@
 // need enough rows to fill the word, which is the rule of lut_shape().
 //
 // What bounds it: the lookups (one shared-memory wavefront each) and, with one
-// word per product, as many ALU operations around them (address PRMT, XOR,
-// index masks). Measured on B200 against the kernels it replaced, with 32
+// word per product, the issue slots of the operations around them (address dot
+// product, XOR, index masks). Measured on B200 against the kernels it replaced, with 32
 // table copies per lane (or unreplicated nibbles for 8-byte elements):
-//   GF(2^64) RS(10,4), 16 MiB shards     308 -> 206 us (lookups per element 992 -> 483)
+//   GF(2^64) RS(10,4), 16 MiB shards     308 -> 173 us (lookups per element 992 -> 483)
 //   256 stripes of Gf8D and Gf16, k 4..32, m 1..8, 4 KiB .. 4 MiB, one batch
-//                                        3260 -> 1711 us (more CTAs resident, no 216 KiB refills)
+//                                        3260 -> 1540 us (more CTAs resident, no 216 KiB refills)
 //   Gf8D RS(12,4), 1000003-byte shards at any offset, 18 -> 4 us on the device
 //   (whole-element bytes one at a time before, 16-byte granules spliced now)
 #pragma once
@@ -55,10 +55,9 @@ struct Lut {
   static constexpr int NE = 16 / E;           // elements per 16-byte column
   static constexpr int NW = (NE * NV + 3) / 4;  // packed words of leaf input bytes per column
   static constexpr int NF = 16 / H;           // accumulator words per column after the fix-up
-  // Index shifts on the multiply pipe: where the ALU work per lookup is the
-  // largest (GF(2^64) RS(10,4), 16 MiB: 204 -> 194 us). 2-byte towers gain 1 %,
-  // 4-byte ones nothing, and the lookup-bound 1-byte shapes lose up to 5 %.
-  static constexpr bool kMulShift = E == 8 || (E == 2 && LEV == 1);
+  // Index shifts on the multiply pipe: GF(2^64) RS(10,4), 16 MiB, 204 -> 173 us;
+  // level or worse for the other widths.
+  static constexpr bool kMulShift = E == 8;
 
   // element and leaf byte (product * H + byte) of byte b of packed word w;
   // elem() < 0: no byte there
@@ -122,9 +121,8 @@ struct Lut {
 
 // Shared-memory tables: per 3 sources five 32-word tables for each (leaf
 // byte, output word), then two 16-word nibble tables per (leaf byte, output
-// word) for each of the k % 3 sources left. Blocks start on 256 bytes, so an
-// address is the block's base with its low byte replaced by the index (one
-// PRMT) plus an immediate.
+// word) for each of the k % 3 sources left. An address is the block's base plus
+// 4 times the index (lut_addr) plus an immediate.
 template <int NV, int W>
 struct LutSmem {
   static constexpr uint32_t block3 = (NV * W * 640u + 255u) / 256u * 256u;
@@ -183,7 +181,16 @@ struct LutAcc {
   }
 };
 
-// Three sources whose tables start at `base` (a multiple of 256).
+// base + M times byte b of x. A dot product of bytes with one nonzero factor:
+// it runs beside the ALU pipe, which a PRMT per lookup kept at 80 % (PRMT ->
+// dot product: GF(2^64) RS(10,4) 16 MiB 190 -> 173 us, Gf32 RS(16,4) 8 MiB
+// 86 -> 79, Gf16 RS(12,4) 4 MiB 27.8 -> 24.8, Gf8D RS(20,4) 4 MiB 29.2 -> 28.5).
+template <uint32_t M>
+__device__ __forceinline__ uint32_t lut_addr(uint32_t x, uint32_t base, int b) {
+  return __dp4a(x, M << (8 * b), base);
+}
+
+// Three sources whose tables start at `base`.
 template <class L, int W>
 __device__ __forceinline__ void lut_fold3(const uint4& c0, const uint4& c1, const uint4& c2, uint32_t base,
                                           LutAcc<L, W>& A) {
@@ -194,17 +201,15 @@ __device__ __forceinline__ void lut_fold3(const uint4& c0, const uint4& c1, cons
   const Shift<L::kMulShift> sh;
 #pragma unroll
   for (int w = 0; w < L::NW; ++w) {
-    const uint32_t i0 = sh.shl(v0[w], 2) & 0x7C7C7C7Cu, i1 = sh.shl(v1[w], 2) & 0x7C7C7C7Cu,
-                   i2 = sh.shl(v2[w], 2) & 0x7C7C7C7Cu;
+    const uint32_t i0 = v0[w] & 0x1F1F1F1Fu, i1 = v1[w] & 0x1F1F1F1Fu, i2 = v2[w] & 0x1F1F1F1Fu;
     const uint32_t i3 = (sh.shr(v0[w], 3) & 0x1C1C1C1Cu) | (v1[w] & 0x60606060u);
     const uint32_t i4 = (sh.shr(v2[w], 3) & 0x1C1C1C1Cu) | (sh.shr(v1[w], 2) & 0x20202020u);
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       if (L::elem(w, b) < 0) continue;
       const int e = L::elem(w, b), vb = L::vb(w, b), p = vb / L::H;
-      const uint32_t sel = 0x7650u | static_cast<uint32_t>(b);
-      const uint32_t q0 = prmt(i0, base, sel), q1 = prmt(i1, base, sel), q2 = prmt(i2, base, sel),
-                     q3 = prmt(i3, base, sel), q4 = prmt(i4, base, sel);
+      const uint32_t q0 = lut_addr<4>(i0, base, b), q1 = lut_addr<4>(i1, base, b), q2 = lut_addr<4>(i2, base, b),
+                     q3 = lut_addr<1>(i3, base, b), q4 = lut_addr<1>(i4, base, b);
 #pragma unroll
       for (int g = 0; g < W; ++g) {
         const uint32_t o = (vb * W + g) * 640u;
@@ -224,13 +229,12 @@ __device__ __forceinline__ void lut_fold1(const uint4& c0, uint32_t base, LutAcc
   const Shift<L::kMulShift> sh;
 #pragma unroll
   for (int w = 0; w < L::NW; ++w) {
-    const uint32_t i0 = sh.shl(v0[w], 2) & 0x3C3C3C3Cu, i1 = sh.shr(v0[w], 2) & 0x3C3C3C3Cu;
+    const uint32_t i0 = v0[w] & 0x0F0F0F0Fu, i1 = sh.shr(v0[w], 2) & 0x3C3C3C3Cu;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       if (L::elem(w, b) < 0) continue;
       const int e = L::elem(w, b), vb = L::vb(w, b), p = vb / L::H;
-      const uint32_t sel = 0x7650u | static_cast<uint32_t>(b);
-      const uint32_t q0 = prmt(i0, base, sel), q1 = prmt(i1, base, sel);
+      const uint32_t q0 = lut_addr<4>(i0, base, b), q1 = lut_addr<1>(i1, base, b);
 #pragma unroll
       for (int g = 0; g < W; ++g) {
         const uint32_t o = (vb * W + g) * 128u;
