@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
   if (threadIdx.x == 0) {
     s_tab = nullptr;
   }
-  const FastRegs r;
+  const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_item = atomicAdd(counter, kClaim);
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
       if (threadIdx.x < K) s_src[threadIdx.x] = reinterpret_cast<const uint8_t*>(ptrs[J.src_idx + threadIdx.x]);
       if (threadIdx.x < J.nrows) s_dst[threadIdx.x] = reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + threadIdx.x]);
       if (!resident) {
-        fill_fast<K>(J.tables, nullptr);
+        fill_fast<K, kByteSrcBatch>(J.tables, nullptr);
         if (threadIdx.x == 0) {
           s_tab = J.tables;
         }
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
           uint32_t acc[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e) acc[e] = 0;
-          fast_fold<K, 4>(w, acc, r);
+          fast_fold<K, kByteSrcBatch, 4>(w, acc, lane4);
           if constexpr (SHIFT)
             store_col4_any(acc, s_dst, J.nrows, off, ovr, valid);
           else
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
             w[t][0] = x;
           }
           uint32_t acc[4] = {0, 0, 0, 0};
-          fast_fold<K, 1>(w, acc, r);
+          fast_fold<K, kByteSrcBatch, 1>(w, acc, lane4);
           for (uint32_t rr = 0; rr < J.nrows; ++rr) {
             const uint32_t o = row_word4(acc, static_cast<int>(rr));
             uint8_t* d = s_dst[rr] + off;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
   if (threadIdx.x == 0) {
     s_tab = nullptr;
   }
-  const FastRegs r;
+  const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
   const uint32_t lane = threadIdx.x & 31u;
   while (v0 < v1) {
     while (vprefix[q + 1] <= v0) ++q;  // sub-jobs without vectors
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
     if (threadIdx.x < K) s_src[threadIdx.x] = reinterpret_cast<const uint8_t*>(ptrs[J.src_idx + threadIdx.x]);
     if (threadIdx.x < J.nrows) s_dst[threadIdx.x] = reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + threadIdx.x]);
     if (!resident) {
-      fill_fast<K>(J.tables, nullptr);
+      fill_fast<K, kByteSrcBatch>(J.tables, nullptr);
       if (threadIdx.x == 0) {
         s_tab = J.tables;
       }
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
       uint32_t acc[16];
 #pragma unroll
       for (int e = 0; e < 16; ++e) acc[e] = 0;
-      fast_fold<K, 4>(w, acc, r);
+      fast_fold<K, kByteSrcBatch, 4>(w, acc, lane4);
       if constexpr (SHIFT)
         store_col4_any(acc, s_dst, J.nrows, off, ovr, valid);
       else
@@ -254,8 +254,8 @@ static_assert(sizeof(UniformParams) <= 32000, "launch parameter block too large"
 template <int K, bool SHIFT>
 __global__ void __launch_bounds__(kFastThreads, 1)
     batch_fast_uniform_kernel(const __grid_constant__ UniformParams P) {
-  fill_fast<K>(P.tables, nullptr);
-  const FastRegs r;
+  fill_fast<K, kByteSrcBatch>(P.tables, nullptr);
+  const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const uint64_t vtotal = P.vprefix[P.njobs];
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
     uint32_t acc[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = 0;
-    fast_fold<K, 4>(w, acc, r);
+    fast_fold<K, kByteSrcBatch, 4>(w, acc, lane4);
     if constexpr (SHIFT)
       store_col4_any(acc, J.dst, J.nrows, off, J.ovr != 0, valid);
     else
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
       w[t][0] = x;
     }
     uint32_t acc[4] = {0, 0, 0, 0};
-    fast_fold<K, 1>(w, acc, r);
+    fast_fold<K, kByteSrcBatch, 1>(w, acc, lane4);
     for (uint32_t rr = 0; rr < J.nrows; ++rr) {
       const uint32_t o = row_word4(acc, static_cast<int>(rr));
       uint8_t* d = J.dst[rr] + off;
@@ -367,7 +367,7 @@ UniformFn uniform_kernel_for(int K, bool shift) {
 uint32_t fast_smem(int K) {
   switch (K) {
 #define FGFC_CASE(k) \
-  case k: return FastLayout<k>::smem;
+  case k: return FastLayout<k, kByteSrcBatch>::smem;
     FGFC_K_CASES(FGFC_CASE)
 #undef FGFC_CASE
     default: return 0;

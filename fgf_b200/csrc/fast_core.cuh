@@ -51,23 +51,29 @@ __device__ __forceinline__ void prefetch_l2(const uint8_t* p) { asm volatile("pr
 //
 // Gf8 fields with at most 4 rows (one table group) and a compile-time number
 // of sources K. Sources t < kByteSrc get a full 256-entry product table (one
-// lookup per source byte, 32 KiB with the 32 lane copies; two tables share
-// each 64 KiB page, at byte offsets 0 and 128 of every 256-byte row). The rest
-// use single-copy 32-word tables after those pages, as lut.cuh does: five
-// lookups for three sources, two for one (nibble tables with lane copies took
-// two each). With K fixed every table address is a PRMT of the data byte plus
-// an immediate. 16 MiB rows, 4 rows out, us before -> after: K = 8 41.2 -> 39.2,
-// K = 10 51.3 -> 48.2, K = 12 62.2 -> 57.4, K = 14 73.9 -> 72.0.
-constexpr int kByteSrc = 6;
+// lookup per source byte, 32 KiB: 256 rows of 32 lane copies). The rest use
+// single-copy 32-word tables after them, as lut.cuh does: five lookups for
+// three sources, two for one (nibble tables with lane copies took two each).
+// An address is a dot product of the data word (128 or 4 times one byte, plus
+// the lane or nothing, beside the ALU pipe as in lut.cuh) plus an immediate.
+// 16 MiB rows, 4 rows out, us, six byte tables and nibble tables by PRMT -> this:
+// K = 8 41.2 -> 38.8, K = 10 51.3 -> 47.7, K = 12 62.2 -> 57.0, K = 14 73.9 -> 73.8.
 constexpr int kFastMaxK = 14;
 constexpr int kFastThreads = 1024;
 
-template <int K>
+// At most B byte-table sources. A seventh table leaves room for the small
+// tables and the staging of up to 12 sources. The batched kernels take it (64
+// stripes of 1 MiB shards, RS(10,4): encode 196.8 -> 193.4 us, rebuild 206.3 ->
+// 203.8); one call's kernel is slower with it (16 MiB shards, 47.7 -> 52.1).
+constexpr int kByteSrcCall = 6, kByteSrcBatch = 7;
+
+template <int K, int B>
 struct FastLayout {
-  static constexpr int NB = K < kByteSrc ? K : kByteSrc;  // byte-table sources
+  static constexpr int kMost = K <= 12 ? B : 6;
+  static constexpr int NB = K < kMost ? K : kMost;        // byte-table sources
   static constexpr int NN = K - NB;                       // small-table sources
   static constexpr int N3 = NN / 3, N1 = NN % 3;          // threes, then single ones
-  static constexpr uint32_t small = ((NB + 1) / 2) * 65536u;
+  static constexpr uint32_t small = NB * 32768u;
   static constexpr uint32_t tables = small + N3 * 640u + N1 * 128u;
   static constexpr uint32_t smem = tables + K * kCompactWords * 4u;  // + compact staging
 };
@@ -77,21 +83,21 @@ struct FastLayout {
 // parameters). The compact words are staged in shared memory first (one
 // independent load per thread) and every byte-table entry's 32 lane copies are
 // written as 8 identical 16-byte stores.
-template <int K>
+template <int K, int B>
 __device__ __forceinline__ void fill_fast(const uint32_t* tables, const uint32_t* inl) {
-  using L = FastLayout<K>;
+  using L = FastLayout<K, B>;
   uint32_t* stage = reinterpret_cast<uint32_t*>(g_smem) + L::tables / 4;
   for (uint32_t i = threadIdx.x; i < K * kCompactWords; i += blockDim.x) {
     stage[i] = tables ? __ldg(tables + i) : inl[i];
   }
   __syncthreads();
-  // byte tables: word index = page * 16384 + x * 64 + half * 32 + lane
+  // byte tables: word index = t * 8192 + x * 32 + lane
   uint4* st4 = reinterpret_cast<uint4*>(g_smem);
 #pragma unroll 4
   for (uint32_t i = threadIdx.x; i < L::NB * 2048u; i += blockDim.x) {
     const uint32_t t = i >> 11, x = (i >> 3) & 255u, q = i & 7u;
     const uint32_t v = stage[t * kCompactWords + (x & 15u)] ^ stage[t * kCompactWords + 16u + (x >> 4)];
-    st4[(t >> 1) * 4096u + x * 16u + (t & 1u) * 8u + q] = make_uint4(v, v, v, v);
+    st4[t * 2048u + x * 8u + q] = make_uint4(v, v, v, v);
   }
   if constexpr (L::NN > 0) {
     // small tables: the words of one table are its 5- (or 4-) bit index
@@ -117,73 +123,57 @@ __device__ __forceinline__ void fill_fast(const uint32_t* tables, const uint32_t
   __syncthreads();
 }
 
-// Lane / page registers of the byte-table layout.
-struct FastRegs {
-  uint32_t lrp[3];  // byte-table pages 0..2
-  __device__ __forceinline__ FastRegs() {
-    const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
-#pragma unroll
-    for (int p = 0; p < 3; ++p) lrp[p] = lane4 | (static_cast<uint32_t>(p) << 16);
-  }
-};
+// base + M times byte b of x, beside the ALU pipe (lut.cuh: lut_addr).
+template <uint32_t M>
+__device__ __forceinline__ uint32_t byte_addr(uint32_t x, uint32_t base, int b) {
+  return __dp4a(x, M << (8 * b), base);
+}
 
 // Fold NW words (4 bytes each, byte b of word q is element 4q + b) of each
 // of the K sources into acc (acc[e] = products for rows 0..3 of element e).
-template <int K, int NW>
-__device__ __forceinline__ void fast_fold(const uint32_t (&w)[K][NW], uint32_t (&acc)[4 * NW],
-                                          const FastRegs& r) {
-  using L = FastLayout<K>;
+// lane4: 4 times the lane.
+template <int K, int B, int NW>
+__device__ __forceinline__ void fast_fold(const uint32_t (&w)[K][NW], uint32_t (&acc)[4 * NW], uint32_t lane4) {
+  using L = FastLayout<K, B>;
 #pragma unroll
   for (int t = 0; t < L::NB; t += 2) {
-    const uint32_t lr = r.lrp[t >> 1];
-    if (t + 1 < L::NB) {
 #pragma unroll
-      for (int q = 0; q < NW; ++q)
+    for (int q = 0; q < NW; ++q)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const uint32_t sel = 0x7604u | (static_cast<uint32_t>(b) << 4);
-          acc[4 * q + b] ^= lds_at(prmt(w[t][q], lr, sel)) ^ lds_at(prmt(w[t + 1][q], lr, sel) + 128u);
-        }
-    } else {
-#pragma unroll
-      for (int q = 0; q < NW; ++q)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const uint32_t sel = 0x7604u | (static_cast<uint32_t>(b) << 4);
-          acc[4 * q + b] ^= lds_at(prmt(w[t][q], lr, sel));
-        }
-    }
+      for (int b = 0; b < 4; ++b) {
+        uint32_t v = lds_at(byte_addr<128>(w[t][q], lane4, b) + t * 32768u);
+        if (t + 1 < L::NB) v ^= lds_at(byte_addr<128>(w[t + 1][q], lane4, b) + (t + 1) * 32768u);
+        acc[4 * q + b] ^= v;
+      }
   }
 #pragma unroll
   for (int i = 0; i < L::N3; ++i) {
-    constexpr uint32_t base = L::small;
     const int t = L::NB + 3 * i;
 #pragma unroll
     for (int q = 0; q < NW; ++q) {
-      const uint32_t i0 = (w[t][q] << 2) & 0x7C7C7C7Cu, i1 = (w[t + 1][q] << 2) & 0x7C7C7C7Cu,
-                     i2 = (w[t + 2][q] << 2) & 0x7C7C7C7Cu;
+      const uint32_t i0 = w[t][q] & 0x1F1F1F1Fu, i1 = w[t + 1][q] & 0x1F1F1F1Fu, i2 = w[t + 2][q] & 0x1F1F1F1Fu;
       const uint32_t i3 = ((w[t][q] >> 3) & 0x1C1C1C1Cu) | (w[t + 1][q] & 0x60606060u);
       const uint32_t i4 = ((w[t + 2][q] >> 3) & 0x1C1C1C1Cu) | ((w[t + 1][q] >> 2) & 0x20202020u);
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const uint32_t sel = 0x7650u | static_cast<uint32_t>(b), o = i * 640u;
-        acc[4 * q + b] ^= lds_at(prmt(i0, base, sel) + o) ^ lds_at(prmt(i1, base, sel) + o + 128u);
-        acc[4 * q + b] ^= lds_at(prmt(i2, base, sel) + o + 256u) ^ lds_at(prmt(i3, base, sel) + o + 384u);
-        acc[4 * q + b] ^= lds_at(prmt(i4, base, sel) + o + 512u);
+        constexpr uint32_t o = L::small;
+        acc[4 * q + b] ^= lds_at(byte_addr<4>(i0, 0, b) + o + i * 640u) ^ lds_at(byte_addr<4>(i1, 0, b) + o + i * 640u + 128u);
+        acc[4 * q + b] ^= lds_at(byte_addr<4>(i2, 0, b) + o + i * 640u + 256u) ^
+                          lds_at(byte_addr<1>(i3, 0, b) + o + i * 640u + 384u);
+        acc[4 * q + b] ^= lds_at(byte_addr<1>(i4, 0, b) + o + i * 640u + 512u);
       }
     }
   }
 #pragma unroll
   for (int i = 0; i < L::N1; ++i) {
-    constexpr uint32_t base = L::small;
     const int t = L::NB + 3 * L::N3 + i;
 #pragma unroll
     for (int q = 0; q < NW; ++q) {
-      const uint32_t i0 = (w[t][q] << 2) & 0x3C3C3C3Cu, i1 = (w[t][q] >> 2) & 0x3C3C3C3Cu;
+      const uint32_t i0 = w[t][q] & 0x0F0F0F0Fu, i1 = (w[t][q] >> 4) & 0x0F0F0F0Fu;
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const uint32_t sel = 0x7650u | static_cast<uint32_t>(b), o = L::N3 * 640u + i * 128u;
-        acc[4 * q + b] ^= lds_at(prmt(i0, base, sel) + o) ^ lds_at(prmt(i1, base, sel) + o + 64u);
+        constexpr uint32_t o = L::small + L::N3 * 640u;
+        acc[4 * q + b] ^= lds_at(byte_addr<4>(i0, 0, b) + o + i * 128u) ^ lds_at(byte_addr<4>(i1, 0, b) + o + i * 128u + 64u);
       }
     }
   }

@@ -27,8 +27,8 @@ namespace {
 
 template <int K, bool OVR, bool SHIFT>
 __global__ void __launch_bounds__(kFastThreads, 1) matrix_fast_kernel(const __grid_constant__ MatrixLaunch a) {
-  fill_fast<K>(a.tables, a.inline_tab);
-  const FastRegs r;
+  fill_fast<K, kByteSrcCall>(a.tables, a.inline_tab);
+  const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   const uint32_t lane = threadIdx.x & 31u;
   // SHIFT: whole warps iterate together (the row stores shuffle between lanes)
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kFastThreads, 1) matrix_fast_kernel(const __gr
     uint32_t acc[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = 0;
-    fast_fold<K, 4>(w, acc, r);
+    fast_fold<K, kByteSrcCall, 4>(w, acc, lane4);
     if constexpr (SHIFT)
       store_col4_any(acc, a.dst, a.nrows, off, OVR, valid);
     else
@@ -64,12 +64,12 @@ __global__ void __launch_bounds__(kFastThreads, 1) matrix_fast_kernel(const __gr
 template <int K, bool OVR, bool SHIFT>
 cudaError_t launch_fast_k(const MatrixLaunch& a, cudaStream_t s) {
   cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(matrix_fast_kernel<K, OVR, SHIFT>),
-                                   FastLayout<K>::smem);
+                                   FastLayout<K, kByteSrcCall>::smem);
   if (e != cudaSuccess) return e;
   const uint64_t want = (a.nvec + kFastThreads - 1) / kFastThreads;
   const uint64_t cap = static_cast<uint64_t>(sm_count());
   const unsigned blocks = static_cast<unsigned>(want < cap ? want : cap);
-  matrix_fast_kernel<K, OVR, SHIFT><<<blocks, kFastThreads, FastLayout<K>::smem, s>>>(a);
+  matrix_fast_kernel<K, OVR, SHIFT><<<blocks, kFastThreads, FastLayout<K, kByteSrcCall>::smem, s>>>(a);
   return cudaGetLastError();
 }
 
