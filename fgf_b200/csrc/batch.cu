@@ -389,6 +389,7 @@ struct BatchClass {
   std::vector<size_t> cuts;    // first item of each launch after the first
   std::vector<uint32_t> seg_jobs;   // byte-table class with own plans: sub-jobs with vectors, plan order
   std::vector<uint64_t> seg_prefix; // and the prefix of their vector counts (the segmented launch)
+  double cost = 0;             // lookups, roughly
   bool uniform = false;        // byte-table class whose sub-jobs share one plan
   bool shift = false;          // its rows are not all at the sources' offset within 16 bytes
 };
@@ -534,11 +535,21 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   std::vector<size_t> order(jobs.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t c) { return jobs[a].img < jobs[c].img; });
+  // Byte-table classes (a source count K) with fewer columns than this run the
+  // table kernels instead, together with the other 1-byte sub-jobs: a 1024-thread
+  // CTA with 227 KiB of tables waits for a whole SM to drain, which a mixed
+  // submission's dozens of small classes did one after the other (256 mixed
+  // stripes, with the order of items and launches below: 1505 -> 1463 us). One call crosses over between 4 MiB rows (K =
+  // 10: 17.3 us by table kernel, 19.1 by byte tables) and 16 MiB (54.7, 47.7).
+  constexpr uint64_t kByteClassCols = 8u << 16;
+  std::map<size_t, uint64_t> byte_cols;
+  for (size_t i = 0; i < jobs.size(); ++i)
+    if (jobs[i].byte_tab && al[i].sources) byte_cols[jobs[i].k] += jobs[i].len / 16;
   std::map<int, BatchClass> classes;
   for (size_t i : order) {
     const LoweredJob& L = jobs[i];
     const int E = field_bytes(L.field);
-    const bool fast = L.byte_tab && al[i].sources;
+    const bool fast = L.byte_tab && al[i].sources && byte_cols[L.k] >= kByteClassCols;
     const LutShape shape = lut_shape(E, L.nrows);
     const int key = fast ? 1000 + 2 * static_cast<int>(L.k) + al[i].unal
                          : ((E * 4 + shape.lev) * 8 + shape.w) * 3 + al[i].mode;
@@ -572,33 +583,35 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   for (auto& kv : classes) {
     BatchClass& c = kv.second;
     if (c.K == 0) {
-      // Tiles per item: the class's tile shape (tune.cpp: tile_cols; 8 columns
-      // per thread built in), fewer when the class is too small to give every
-      // resident CTA a few items (a small class runs beside the others on its
-      // own stream, see enqueue).
+      // Items of about equal work, 16 for every resident CTA, at most the class's
+      // tile shape (tune.cpp: tile_cols; 8 columns per thread built in); the
+      // stripes with the most sources, whose items are the longest, first.
       const int G = static_cast<int>((jobs[c.jobs[0]].nrows * c.E + 3) / 4);
       const uint64_t tile = c.E == 8 ? kTileColsDefault : tile_cols(c.E, G);
       if (c.E < 8) b->last_classes.emplace_back(c.E, G);
       const int mode = kv.first % 3;
-      uint64_t total = 0;
-      for (uint32_t i : c.jobs) total += lut_tiles(dj[i].lut.g, mode, kLutThreads);
-      const uint64_t slots = 4 * static_cast<uint64_t>(sm_count() * c.kern.ctas);
-      const uint64_t per = std::max<uint64_t>(1, std::min<uint64_t>(tile, (total + slots - 1) / slots));
-      // Stripes of one plan and of the byte tables' shape, but with sources at
-      // different offsets: one launch per kUniformJobs stripes, so that such a
-      // submission counts the same launches whatever its alignment.
+      std::stable_sort(c.jobs.begin(), c.jobs.end(), [&](uint32_t p, uint32_t q) { return jobs[p].k > jobs[q].k; });
+      uint64_t total = 0;  // tiles times sources
+      for (uint32_t i : c.jobs) total += lut_tiles(dj[i].lut.g, mode, kLutThreads) * jobs[i].k;
+      c.cost = static_cast<double>(total) * c.shape.nv * c.shape.w * (16 / c.E);
+      const uint64_t slots = 16 * static_cast<uint64_t>(sm_count() * c.kern.ctas);
+      // Stripes of one plan and of the byte tables' shape: one launch per
+      // kUniformJobs stripes, so that such a submission counts the same launches
+      // whatever its size and alignment.
       bool one_plan = jobs[c.jobs[0]].byte_tab != nullptr;
       for (uint32_t i : c.jobs) one_plan = one_plan && jobs[i].byte_tab == jobs[c.jobs[0]].byte_tab;
       for (size_t q = 0; q < c.jobs.size(); ++q) {
         const uint32_t i = c.jobs[q];
         if (one_plan && q && q % kUniformJobs == 0) c.cuts.push_back(c.items.size());
         LutBatchJob& J = dj[i].lut;
+        const uint64_t per = std::max<uint64_t>(1, std::min<uint64_t>(tile, total / (slots * jobs[i].k)));
         J.parts = static_cast<uint32_t>((lut_tiles(J.g, mode, kLutThreads) + per - 1) / per);
         const uint32_t n = J.parts + (lut_has_edges(J.g, mode) ? 1u : 0u);
         for (uint32_t p = 0; p < n; ++p) c.items.push_back(make_uint2(i, p));
       }
       continue;
     }
+    for (uint32_t i : c.jobs) c.cost += static_cast<double>(jobs[i].len) * jobs[i].k * 1.3;  // lookups per byte
     c.uniform = true;
     for (uint32_t i : c.jobs) c.uniform = c.uniform && jobs[i].byte_tab == jobs[c.jobs[0]].byte_tab;
     if (c.uniform) continue;
@@ -729,6 +742,8 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     uint32_t* counter = nullptr;
     size_t uparam = 0;
     int tc_group = -1;  // >= 0: a tensor-core launch over that group's stripes
+    double cost = 0;
+    std::string key;
     SegmentFn sfn = nullptr;  // segmented launch over the class's vectors
     const uint32_t* seg_jobs = nullptr;
     const uint64_t* seg_prefix = nullptr;
@@ -745,6 +760,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     const auto& x = cb[ci++];
     const bool fast = c.K > 0;
     Launch L;
+    L.cost = c.cost;
     const int akey = kv.first + (c.uniform ? 10000 : 0);
     if (c.uniform) {
       L.ufn = uniform_kernel_for(c.K, c.shift);
@@ -802,7 +818,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         uint64_t h = 1469598103934665603ull;
         const uint64_t* pw = reinterpret_cast<const uint64_t*>(&P);
         for (size_t i = 0; i < sizeof P / 8; ++i) h = (h ^ (h >> 29) ^ pw[i]) * 1099511628211ull;
-        key += "|u" + std::to_string(akey) + "," + std::to_string(h) + "," + std::to_string(U.grid);
+        U.key = "|u" + std::to_string(akey) + "," + std::to_string(h) + "," + std::to_string(U.grid);
         launches.push_back(U);
       }
       b->last_items += c.jobs.size();
@@ -820,7 +836,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         const uint64_t rows = (c.seg_prefix.back() + S.threads - 1) / S.threads;
         S.grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(rows, sms)));
         b->last_items += c.seg_jobs.size();
-        key += "|s" + std::to_string(akey) + "," + std::to_string(S.n) + "," + std::to_string(S.grid);
+        S.key = "|s" + std::to_string(akey) + "," + std::to_string(S.n) + "," + std::to_string(S.grid);
         launches.push_back(S);
       }
       if (!c.items.empty()) {
@@ -831,7 +847,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
                          : static_cast<unsigned>(std::min<uint64_t>((L.n + kClaim - 1) / kClaim, sms));
           L.items = reinterpret_cast<const uint2*>(s.dev + x.first) + i0;
           L.counter = reinterpret_cast<uint32_t*>(s.dev + x.second) + q;
-          key += "|" + std::to_string(akey) + "," + std::to_string(L.n) + "," + std::to_string(L.grid) + "," +
+          L.key = "|" + std::to_string(akey) + "," + std::to_string(L.n) + "," + std::to_string(L.grid) + "," +
                  std::to_string(L.smem);
           launches.push_back(L);
         }
@@ -845,12 +861,16 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     if (e != cudaSuccess) return e;
     Launch L;
     L.tc_group = static_cast<int>(g);
+    L.cost = 1e30;
     b->last_items += tcg[g].idx.size();
-    key += "|g" + std::to_string(J0.bits_key) + "," + std::to_string(J0.field) + "," + std::to_string(J0.k) + "," +
+    L.key = "|g" + std::to_string(J0.bits_key) + "," + std::to_string(J0.field) + "," + std::to_string(J0.k) + "," +
            std::to_string(J0.m) + "," + std::to_string(J0.ovr) + "," + std::to_string(tcg[g].idx.size()) + "," +
            std::to_string(tcg[g].nblk);
     launches.push_back(L);
   }
+  // the largest class first, so that the small ones fill the others' last waves
+  std::stable_sort(launches.begin(), launches.end(), [](const Launch& p, const Launch& q) { return p.cost > q.cost; });
+  for (const Launch& L : launches) key += L.key;
   const BatchDesc* djobs = reinterpret_cast<const BatchDesc*>(s.dev + off_jobs);
   const uint64_t* dptrs = reinterpret_cast<const uint64_t*>(s.dev + off_ptrs);
 
