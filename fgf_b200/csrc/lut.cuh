@@ -387,13 +387,14 @@ struct LutAhead {
   uint4 c[3];
 };
 
-// Does a shape's aligned path fetch the next column's first sources during the
-// last lookups of this one? Where the accumulators leave 16 warps an SM it hides the fetch (us,
-// without -> with: Gf16 RS(32,8) 16 MiB 355 -> 339, Gf32 RS(16,4) 8 MiB 91 -> 86,
-// Gf8D RS(32,12) 4 MiB 103 -> 99); smaller shapes have the warps to hide it and
-// pay for the registers (Gf8D RS(10,4) 4 MiB 17.6 -> 18.4).
+// Does a shape fetch the next column's first sources during the last lookups of
+// this one (not with unaligned sources)? It hides the fetch where 16 to 24 warps
+// an SM do not (us, without -> with: Gf16 RS(32,8) 16 MiB 355 -> 339, Gf32
+// RS(16,4) 8 MiB 91 -> 86, Gf8D RS(32,12) 4 MiB 103 -> 99); shapes of few
+// accumulators keep their warps instead, and two rows of 8-byte elements (18)
+// lose (RS(8,2) 4 MiB 29.7 against 30.1).
 template <class L, int W>
-constexpr bool kLutAhead = L::NP * W * L::NE >= 32;
+constexpr bool kLutAhead = L::NP * W * L::NE >= (L::NE == 2 ? 32 : 16);
 
 // Fold all sources of one column. load(t) fetches source t's 16 bytes, fix(t, x)
 // puts a fetch in place once it is needed. The fetches of the next three

@@ -6,12 +6,17 @@
 
 namespace fgfc {
 
-// CTAs per SM the register budget is set for: accumulators (3^LEV leaf
-// products x W words x 16 / E elements) plus three sources and their packed words.
+// CTAs per SM the register budget is set for: accumulators (3^LEV leaf products
+// x W words x 16 / E elements) plus two sets of three sources and their packed
+// words. Fewer, larger budgets win over more CTAs once the next column is
+// fetched ahead (16 accumulators, 4 -> 3 CTAs and ahead: Gf8D RS(10,4) 4 MiB
+// 17.6 -> 16.2 us; 4 and 6 accumulators, 4 -> 3: Gf32 RS(10,1) 4 MiB 16.4 -> 15.7,
+// GF(2^64) RS(8,1) 20.4 -> 19.7), but for the 2-byte rows without a split
+// (RS(10,2) 8 MiB 27.0 against 28.9); unaligned rows of 24 and 32 spill at 3.
 template <int E, int LEV, int W, int MODE>
 constexpr int lut_min_ctas() {
-  return pow3(LEV) * W * (16 / E) <= 16 ? (MODE == kAnyOff ? 3 : 4)
-         : pow3(LEV) * W * (16 / E) <= 32 && MODE != kAnyOff ? 3 : 2;
+  constexpr int n = pow3(LEV) * W * (16 / E);
+  return E == 2 && LEV == 0 && MODE != kAnyOff ? 4 : n <= 16 ? 3 : n <= 32 && MODE == kAligned ? 3 : 2;
 }
 
 template <int E, int LEV, int W, int MODE>
