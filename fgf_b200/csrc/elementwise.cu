@@ -5,12 +5,12 @@
 // plane by plane: one LOP3 (and, xor) per pair of input bits, the tower levels
 // by Karatsuba, reductions and tower constants as XORs of planes. Both inputs
 // are data here, so no table helps; shift-and-mask products of packed bytes
-// cost 9 to 85 operations per byte (1- to 8-byte elements), the planes cost 6
-// to 14, transposes included. It is bound by the ALU pipe (HBM's time is worth
-// about 8 operations per byte), 1-byte fields by both. us on B200, 64 MiB
+// cost 9 to 85 operations per byte (1- to 8-byte elements), the planes cost 5
+// to 16, transposes included. 1-byte fields run at HBM's rate, the others are
+// bound by the ALU pipe (HBM's time is worth about 8 operations per byte). us on B200, 64 MiB
 // vectors, shift-and-mask (Fan-Paar: log tables) -> planes:
-//   Gf8D 44.6 -> 39.0   Gf16 77.2 -> 47.8   Gf32 185 -> 68   Gf64 322 -> 104
-//   FP8  149 -> 43      FP16 129 -> 49      FP32 168 -> 76   FP64 246 -> 109
+//   Gf8D 44.6 -> 33.6   Gf16 77.2 -> 40.6   Gf32 185 -> 56   Gf64 322 -> 86
+//   FP8  149 -> 35      FP16 129 -> 43      FP32 168 -> 65   FP64 246 -> 99
 //
 // The order of elements within a transposed block does not matter as long as
 // all three vectors use the same, so a thread's words are whichever 16-byte
@@ -27,6 +27,23 @@ namespace fgfc {
 
 namespace {
 
+// ---------------------------------------------------------------- three-input logic
+
+// Written out: left to itself the compiler rebalances the XOR chains and spends
+// a quarter more instructions on them (ALU instructions per 32 products: 245 ->
+// 172 for 1 byte, 661 -> 504 for Gf16, 1911 -> 1554 for Gf32; 64 MiB of Gf16
+// 47.8 -> 40.6 us).
+template <uint32_t LUT>
+__device__ __forceinline__ uint32_t lop3(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(d) : "r"(a), "r"(b), "r"(c), "n"(LUT));
+  return d;
+}
+__device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t b, uint32_t c) { return lop3<0x6Au>(a, b, c); }
+__device__ __forceinline__ uint32_t xor3(uint32_t a, uint32_t b, uint32_t c) { return lop3<0x96u>(a, b, c); }
+// m ? a : b, bit by bit
+__device__ __forceinline__ uint32_t pick(uint32_t m, uint32_t a, uint32_t b) { return lop3<0xCAu>(m, a, b); }
+
 // ---------------------------------------------------------------- bit planes
 
 // Right shifts of the transposes on the multiply pipe: 64 MiB products of 1-
@@ -37,8 +54,8 @@ constexpr bool kMulShift = E <= 2;
 // 8x8 bit transpose in each byte lane of 8 words (its own inverse).
 template <bool MUL>
 __device__ __forceinline__ void swap_bits(uint32_t& a, uint32_t& b, int s, uint32_t m, const Shift<MUL>& sh) {
-  const uint32_t x = (a & m) | ((b << s) & ~m);
-  b = (sh.shr(a, s) & m) | (b & ~m);
+  const uint32_t x = pick(m, a, b << s);
+  b = pick(m, sh.shr(a, s), b);
   a = x;
 }
 template <bool MUL>
@@ -124,14 +141,15 @@ enum Family { kPoly1B, kPoly1D, kFanPaar };  // flat bytes mod 0x11B (and its to
 template <int N>
 __device__ __forceinline__ void mul_beta(const uint32_t* v, uint32_t* o) {
   if constexpr (N == 8) {
-    o[0] = v[3] ^ v[7];
-    o[1] = v[3] ^ v[4] ^ v[7];
-    o[2] = v[4] ^ v[5];
-    o[3] = v[3] ^ v[5] ^ v[6] ^ v[7];
-    o[4] = v[3] ^ v[4] ^ v[6];
-    o[5] = v[0] ^ v[4] ^ v[5] ^ v[7];
-    o[6] = v[1] ^ v[5] ^ v[6];
-    o[7] = v[2] ^ v[6] ^ v[7];
+    const uint32_t a = v[3] ^ v[7], b = v[4] ^ v[5];
+    o[0] = a;
+    o[1] = a ^ v[4];
+    o[2] = b;
+    o[3] = xor3(a, v[5], v[6]);
+    o[4] = xor3(v[3], v[4], v[6]);
+    o[5] = xor3(b, v[0], v[7]);
+    o[6] = xor3(v[1], v[5], v[6]);
+    o[7] = xor3(v[2], v[6], v[7]);
   } else {
     constexpr int M = N / 2;
     uint32_t s[M], t[M];
@@ -166,22 +184,35 @@ __device__ __forceinline__ void mul_planes(const uint32_t* a, const uint32_t* b,
   if constexpr (F != kFanPaar && N == 8) {
     uint32_t p[15];
 #pragma unroll
-    for (int i = 0; i < 15; ++i) p[i] = 0;
+    for (int k = 0; k < 15; ++k) {
+      const int lo = k < 8 ? 0 : k - 7, hi = k < 8 ? k : 7;
+      p[k] = a[lo] & b[k - lo];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) p[i + j] ^= a[i] & b[j];
-    constexpr uint32_t R = F == kPoly1D ? 0x1Du : 0x1Bu;
-#pragma unroll
-    for (int i = 14; i >= 8; --i)
-#pragma unroll
-      for (int j = 0; j < 5; ++j)
-        if ((R >> j) & 1u) p[i - 8 + j] ^= p[i];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) c[i] = p[i];
+      for (int i = lo + 1; i <= hi; ++i) p[k] = and_xor(a[i], b[k - i], p[k]);
+    }
+    // x^8 .. x^14 reduced, for each power of the result the ones that reach it
+    if constexpr (F == kPoly1D) {  // x^8 = x^4 + x^3 + x^2 + 1
+      c[0] = xor3(xor3(p[0], p[8], p[12]), p[13], p[14]);
+      c[1] = xor3(p[1], p[9], p[13]) ^ p[14];
+      c[2] = xor3(xor3(p[2], p[8], p[10]), p[12], p[13]);
+      c[3] = xor3(xor3(p[3], p[8], p[9]), p[11], p[12]);
+      c[4] = xor3(xor3(p[4], p[8], p[9]), p[10], p[14]);
+      c[5] = xor3(p[5], p[9], p[10]) ^ p[11];
+      c[6] = xor3(p[6], p[10], p[11]) ^ p[12];
+      c[7] = xor3(p[7], p[11], p[12]) ^ p[13];
+    } else {  // x^8 = x^4 + x^3 + x + 1
+      c[0] = xor3(p[0], p[8], p[12]) ^ p[13];
+      c[1] = xor3(xor3(p[1], p[8], p[9]), p[12], p[14]);
+      c[2] = xor3(p[2], p[9], p[10]) ^ p[13];
+      c[3] = xor3(xor3(xor3(p[3], p[8], p[10]), p[11], p[12]), p[13], p[14]);
+      c[4] = xor3(xor3(p[4], p[8], p[9]), p[11], p[14]);
+      c[5] = xor3(p[5], p[9], p[10]) ^ p[12];
+      c[6] = xor3(p[6], p[10], p[11]) ^ p[13];
+      c[7] = xor3(p[7], p[11], p[12]) ^ p[14];
+    }
   } else if constexpr (F == kFanPaar && N == 2) {
-    c[0] = (a[0] & b[0]) ^ (a[1] & b[1]);
-    c[1] = (a[0] & b[1]) ^ (a[1] & (b[0] ^ b[1]));
+    c[0] = and_xor(a[1], b[1], a[0] & b[0]);
+    c[1] = and_xor(a[1], b[0] ^ b[1], a[0] & b[1]);
   } else {
     constexpr int M = N / 2;
     uint32_t z0[M], z2[M], t[M], sa[M], sb[M];
@@ -200,7 +231,7 @@ __device__ __forceinline__ void mul_planes(const uint32_t* a, const uint32_t* b,
 #pragma unroll
     for (int i = 0; i < M; ++i) {
       c[i] = z0[i] ^ (F == kFanPaar ? z2[i] : t[i]);
-      c[M + i] ^= F == kFanPaar ? z0[i] ^ z2[i] ^ t[i] : z0[i];
+      c[M + i] = F == kFanPaar ? xor3(c[M + i] ^ z0[i], z2[i], t[i]) : c[M + i] ^ z0[i];
     }
   }
 }

@@ -456,17 +456,17 @@ static cudaError_t launch_elementwise_fp(int field, uint8_t* dst, const uint8_t*
 }
 
 // Vectors shorter than this run one element per thread: a planes warp takes
-// 1 KiB times the element width through 1400 (4 bytes) to 3500 (8 bytes)
+// 1 KiB times the element width through 1600 (4 bytes) to 4000 (8 bytes)
 // instructions, which a short vector does not amortise. us on B200, element
-// kernel / planes: Gf32 64 KiB 3.2 / 4.6, 1 MiB 4.9 / 4.6; FP32 64 KiB 3.5 / 4.8,
-// 1 MiB 10.5 / 4.8; Gf64 1 MiB 7.4 / 10.5, 64 MiB 322 / 107; FP64 1 MiB 9.8 /
-// 11.0, 64 MiB 246 / 108. 1- and 2-byte fields are level at 64 KiB.
+// kernel / planes: Gf32 256 KiB 2.3 / 3.1, 512 KiB 3.3 / 3.3; FP32 128 KiB 3.5 /
+// 3.7, 256 KiB 4.8 / 3.7; Gf64 1 MiB 7.4 / 8.9, 1.5 MiB 10.2 / 9.1; FP64 768 KiB
+// 8.2 / 10.0, 1 MiB 9.9 / 10.0. 1- and 2-byte fields are level at 64 KiB.
 static uint64_t planes_min_bytes(int field) {
   switch (field) {
-    case kGf32: return 1u << 20;
+    case kGf32: return 1u << 19;
     case kFp32: return 1u << 18;
-    case kGf64:
-    case kFp64: return 2u << 20;
+    case kGf64: return 5u << 18;
+    case kFp64: return 1u << 20;
     default: return 0;
   }
 }

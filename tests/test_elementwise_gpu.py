@@ -17,11 +17,11 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("field", list(FIELDS.values()), ids=lambda f: f.__name__)
 def test_blocks_and_edges(cuda, field, offset):
     b = field.BYTES
-    first = {4: 1 << 18, 8: 2 << 20}.get(b, 0)  # shortest vector of the planes kernel (FP32's for 4 bytes)
+    first = {4: 1 << 18, 8: 1 << 20}.get(b, 0)  # shortest vector of the planes kernel (the Fan-Paar fields')
     block = 1024 * b
     lengths = {first + n for n in (b, 16, block - 16, block, block + 16 + b, 5 * block + 3 * b, 700 * block + 48)}
     if b >= 4:
-        lengths |= {first - b, (1 << 20) - b, 1 << 20}
+        lengths |= {first - b, (1 << 19) - b, 1 << 19, (5 << 18) - b, 5 << 18}
     rng = np.random.default_rng(field.ID * 10 + offset)
     for n in sorted(lengths):
         if n > 6 << 20:
