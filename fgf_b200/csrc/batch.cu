@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
       if (threadIdx.x < K) s_src[threadIdx.x] = reinterpret_cast<const uint8_t*>(ptrs[J.src_idx + threadIdx.x]);
       if (threadIdx.x < J.nrows) s_dst[threadIdx.x] = reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + threadIdx.x]);
       if (!resident) {
-        fill_fast<K, kByteSrcBatch>(J.tables, nullptr);
+        fill_fast<K>(J.tables, nullptr);
         if (threadIdx.x == 0) {
           s_tab = J.tables;
         }
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
           uint32_t acc[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e) acc[e] = 0;
-          fast_fold<K, kByteSrcBatch, 4>(w, acc, lane4);
+          fast_fold<K, 4>(w, acc, lane4);
           if constexpr (SHIFT)
             store_col4_any(acc, s_dst, J.nrows, off, ovr, valid);
           else
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
             w[t][0] = x;
           }
           uint32_t acc[4] = {0, 0, 0, 0};
-          fast_fold<K, kByteSrcBatch, 1>(w, acc, lane4);
+          fast_fold<K, 1>(w, acc, lane4);
           for (uint32_t rr = 0; rr < J.nrows; ++rr) {
             const uint32_t o = row_word4(acc, static_cast<int>(rr));
             uint8_t* d = s_dst[rr] + off;
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
 // at every item boundary instead; that kernel keeps the scalar heads and
 // tails of the class.
 template <int K, bool SHIFT>
-__global__ void __launch_bounds__(kFastThreads, 1)
+__global__ void __launch_bounds__(fast_threads(K), 1)
     batch_fast_segment_kernel(const BatchDesc* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
                               const uint32_t* __restrict__ jidx, const uint64_t* __restrict__ vprefix,
                               uint32_t njobs) {
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
     if (threadIdx.x < K) s_src[threadIdx.x] = reinterpret_cast<const uint8_t*>(ptrs[J.src_idx + threadIdx.x]);
     if (threadIdx.x < J.nrows) s_dst[threadIdx.x] = reinterpret_cast<uint8_t*>(ptrs[J.dst_idx + threadIdx.x]);
     if (!resident) {
-      fill_fast<K, kByteSrcBatch>(J.tables, nullptr);
+      fill_fast<K>(J.tables, nullptr);
       if (threadIdx.x == 0) {
         s_tab = J.tables;
       }
@@ -195,28 +195,37 @@ __global__ void __launch_bounds__(kFastThreads, 1)
     const bool ovr = J.ovr != 0;
     // SHIFT: whole warps iterate together (the row stores shuffle between
     // lanes) and lanes past the end reload the last column
+    uint32_t wn[K][4];
+    if constexpr (fast_pipe(K)) {
+      const uint64_t u = v0 + threadIdx.x < vend ? v0 + threadIdx.x : vend - 1;
+      fast_load<K>(s_src, J.head + (u - base) * 16u, wn);
+    }
     for (uint64_t ub = v0 + threadIdx.x - (SHIFT ? lane : 0u); ub < vend; ub += blockDim.x) {
       const uint64_t u0 = SHIFT ? ub + lane : ub;
       const bool valid = !SHIFT || u0 < vend;
       const uint64_t u = valid ? u0 : vend - 1;
       const uint64_t off = J.head + (u - base) * 16u;
-      if (u + blockDim.x < vend) {  // this thread's next column: into L2 now
+      if (!fast_pipe(K) && u + blockDim.x < vend) {  // this thread's next column: into L2 now
 #pragma unroll
         for (int t = 0; t < K; ++t) prefetch_l2(s_src[t] + off + blockDim.x * 16u);
       }
       uint32_t w[K][4];
+      if constexpr (fast_pipe(K)) {
 #pragma unroll
-      for (int t = 0; t < K; ++t) {
-        const uint4 x = ldg16(s_src[t] + off);
-        w[t][0] = x.x;
-        w[t][1] = x.y;
-        w[t][2] = x.z;
-        w[t][3] = x.w;
+        for (int t = 0; t < K; ++t)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) w[t][q] = wn[t][q];
+        if (ub + blockDim.x < vend) {
+          const uint64_t un = u0 + blockDim.x < vend ? u0 + blockDim.x : vend - 1;
+          fast_load<K>(s_src, J.head + (un - base) * 16u, wn);
+        }
+      } else {
+        fast_load<K>(s_src, off, w);
       }
       uint32_t acc[16];
 #pragma unroll
       for (int e = 0; e < 16; ++e) acc[e] = 0;
-      fast_fold<K, kByteSrcBatch, 4>(w, acc, lane4);
+      fast_fold<K, 4>(w, acc, lane4);
       if constexpr (SHIFT)
         store_col4_any(acc, s_dst, J.nrows, off, ovr, valid);
       else
@@ -252,9 +261,9 @@ struct UniformParams {
 static_assert(sizeof(UniformParams) <= 32000, "launch parameter block too large");
 
 template <int K, bool SHIFT>
-__global__ void __launch_bounds__(kFastThreads, 1)
+__global__ void __launch_bounds__(fast_threads(K), 1)
     batch_fast_uniform_kernel(const __grid_constant__ UniformParams P) {
-  fill_fast<K, kByteSrcBatch>(P.tables, nullptr);
+  fill_fast<K>(P.tables, nullptr);
   const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -264,6 +273,14 @@ __global__ void __launch_bounds__(kFastThreads, 1)
   // SHIFT: whole warps iterate together (the row stores shuffle between
   // lanes; a warp may straddle two stripes) and lanes past the end reload the
   // last column
+  uint32_t wn[K][4];
+  if constexpr (fast_pipe(K)) {
+    if (tid - (SHIFT ? lane : 0u) < vtotal) {
+      const uint64_t u = tid < vtotal ? tid : vtotal - 1;
+      while (u >= P.vprefix[jn + 1]) ++jn;
+      fast_load<K>(P.jobs[jn].src, P.jobs[jn].head + (u - P.vprefix[jn]) * 16u, wn);
+    }
+  }
   for (uint64_t ub = tid - (SHIFT ? lane : 0u); ub < vtotal; ub += stride) {
     const uint64_t u0 = SHIFT ? ub + lane : ub;
     const bool valid = !SHIFT || u0 < vtotal;
@@ -271,27 +288,32 @@ __global__ void __launch_bounds__(kFastThreads, 1)
     while (u >= P.vprefix[j + 1]) ++j;
     const UJob& J = P.jobs[j];
     const uint64_t off = J.head + (u - P.vprefix[j]) * 16u;
-    const uint64_t un = u + stride;  // this thread's next column: into L2 now
-    if (un < vtotal) {
-      while (un >= P.vprefix[jn + 1]) ++jn;
-      const UJob& JN = P.jobs[jn];
-      const uint64_t offn = JN.head + (un - P.vprefix[jn]) * 16u;
-#pragma unroll
-      for (int t = 0; t < K; ++t) prefetch_l2(JN.src[t] + offn);
-    }
     uint32_t w[K][4];
+    if constexpr (fast_pipe(K)) {
 #pragma unroll
-    for (int t = 0; t < K; ++t) {
-      const uint4 x = ldg16(J.src[t] + off);
-      w[t][0] = x.x;
-      w[t][1] = x.y;
-      w[t][2] = x.z;
-      w[t][3] = x.w;
+      for (int t = 0; t < K; ++t)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w[t][q] = wn[t][q];
+      if (ub + stride < vtotal) {
+        const uint64_t un = u0 + stride < vtotal ? u0 + stride : vtotal - 1;
+        while (un >= P.vprefix[jn + 1]) ++jn;
+        fast_load<K>(P.jobs[jn].src, P.jobs[jn].head + (un - P.vprefix[jn]) * 16u, wn);
+      }
+    } else {
+      const uint64_t un = u + stride;  // this thread's next column: into L2 now
+      if (un < vtotal) {
+        while (un >= P.vprefix[jn + 1]) ++jn;
+        const UJob& JN = P.jobs[jn];
+        const uint64_t offn = JN.head + (un - P.vprefix[jn]) * 16u;
+#pragma unroll
+        for (int t = 0; t < K; ++t) prefetch_l2(JN.src[t] + offn);
+      }
+      fast_load<K>(J.src, off, w);
     }
     uint32_t acc[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = 0;
-    fast_fold<K, kByteSrcBatch, 4>(w, acc, lane4);
+    fast_fold<K, 4>(w, acc, lane4);
     if constexpr (SHIFT)
       store_col4_any(acc, J.dst, J.nrows, off, J.ovr != 0, valid);
     else
@@ -316,7 +338,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
       w[t][0] = x;
     }
     uint32_t acc[4] = {0, 0, 0, 0};
-    fast_fold<K, kByteSrcBatch, 1>(w, acc, lane4);
+    fast_fold<K, 1>(w, acc, lane4);
     for (uint32_t rr = 0; rr < J.nrows; ++rr) {
       const uint32_t o = row_word4(acc, static_cast<int>(rr));
       uint8_t* d = J.dst[rr] + off;
@@ -367,7 +389,7 @@ UniformFn uniform_kernel_for(int K, bool shift) {
 uint32_t fast_smem(int K) {
   switch (K) {
 #define FGFC_CASE(k) \
-  case k: return FastLayout<k, kByteSrcBatch>::smem;
+  case k: return FastLayout<k>::smem;
     FGFC_K_CASES(FGFC_CASE)
 #undef FGFC_CASE
     default: return 0;
@@ -815,7 +837,8 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
           P.gprefix[q + 1] = P.gprefix[q] + (J.head + 3) / 4 + (tail + 3) / 4;
         }
         Launch U = L;
-        const uint64_t want = (std::max(P.vprefix[nq], P.gprefix[nq]) + L.threads - 1) / L.threads;
+        U.threads = static_cast<unsigned>(fast_threads(c.K));
+        const uint64_t want = (std::max(P.vprefix[nq], P.gprefix[nq]) + U.threads - 1) / U.threads;
         U.grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(want, sms)));
         U.uparam = uparams.size() - 1;
         // the parameter block is baked into a captured graph: hash it into the key
@@ -839,6 +862,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         S.n = static_cast<uint32_t>(c.seg_jobs.size());
         S.seg_jobs = reinterpret_cast<const uint32_t*>(s.dev + y.first);
         S.seg_prefix = reinterpret_cast<const uint64_t*>(s.dev + y.second);
+        S.threads = static_cast<unsigned>(fast_threads(c.K));
         const uint64_t rows = (c.seg_prefix.back() + S.threads - 1) / S.threads;
         S.grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(rows, sms)));
         b->last_items += c.seg_jobs.size();

@@ -50,26 +50,31 @@ __device__ __forceinline__ void prefetch_l2(const uint8_t* p) { asm volatile("pr
 // ---------------------------------------------------------------- byte-table layout
 //
 // Gf8 fields with at most 4 rows (one table group) and a compile-time number
-// of sources K. Sources t < kByteSrc get a full 256-entry product table (one
+// of sources K. The first ones get a full 256-entry product table (one
 // lookup per source byte, 32 KiB: 256 rows of 32 lane copies). The rest use
 // single-copy 32-word tables after them, as lut.cuh does: five lookups for
 // three sources, two for one (nibble tables with lane copies took two each).
 // An address is a dot product of the data word (128 or 4 times one byte, plus
 // the lane or nothing, beside the ALU pipe as in lut.cuh) plus an immediate.
-// 16 MiB rows, 4 rows out, us, six byte tables and nibble tables by PRMT -> this:
-// K = 8 41.2 -> 38.8, K = 10 51.3 -> 47.7, K = 12 62.2 -> 57.0, K = 14 73.9 -> 73.8.
 constexpr int kFastMaxK = 14;
 constexpr int kFastThreads = 1024;
+// 2 to 10 sources: a thread holds two columns, the next one on its way while
+// this one's lookups run (half the threads from 5 sources on, for the
+// registers). More sources, and one alone, take 1024 threads and a prefetch of
+// each thread's next column into L2. 16 MiB rows, 4 rows out, prefetch -> two
+// columns, us: K = 6 33.2 -> 30.8, K = 8 38.8 -> 33.9, K = 10 47.7 -> 43.5; 4
+// sources of 64 MiB into one row 55.9 -> 53.8, one into one 24.8 -> 29.1.
+__host__ __device__ constexpr bool fast_pipe(int K) { return K >= 2 && K <= 10; }
+__host__ __device__ constexpr int fast_threads(int K) { return K > 4 && fast_pipe(K) ? 512 : kFastThreads; }
 
-// At most B byte-table sources. A seventh table leaves room for the small
-// tables and the staging of up to 12 sources. The batched kernels take it (64
-// stripes of 1 MiB shards, RS(10,4): encode 196.8 -> 193.4 us, rebuild 206.3 ->
-// 203.8); one call's kernel is slower with it (16 MiB shards, 47.7 -> 52.1).
-constexpr int kByteSrcCall = 6, kByteSrcBatch = 7;
-
-template <int K, int B>
+// Byte-table sources. Loads in flight live in what the tables leave of the 256
+// KiB of L1: a seventh table (28 KiB left instead of 60) saves a lookup but cost
+// one call over 16 MiB shards of RS(10,4) 52.1 us against 47.7, and fetching
+// ahead with it cost batches 13 %. From 13 sources on four tables are better
+// (K = 14: 73.8 -> 67.9 us), up to 12 six (K = 12: 57.2 against 59.4).
+template <int K>
 struct FastLayout {
-  static constexpr int kMost = K <= 12 ? B : 6;
+  static constexpr int kMost = K <= 12 ? 6 : 4;
   static constexpr int NB = K < kMost ? K : kMost;        // byte-table sources
   static constexpr int NN = K - NB;                       // small-table sources
   static constexpr int N3 = NN / 3, N1 = NN % 3;          // threes, then single ones
@@ -83,9 +88,9 @@ struct FastLayout {
 // parameters). The compact words are staged in shared memory first (one
 // independent load per thread) and every byte-table entry's 32 lane copies are
 // written as 8 identical 16-byte stores.
-template <int K, int B>
+template <int K>
 __device__ __forceinline__ void fill_fast(const uint32_t* tables, const uint32_t* inl) {
-  using L = FastLayout<K, B>;
+  using L = FastLayout<K>;
   uint32_t* stage = reinterpret_cast<uint32_t*>(g_smem) + L::tables / 4;
   for (uint32_t i = threadIdx.x; i < K * kCompactWords; i += blockDim.x) {
     stage[i] = tables ? __ldg(tables + i) : inl[i];
@@ -132,9 +137,9 @@ __device__ __forceinline__ uint32_t byte_addr(uint32_t x, uint32_t base, int b) 
 // Fold NW words (4 bytes each, byte b of word q is element 4q + b) of each
 // of the K sources into acc (acc[e] = products for rows 0..3 of element e).
 // lane4: 4 times the lane.
-template <int K, int B, int NW>
+template <int K, int NW>
 __device__ __forceinline__ void fast_fold(const uint32_t (&w)[K][NW], uint32_t (&acc)[4 * NW], uint32_t lane4) {
-  using L = FastLayout<K, B>;
+  using L = FastLayout<K>;
 #pragma unroll
   for (int t = 0; t < L::NB; t += 2) {
 #pragma unroll
@@ -176,6 +181,19 @@ __device__ __forceinline__ void fast_fold(const uint32_t (&w)[K][NW], uint32_t (
         acc[4 * q + b] ^= lds_at(byte_addr<4>(i0, 0, b) + o + i * 128u) ^ lds_at(byte_addr<4>(i1, 0, b) + o + i * 128u + 64u);
       }
     }
+  }
+}
+
+// 16 bytes of each of the K sources at byte off.
+template <int K>
+__device__ __forceinline__ void fast_load(const uint8_t* const* src, uint64_t off, uint32_t (&w)[K][4]) {
+#pragma unroll
+  for (int t = 0; t < K; ++t) {
+    const uint4 x = ldg16(src[t] + off);
+    w[t][0] = x.x;
+    w[t][1] = x.y;
+    w[t][2] = x.z;
+    w[t][3] = x.w;
   }
 }
 

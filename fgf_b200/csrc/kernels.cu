@@ -26,34 +26,41 @@ namespace {
 // (tune.cpp): short rows use the 32-word tables (lut.cuh), which fill faster.
 
 template <int K, bool OVR, bool SHIFT>
-__global__ void __launch_bounds__(kFastThreads, 1) matrix_fast_kernel(const __grid_constant__ MatrixLaunch a) {
-  fill_fast<K, kByteSrcCall>(a.tables, a.inline_tab);
+__global__ void __launch_bounds__(fast_threads(K), 1) matrix_fast_kernel(const __grid_constant__ MatrixLaunch a) {
+  fill_fast<K>(a.tables, a.inline_tab);
   const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   const uint32_t lane = threadIdx.x & 31u;
   // SHIFT: whole warps iterate together (the row stores shuffle between lanes)
-  for (uint64_t vb = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x - (SHIFT ? lane : 0u);
-       vb < a.nvec; vb += stride) {
+  uint64_t vb = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x - (SHIFT ? lane : 0u);
+  uint32_t wn[K][4];
+  if constexpr (fast_pipe(K)) {
+    const uint64_t v = SHIFT ? vb + lane : vb;
+    if (vb < a.nvec) fast_load<K>(a.src, a.head + (v < a.nvec ? v : a.nvec - 1) * 16u, wn);
+  }
+  for (; vb < a.nvec; vb += stride) {
     const uint64_t v = SHIFT ? vb + lane : vb;
     const bool valid = !SHIFT || v < a.nvec;
     const uint64_t off = a.head + (valid ? v : a.nvec - 1) * 16u;
-    if (v + stride < a.nvec) {  // this thread's next column: into L2 now
-#pragma unroll
-      for (int t = 0; t < K; ++t) prefetch_l2(a.src[t] + off + stride * 16u);
-    }
     uint32_t w[K][4];
+    if constexpr (fast_pipe(K)) {
 #pragma unroll
-    for (int t = 0; t < K; ++t) {
-      const uint4 x = ldg16(a.src[t] + off);
-      w[t][0] = x.x;
-      w[t][1] = x.y;
-      w[t][2] = x.z;
-      w[t][3] = x.w;
+      for (int t = 0; t < K; ++t)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w[t][q] = wn[t][q];
+      if (vb + stride < a.nvec)
+        fast_load<K>(a.src, a.head + (v + stride < a.nvec ? v + stride : a.nvec - 1) * 16u, wn);
+    } else {
+      if (v + stride < a.nvec) {  // this thread's next column: into L2 now
+#pragma unroll
+        for (int t = 0; t < K; ++t) prefetch_l2(a.src[t] + off + stride * 16u);
+      }
+      fast_load<K>(a.src, off, w);
     }
     uint32_t acc[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = 0;
-    fast_fold<K, kByteSrcCall, 4>(w, acc, lane4);
+    fast_fold<K, 4>(w, acc, lane4);
     if constexpr (SHIFT)
       store_col4_any(acc, a.dst, a.nrows, off, OVR, valid);
     else
@@ -64,12 +71,12 @@ __global__ void __launch_bounds__(kFastThreads, 1) matrix_fast_kernel(const __gr
 template <int K, bool OVR, bool SHIFT>
 cudaError_t launch_fast_k(const MatrixLaunch& a, cudaStream_t s) {
   cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(matrix_fast_kernel<K, OVR, SHIFT>),
-                                   FastLayout<K, kByteSrcCall>::smem);
+                                   FastLayout<K>::smem);
   if (e != cudaSuccess) return e;
-  const uint64_t want = (a.nvec + kFastThreads - 1) / kFastThreads;
+  const uint64_t want = (a.nvec + fast_threads(K) - 1) / fast_threads(K);
   const uint64_t cap = static_cast<uint64_t>(sm_count());
   const unsigned blocks = static_cast<unsigned>(want < cap ? want : cap);
-  matrix_fast_kernel<K, OVR, SHIFT><<<blocks, kFastThreads, FastLayout<K, kByteSrcCall>::smem, s>>>(a);
+  matrix_fast_kernel<K, OVR, SHIFT><<<blocks, fast_threads(K), FastLayout<K>::smem, s>>>(a);
   return cudaGetLastError();
 }
 
