@@ -441,8 +441,7 @@ struct BatchState {
   BatchSlot slot[kBatchSlots];
   int next = 0;
   bool graphs = true;
-  cudaStream_t capture = nullptr;
-  cudaStream_t upload = nullptr;
+  cudaStream_t capture = nullptr;  // records graphs, and carries the descriptor copies
   cudaStream_t side[kSideStreams] = {};
   cudaEvent_t fork = nullptr, join[kSideStreams] = {};
   size_t last_launches = 0, last_items = 0;
@@ -490,7 +489,6 @@ void batch_state_destroy(void* p) {
     if (s.done) cudaEventDestroy(s.done);
     if (s.up) cudaEventDestroy(s.up);
   }
-  if (b->upload) cudaStreamDestroy(b->upload);
   if (b->capture) cudaStreamDestroy(b->capture);
   for (int i = 0; i < kSideStreams; ++i) {
     if (b->side[i]) cudaStreamDestroy(b->side[i]);
@@ -916,7 +914,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
     if (e != cudaSuccess) return e;
   }
-  // The blob goes up on a stream of its own, under whatever the caller's stream
+  // The blob goes up on the stream that records graphs, under whatever the caller's stream
   // still runs (the slot is free: its last submission finished), and the
   // caller's stream waits for it: in line the copy and the gaps around it cost
   // 10 us between two submissions (64 stripes of 1 MiB shards, RS(10,4): encode
@@ -930,13 +928,13 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   bool blob = false;
   for (const Launch& L : launches) blob = blob || !L.ufn;
   if (inline_copy) key += "|copy";
+  if (!b->capture) {
+    e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return e;
+  }
   if (blob && !inline_copy) {
-    if (!b->upload) {
-      e = cudaStreamCreateWithFlags(&b->upload, cudaStreamNonBlocking);
-      if (e != cudaSuccess) return e;
-    }
-    e = cudaMemcpyAsync(s.dev, s.host, bytes, cudaMemcpyHostToDevice, b->upload);
-    if (e == cudaSuccess) e = cudaEventRecord(s.up, b->upload);
+    e = cudaMemcpyAsync(s.dev, s.host, bytes, cudaMemcpyHostToDevice, b->capture);
+    if (e == cudaSuccess) e = cudaEventRecord(s.up, b->capture);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, s.up, 0);
     if (e != cudaSuccess) return e;
   }
@@ -988,10 +986,6 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       if (s.graph) {
         cudaGraphExecDestroy(s.graph);
         s.graph = nullptr;
-      }
-      if (!b->capture) {
-        e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking);
-        if (e != cudaSuccess) return e;
       }
       cudaGraph_t g = nullptr;
       e = cudaStreamBeginCapture(b->capture, cudaStreamCaptureModeThreadLocal);
