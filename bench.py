@@ -1376,7 +1376,7 @@ def run_case(args):
         ok = all(oracle_matrix_windows(field.ID, chk[i][0], None, [chk[i][1][j * n:(j + 1) * n] for j in range(m)],
                                        chk[i][2], True, rng) for i in (0, ns // 2, ns - 1))
         alg, src_b = ns * (k + m) * n, ns * k * n
-        kernel = "batch (Gf16 half-products)" if os.environ.get("FGFC_GF16_HALF", "1") != "0" else "batch (Gf16 tables)"
+        kernel = "batch (table kernels)"
     elif spec == "uneven":
         res = uneven_batch(dev, max(16, int(args.case_mib)), max(1, args.steps))
         print(json.dumps({"case": args.case, **res}))

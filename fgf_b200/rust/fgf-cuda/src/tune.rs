@@ -1,4 +1,4 @@
-//! Kernel-family choice (`fgfc_tune_*`): split-nibble tables, byte tables or
+//! Kernel-family choice (`fgfc_tune_*`): 32-word tables (`nibble`), byte tables or
 //! the tensor-core GF(2) contraction; all give the same bytes.
 use std::ffi::CString;
 
@@ -49,7 +49,7 @@ pub fn tune_shape<F: CudaField>(nsrcs: usize, nrows: usize, row_len: usize) -> K
 }
 
 /// Element-vector columns per thread per work item of a batched
-/// split-nibble class (`fgfc_tune_set_tile`: 1, 2, 4, 8 or 16; 0 = built-in).
+/// table class (`fgfc_tune_set_tile`: 1, 2, 4, 8 or 16; 0 = built-in).
 pub fn set_tile(elem_bytes: usize, groups: usize, cols: u32) {
     check(unsafe { sys::fgfc_tune_set_tile(elem_bytes, groups, cols) });
 }

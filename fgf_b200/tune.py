@@ -1,6 +1,6 @@
 """Kernel-family choice (`fgfc_tune_*`): which kernel computes a matrix call.
 
-A call runs the split-nibble table kernels, the byte-table kernels or the
+A call runs the table kernels ("nibble"), the byte-table kernels or the
 bit-sliced tensor-core contraction; every family gives the same bytes. The
 choice per (field, sources, rows, row-length bucket) is a process-wide
 override, else a measured winner (`tune_shape`, persisted as JSON), else a
@@ -61,7 +61,7 @@ def tune_shape(field, nsrcs: int, nrows: int, row_len: int) -> str:
 
 def set_tile(elem_bytes: int, groups: int, cols: int) -> None:
     """Element-vector columns per thread per work item of a batched
-    split-nibble class (1, 2, 4, 8 or 16; 0 = built-in)."""
+    table class (1, 2, 4, 8 or 16; 0 = built-in)."""
     check(lib().fgfc_tune_set_tile(elem_bytes, groups, cols))
 
 

@@ -396,7 +396,7 @@ fgfc_status fgfc_tune_set_tile(size_t elem_bytes, size_t groups, unsigned cols);
 unsigned fgfc_tune_tile(size_t elem_bytes, size_t groups);
 /* Measures tile shapes on one submission (run on `stream`, repeatedly: its
  * jobs must be safe to run again, e.g. overwrite forms): for each
- * split-nibble class it uses, every tile shape with the other classes fixed,
+ * table class it uses, every tile shape with the other classes fixed,
  * keeping a shape that is at least 2 % faster; *us_before and *us_after
  * receive the submission's device time with the starting and the chosen
  * tiles (either may be NULL). fgfc_tune_save / fgfc_tune_load persist the
