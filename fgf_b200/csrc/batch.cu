@@ -777,7 +777,9 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   std::vector<Launch> launches;
   std::vector<UniformParams>& uparams = b->uparams;
   uparams.clear();
-  std::string key = std::to_string(reinterpret_cast<uintptr_t>(s.dev)) + ":" + std::to_string(bytes);
+  // (off_ptrs: eight pointers weigh as much as one descriptor)
+  std::string key = std::to_string(reinterpret_cast<uintptr_t>(s.dev)) + ":" + std::to_string(bytes) + ":" +
+                    std::to_string(off_ptrs);
   const int sms = sm_count();
   size_t ci = 0;
   for (auto& kv : classes) {

@@ -107,3 +107,27 @@ def test_in_place_at_any_offset(cuda, field):
             ops.mul_assign(field, t, c)
             torch.cuda.synchronize()
             assert np.array_equal(t.cpu().numpy(), want), (field.__name__, off, n)
+
+
+def test_graphs_of_submissions_with_equal_sizes(cuda):
+    """One more descriptor and eight fewer pointers give a blob of the same size
+    and the same items: a recorded graph must not serve both."""
+    field = FIELDS[1]
+    rng = np.random.default_rng(5)
+
+    def jobs(shapes):
+        out = []
+        for k, n in shapes:
+            plan = ops.Plan.matrix(field, k, 2, _coeffs(field, 2 * k, rng))
+            out.append(fb.Job(plan, [_buf(rng, n, 0)[1] for _ in range(k)], _buf(rng, 2 * n, 0)[1], n, 2))
+        return out
+
+    first = jobs([(20, 4096), (5, 4096), (5, 4096)])
+    second = jobs([(20, 8192), (20, 4096)])
+    runner = fb.Batch()
+    for submission in [first] * 4 + [second]:
+        runner.run(submission)
+    for j in first + second:
+        want = torch.zeros_like(j.dst)
+        ops.dot_product_matrix_with(want, j.row_len, 2, j.plan, j.srcs)
+        assert torch.equal(j.dst, want)
