@@ -28,11 +28,11 @@
 // word per product, the issue slots of the operations around them (address dot
 // product, XOR, index masks). Measured on B200 against the kernels it replaced, with 32
 // table copies per lane (or unreplicated nibbles for 8-byte elements):
-//   GF(2^64) RS(10,4), 16 MiB shards     308 -> 173 us (lookups per element 992 -> 483)
+//   GF(2^64) RS(10,4), 16 MiB shards     308 -> 173 us (lookups per element 992 -> 459)
 //   256 stripes of Gf8D and Gf16, k 4..32, m 1..8, 4 KiB .. 4 MiB, one batch
-//                                        3260 -> 1540 us (more CTAs resident, no 216 KiB refills)
-//   Gf8D RS(12,4), 1000003-byte shards at any offset, 18 -> 4 us on the device
-//   (whole-element bytes one at a time before, 16-byte granules spliced now)
+//                                        3240 -> 1434 us (more CTAs resident, no 216 KiB refills)
+//   Gf8D RS(12,4), consecutive shards of 1000003 bytes: 24.1 -> 7.7 us (single
+//   bytes before, 16-byte granules spliced now)
 #pragma once
 #include <cuda_runtime.h>
 
