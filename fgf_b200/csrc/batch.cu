@@ -608,9 +608,12 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   for (auto& kv : classes) {
     BatchClass& c = kv.second;
     if (c.K == 0) {
-      // Items of about equal work, 16 for every resident CTA, at most the class's
+      // Items of about equal work, two for every resident CTA, at most the class's
       // tile shape (tune.cpp: tile_cols; 8 columns per thread built in); the
-      // stripes with the most sources, whose items are the longest, first.
+      // stripes with the most sources, whose items are the longest, first. An
+      // item's start (descriptors, tables, a cold pipeline) costs more than the
+      // last items' imbalance: 256 mixed stripes with 16, 8, 4, 3, 2 items per
+      // CTA 1438, 1384, 1343, 1332, 1320 us.
       const int G = static_cast<int>((jobs[c.jobs[0]].nrows * c.E + 3) / 4);
       const uint64_t tile = c.E == 8 ? kTileColsDefault : tile_cols(c.E, G);
       if (c.E < 8) b->last_classes.emplace_back(c.E, G);
@@ -619,7 +622,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       uint64_t total = 0;  // tiles times sources
       for (uint32_t i : c.jobs) total += lut_tiles(dj[i].lut.g, mode, kLutThreads) * jobs[i].k;
       c.cost = static_cast<double>(total) * c.shape.nv * c.shape.w * (16 / c.E);
-      const uint64_t slots = 16 * static_cast<uint64_t>(sm_count() * c.kern.ctas);
+      const uint64_t slots = 2 * static_cast<uint64_t>(sm_count() * c.kern.ctas);
       // Stripes of one plan and of the byte tables' shape: one launch per
       // kUniformJobs stripes, so that such a submission counts the same launches
       // whatever its size and alignment.

@@ -30,7 +30,7 @@
 // table copies per lane (or unreplicated nibbles for 8-byte elements):
 //   GF(2^64) RS(10,4), 16 MiB shards     308 -> 173 us (lookups per element 992 -> 459)
 //   256 stripes of Gf8D and Gf16, k 4..32, m 1..8, 4 KiB .. 4 MiB, one batch
-//                                        3240 -> 1434 us (more CTAs resident, no 216 KiB refills)
+//                                        3240 -> 1320 us (more CTAs resident, no 216 KiB refills)
 //   Gf8D RS(12,4), consecutive shards of 1000003 bytes: 24.1 -> 7.7 us (single
 //   bytes before, 16-byte granules spliced now)
 #pragma once
