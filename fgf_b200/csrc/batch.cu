@@ -608,15 +608,23 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   for (auto& kv : classes) {
     BatchClass& c = kv.second;
     if (c.K == 0) {
-      // Items of about equal work, two for every resident CTA, at most the class's
-      // tile shape (tune.cpp: tile_cols; 8 columns per thread built in); the
-      // stripes with the most sources, whose items are the longest, first. An
-      // item's start (descriptors, tables, a cold pipeline) costs more than the
-      // last items' imbalance: 256 mixed stripes with 16, 8, 4, 3, 2 items per
-      // CTA 1438, 1384, 1343, 1332, 1320 us.
-      const int G = static_cast<int>((jobs[c.jobs[0]].nrows * c.E + 3) / 4);
-      const uint64_t tile = c.E == 8 ? kTileColsDefault : tile_cols(c.E, G);
-      if (c.E < 8) b->last_classes.emplace_back(c.E, G);
+      // Items of about equal work, two for every resident CTA, at most the tile
+      // shape of the job's groups (tune.cpp: tile_cols; 8 columns per thread built
+      // in; jobs of 3 and 4 groups share a class); the stripes with the most
+      // sources, whose items are the longest, first. An item's start
+      // (descriptors, tables, a cold pipeline) costs more than the last items'
+      // imbalance: 256 mixed stripes with 16, 8, 4, 3, 2 items per CTA 1438,
+      // 1384, 1343, 1332, 1320 us.
+      uint64_t tile[5] = {0};  // by groups
+      const auto job_tile = [&](uint32_t i) -> uint64_t {
+        if (c.E == 8) return kTileColsDefault;
+        const int G = static_cast<int>((jobs[i].nrows * c.E + 3) / 4);
+        if (!tile[G]) {
+          tile[G] = static_cast<uint64_t>(tile_cols(c.E, G));
+          b->last_classes.emplace_back(c.E, G);
+        }
+        return tile[G];
+      };
       const int mode = kv.first % 3;
       std::stable_sort(c.jobs.begin(), c.jobs.end(), [&](uint32_t p, uint32_t q) { return jobs[p].k > jobs[q].k; });
       uint64_t total = 0;  // tiles times sources
@@ -632,7 +640,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         const uint32_t i = c.jobs[q];
         if (one_plan && q && q % kUniformJobs == 0) c.cuts.push_back(c.items.size());
         LutBatchJob& J = dj[i].lut;
-        const uint64_t per = std::max<uint64_t>(1, std::min<uint64_t>(tile, total / (slots * jobs[i].k)));
+        const uint64_t per = std::max<uint64_t>(1, std::min<uint64_t>(job_tile(i), total / (slots * jobs[i].k)));
         J.parts = static_cast<uint32_t>((lut_tiles(J.g, mode, kLutThreads) + per - 1) / per);
         const uint32_t n = J.parts + (lut_has_edges(J.g, mode) ? 1u : 0u);
         for (uint32_t p = 0; p < n; ++p) c.items.push_back(make_uint2(i, p));
