@@ -1051,6 +1051,14 @@ fgfc_status fgfc_batch_stats(const fgfc_batch* batch, size_t* launches, size_t* 
 fgfc_status fgfc_batch_run(fgfc_batch* batch, const fgfc_matrix_job* jobs, size_t njobs,
                            fgfc_stream stream) {
   if (!batch || (njobs && !jobs)) return fail(FGFC_ERR_ARG, "batch: null argument");
+  // A graph recorded from this call would replay whatever its descriptor slot
+  // holds by then, and the slot's event would belong to the recording.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaError_t e = cudaStreamIsCapturing(stream, &cap); e != cudaSuccess) return cuda_fail(e, "batch");
+  if (cap != cudaStreamCaptureStatusNone)
+    for (size_t i = 0; i < njobs; ++i)
+      if (jobs[i].nsrcs && jobs[i].nrows && jobs[i].row_len)
+        return fail(FGFC_ERR_ARG, "batch_run: the stream is being captured; this call cannot be recorded");
   std::vector<LoweredJob> low;
   std::vector<Gf2Job> tc;
   low.reserve(njobs);

@@ -931,21 +931,15 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // still runs (the slot is free: its last submission finished), and the
   // caller's stream waits for it: in line the copy and the gaps around it cost
   // 10 us between two submissions (64 stripes of 1 MiB shards, RS(10,4): encode
-  // 192.5 -> 186.9 us, rebuild 203.5 -> 199.9). A caller that is capturing gets the copy in
-  // line, since its graph may not depend on work outside it. Launches that carry
-  // everything in their parameters need no blob.
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  e = cudaStreamIsCapturing(stream, &cap);
-  if (e != cudaSuccess) return e;
-  const bool inline_copy = cap != cudaStreamCaptureStatusNone;
+  // 192.5 -> 186.9 us, rebuild 203.5 -> 199.9). Launches that carry everything in
+  // their parameters need no blob.
   bool blob = false;
   for (const Launch& L : launches) blob = blob || !L.ufn;
-  if (inline_copy) key += "|copy";
   if (!b->capture) {
     e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking);
     if (e != cudaSuccess) return e;
   }
-  if (blob && !inline_copy) {
+  if (blob) {
     e = cudaMemcpyAsync(s.dev, s.host, bytes, cudaMemcpyHostToDevice, b->capture);
     if (e == cudaSuccess) e = cudaEventRecord(s.up, b->capture);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, s.up, 0);
@@ -955,8 +949,6 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // i % kSideStreams) and join back
   auto enqueue = [&](cudaStream_t st) -> cudaError_t {
     cudaError_t err = cudaSuccess;
-    if (blob && inline_copy) err = cudaMemcpyAsync(s.dev, s.host, bytes, cudaMemcpyHostToDevice, st);
-    if (err != cudaSuccess) return err;
     if (nside) {
       err = cudaEventRecord(b->fork, st);
       for (int i = 0; i < nside && err == cudaSuccess; ++i) err = cudaStreamWaitEvent(b->side[i], b->fork, 0);

@@ -288,7 +288,10 @@ void fgfc_batch_destroy(fgfc_batch *batch);
  * (default on). */
 fgfc_status fgfc_batch_set_graphs(fgfc_batch *batch, int enable);
 /* Enqueue all jobs on `stream`. Jobs must not write memory another job of the
- * same submission reads or writes. */
+ * same submission reads or writes. A call made while `stream` is being
+ * captured returns FGFC_ERR_ARG and enqueues nothing (unless no job has
+ * sources): the runner reuses its descriptors, so a recorded submission could
+ * not be replayed. Record the per-call ops instead. */
 fgfc_status fgfc_batch_run(fgfc_batch *batch, const fgfc_matrix_job *jobs, size_t njobs,
                            fgfc_stream stream);
 /* Statistics of the last submission: kernel launches issued, work items,
