@@ -53,10 +53,17 @@ def _buf(x) -> tuple[int, int]:
 def _stream(stream) -> int:
     if stream is None:
         torch = sys.modules.get("torch")
-        if torch is None or not torch.cuda.is_initialized():
+        if torch is None:
             return 0
-        # the handle of torch.cuda.current_stream(), without building a Stream object
-        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+        try:
+            if not torch.cuda.is_initialized():
+                return 0
+            # the handle of torch.cuda.current_stream(), without building a Stream object
+            return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+        except AttributeError:  # torch lacks these names, or another thread is still importing it
+            import torch
+
+            return int(torch.cuda.current_stream().cuda_stream) if torch.cuda.is_initialized() else 0
     if hasattr(stream, "cuda_stream"):
         return int(stream.cuda_stream)
     return int(stream)
