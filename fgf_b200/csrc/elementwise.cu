@@ -238,18 +238,28 @@ __device__ __forceinline__ void mul_planes(const uint32_t* a, const uint32_t* b,
 
 // ---------------------------------------------------------------- kernel
 
-__device__ __forceinline__ uint4 edge_bytes(const uint8_t* p, uint32_t n) {
-  uint32_t w[4] = {0, 0, 0, 0};
+// An element at p, bytewise, in the low bytes of a vector.
+template <int E>
+__device__ __forceinline__ uint4 get_element(const uint8_t* p) {
+  uint32_t w[2] = {0, 0};
 #pragma unroll
-  for (uint32_t b = 0; b < 16; ++b)
-    if (b < n) w[b >> 2] |= static_cast<uint32_t>(p[b]) << (8 * (b & 3));
-  return make_uint4(w[0], w[1], w[2], w[3]);
+  for (int i = 0; i < E; ++i) w[i / 4] |= static_cast<uint32_t>(p[i]) << (8 * (i & 3));
+  return make_uint4(w[0], w[1], 0, 0);
+}
+template <int E>
+__device__ __forceinline__ void put_element(uint8_t* p, const uint4& v) {
+#pragma unroll
+  for (int i = 0; i < E; ++i) p[i] = static_cast<uint8_t>((i < 4 ? v.x : v.y) >> (8 * (i & 3)));
 }
 
 // nvec 16-byte vectors from byte `head` on, whole warps taking blocks of 64 E;
-// the last block ends where the vectors do. One more thread takes the head and
-// the tail, fewer than 16 bytes each, as two vectors of its own. The next
-// block's vectors are in flight during the product where registers allow it.
+// the last block ends where the vectors do. One more block is the head and the
+// tail, fewer than 16 bytes each: an element of the head per lane, one of the
+// tail per lane from lane 16 on. It goes through the same code: a second copy of
+// the product for the edges alone took longer to fetch than to run (8 bytes past
+// a boundary, us, copy -> same code: Gf8D 64 KiB 2.9 -> 2.0, FP64 1.5 MiB 15.5 ->
+// 10.4, Gf64 64 MiB 90 -> 85). The next block's vectors are in flight during the
+// product where registers allow it.
 template <int E, Family F>
 __global__ void __launch_bounds__(128) elementwise_planes_kernel(uint8_t* dst, const uint8_t* a, const uint8_t* b,
                                                                  uint64_t len, uint32_t head, uint64_t nvec) {
@@ -260,6 +270,10 @@ __global__ void __launch_bounds__(128) elementwise_planes_kernel(uint8_t* dst, c
   const uint64_t nblocks = (nvec + 32 * V - 1) / (32 * V);
   const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (blockDim.x / 32);
   const uint64_t tail0 = head + 16 * nvec;
+  const uint64_t total = nblocks + (head || tail0 != len ? 1 : 0);
+  // this lane's element of the edge block
+  const uint64_t eo = (lane < 16 ? 0 : tail0) + (lane & 15u) * E;
+  const bool edge = eo < (lane < 16 ? head : len);
   uint64_t blk = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32;
   uint4 x[V], y[V];
   uint32_t pa[8 * E], pb[8 * E], pc[8 * E];
@@ -267,14 +281,14 @@ __global__ void __launch_bounds__(128) elementwise_planes_kernel(uint8_t* dst, c
   const uint64_t whole = nvec / (32 * V);
   const auto load = [&](uint64_t q) {
     const uint64_t o = head + 16 * (q * (32 * V) + lane);
-    const uint32_t left = q < whole ? 32 * V : static_cast<uint32_t>(nvec - q * (32 * V));
-    if (left == 32 * V) {
+    if (q < whole) {
 #pragma unroll
       for (int j = 0; j < V; ++j) {
         x[j] = ldg16(a + o + 512 * j);
         y[j] = ldg16(b + o + 512 * j);
       }
     } else {
+      const uint32_t left = q < nblocks ? static_cast<uint32_t>(nvec - q * (32 * V)) : 0u;
 #pragma unroll
       for (int j = 0; j < V; ++j) {
         x[j] = y[j] = make_uint4(0, 0, 0, 0);
@@ -283,14 +297,18 @@ __global__ void __launch_bounds__(128) elementwise_planes_kernel(uint8_t* dst, c
           y[j] = ldg16(b + o + 512 * j);
         }
       }
+      if (q == nblocks && edge) {
+        x[0] = get_element<E>(a + eo);
+        y[0] = get_element<E>(b + eo);
+      }
     }
   };
-  if (kAhead && blk < nblocks) load(blk);
-  for (; blk < nblocks; blk += warps) {
+  if (kAhead && blk < total) load(blk);
+  for (; blk < total; blk += warps) {
     if (!kAhead) load(blk);
     to_planes<E>(x, pa, sh);
     to_planes<E>(y, pb, sh);
-    if (kAhead && blk + warps < nblocks) load(blk + warps);
+    if (kAhead && blk + warps < total) load(blk + warps);
     mul_planes<8 * E, F>(pa, pb, pc);
     uint4 r[V];
     from_planes<E>(pc, r, sh);
@@ -299,24 +317,12 @@ __global__ void __launch_bounds__(128) elementwise_planes_kernel(uint8_t* dst, c
 #pragma unroll
       for (int j = 0; j < V; ++j) *reinterpret_cast<uint4*>(o + 512 * j) = r[j];
     } else {
-      const uint32_t left = static_cast<uint32_t>(nvec - blk * (32 * V));
+      const uint32_t left = blk < nblocks ? static_cast<uint32_t>(nvec - blk * (32 * V)) : 0u;
 #pragma unroll
       for (int j = 0; j < V; ++j)
         if (32 * j + lane < left) *reinterpret_cast<uint4*>(o + 512 * j) = r[j];
+      if (blk == nblocks && edge) put_element<E>(dst + eo, r[0]);
     }
-  }
-  if (blk == nblocks && lane == 0 && (head || tail0 != len)) {
-    const uint32_t nt = static_cast<uint32_t>(len - tail0);
-#pragma unroll
-    for (int j = 0; j < V; ++j) x[j] = y[j] = make_uint4(0, 0, 0, 0);
-    x[0] = edge_bytes(a, head), y[0] = edge_bytes(b, head);
-    x[1] = edge_bytes(a + tail0, nt), y[1] = edge_bytes(b + tail0, nt);
-    to_planes<E>(x, pa, sh);
-    to_planes<E>(y, pb, sh);
-    mul_planes<8 * E, F>(pa, pb, pc);
-    from_planes<E>(pc, x, sh);
-    put_bytes(dst, x[0], 0, head, true);
-    put_bytes(dst + tail0, x[1], 0, nt, true);
   }
 }
 
