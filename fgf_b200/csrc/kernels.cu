@@ -467,9 +467,11 @@ static cudaError_t launch_elementwise_fp(int field, uint8_t* dst, const uint8_t*
 // instructions, which a short vector does not amortise. us on B200, element
 // kernel / planes: Gf32 256 KiB 2.3 / 3.1, 512 KiB 3.3 / 3.3; FP32 128 KiB 3.5 /
 // 3.7, 256 KiB 4.8 / 3.7; Gf64 1 MiB 7.4 / 8.9, 1.5 MiB 10.2 / 9.1; FP64 768 KiB
-// 8.2 / 10.0, 1 MiB 9.9 / 10.0. 1- and 2-byte fields are level at 64 KiB.
+// 8.2 / 10.0, 1 MiB 9.9 / 10.0; Gf16 1 KiB 2.0 / 2.5, 64 KiB 2.0 / 2.45, 256 KiB
+// 2.8 / 2.35. 1-byte fields (and FP16, whose log tables take 3.5) are not slower.
 static uint64_t planes_min_bytes(int field) {
   switch (field) {
+    case kGf16: return 1u << 17;
     case kGf32: return 1u << 19;
     case kFp32: return 1u << 18;
     case kGf64: return 5u << 18;
