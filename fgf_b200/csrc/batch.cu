@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
 // at every item boundary instead; that kernel keeps the scalar heads and
 // tails of the class.
 template <int K, bool SHIFT>
-__global__ void __launch_bounds__(fast_threads(K), 1)
+__global__ void __launch_bounds__(fast_threads(K, SHIFT, true), 1)
     batch_fast_segment_kernel(const BatchDesc* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
                               const uint32_t* __restrict__ jidx, const uint64_t* __restrict__ vprefix,
                               uint32_t njobs) {
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(fast_threads(K), 1)
     // SHIFT: whole warps iterate together (the row stores shuffle between
     // lanes) and lanes past the end reload the last column
     uint32_t wn[K][4];
-    if constexpr (fast_pipe(K)) {
+    if constexpr (fast_pipe(K, SHIFT, true)) {
       const uint64_t u = v0 + threadIdx.x < vend ? v0 + threadIdx.x : vend - 1;
       fast_load<K>(s_src, J.head + (u - base) * 16u, wn);
     }
@@ -205,12 +205,12 @@ __global__ void __launch_bounds__(fast_threads(K), 1)
       const bool valid = !SHIFT || u0 < vend;
       const uint64_t u = valid ? u0 : vend - 1;
       const uint64_t off = J.head + (u - base) * 16u;
-      if (!fast_pipe(K) && u + blockDim.x < vend) {  // this thread's next column: into L2 now
+      if (!fast_pipe(K, SHIFT, true) && u + blockDim.x < vend) {  // this thread's next column: into L2 now
 #pragma unroll
         for (int t = 0; t < K; ++t) prefetch_l2(s_src[t] + off + blockDim.x * 16u);
       }
       uint32_t w[K][4];
-      if constexpr (fast_pipe(K)) {
+      if constexpr (fast_pipe(K, SHIFT, true)) {
 #pragma unroll
         for (int t = 0; t < K; ++t)
 #pragma unroll
@@ -261,7 +261,7 @@ struct UniformParams {
 static_assert(sizeof(UniformParams) <= 32000, "launch parameter block too large");
 
 template <int K, bool SHIFT>
-__global__ void __launch_bounds__(fast_threads(K), 1)
+__global__ void __launch_bounds__(fast_threads(K, SHIFT, true), 1)
     batch_fast_uniform_kernel(const __grid_constant__ UniformParams P) {
   fill_fast<K>(P.tables, nullptr);
   const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(fast_threads(K), 1)
   // lanes; a warp may straddle two stripes) and lanes past the end reload the
   // last column
   uint32_t wn[K][4];
-  if constexpr (fast_pipe(K)) {
+  if constexpr (fast_pipe(K, SHIFT, true)) {
     if (tid - (SHIFT ? lane : 0u) < vtotal) {
       const uint64_t u = tid < vtotal ? tid : vtotal - 1;
       while (u >= P.vprefix[jn + 1]) ++jn;
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(fast_threads(K), 1)
     const UJob& J = P.jobs[j];
     const uint64_t off = J.head + (u - P.vprefix[j]) * 16u;
     uint32_t w[K][4];
-    if constexpr (fast_pipe(K)) {
+    if constexpr (fast_pipe(K, SHIFT, true)) {
 #pragma unroll
       for (int t = 0; t < K; ++t)
 #pragma unroll
@@ -848,7 +848,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
           P.gprefix[q + 1] = P.gprefix[q] + (J.head + 3) / 4 + (tail + 3) / 4;
         }
         Launch U = L;
-        U.threads = static_cast<unsigned>(fast_threads(c.K));
+        U.threads = static_cast<unsigned>(fast_threads(c.K, c.shift, true));
         const uint64_t want = (std::max(P.vprefix[nq], P.gprefix[nq]) + U.threads - 1) / U.threads;
         U.grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(want, sms)));
         U.uparam = uparams.size() - 1;
@@ -873,7 +873,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         S.n = static_cast<uint32_t>(c.seg_jobs.size());
         S.seg_jobs = reinterpret_cast<const uint32_t*>(s.dev + y.first);
         S.seg_prefix = reinterpret_cast<const uint64_t*>(s.dev + y.second);
-        S.threads = static_cast<unsigned>(fast_threads(c.K));
+        S.threads = static_cast<unsigned>(fast_threads(c.K, c.shift, true));
         const uint64_t rows = (c.seg_prefix.back() + S.threads - 1) / S.threads;
         S.grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(rows, sms)));
         b->last_items += c.seg_jobs.size();

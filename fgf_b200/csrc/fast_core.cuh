@@ -63,9 +63,18 @@ constexpr int kFastThreads = 1024;
 // registers). More sources, and one alone, take 1024 threads and a prefetch of
 // each thread's next column into L2. 16 MiB rows, 4 rows out, prefetch -> two
 // columns, us: K = 6 33.2 -> 30.8, K = 8 38.8 -> 33.9, K = 10 47.7 -> 43.5; 4
-// sources of 64 MiB into one row 55.9 -> 53.8, one into one 24.8 -> 29.1.
-__host__ __device__ constexpr bool fast_pipe(int K) { return K >= 2 && K <= 10; }
-__host__ __device__ constexpr int fast_threads(int K) { return K > 4 && fast_pipe(K) ? 512 : kFastThreads; }
+// sources of 64 MiB into one row 55.9 -> 53.8, one into one 24.8 -> 29.1. Rows off
+// the sources' boundaries (shift) hold more registers: 4 sources spill, and the
+// batch kernels are slower from 4 on (4 rows, two columns -> prefetch: one call
+// over 16 MiB of 4 sources 42.5 -> 40.2; 32 stripes of 1 MiB + 4 bytes, K = 4
+// 112.8 -> 107.4, K = 6 148.4 -> 120.6, K = 8 164.2 -> 139.1, K = 10 179.2 ->
+// 155.6; K = 2 with a plan per stripe 93.4 -> 98.2).
+__host__ __device__ constexpr bool fast_pipe(int K, bool shift, bool batch) {
+  return K >= 2 && K <= 10 && !(shift && (batch ? K >= 4 : K == 4));
+}
+__host__ __device__ constexpr int fast_threads(int K, bool shift, bool batch) {
+  return K > 4 && fast_pipe(K, shift, batch) ? 512 : kFastThreads;
+}
 
 // Byte-table sources. Loads in flight live in what the tables leave of the 256
 // KiB of L1: a seventh table (28 KiB left instead of 60) saves a lookup but cost

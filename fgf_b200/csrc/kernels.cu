@@ -26,7 +26,7 @@ namespace {
 // (tune.cpp): short rows use the 32-word tables (lut.cuh), which fill faster.
 
 template <int K, bool OVR, bool SHIFT>
-__global__ void __launch_bounds__(fast_threads(K), 1) matrix_fast_kernel(const __grid_constant__ MatrixLaunch a) {
+__global__ void __launch_bounds__(fast_threads(K, SHIFT, false), 1) matrix_fast_kernel(const __grid_constant__ MatrixLaunch a) {
   fill_fast<K>(a.tables, a.inline_tab);
   const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(fast_threads(K), 1) matrix_fast_kernel(const _
   // SHIFT: whole warps iterate together (the row stores shuffle between lanes)
   uint64_t vb = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x - (SHIFT ? lane : 0u);
   uint32_t wn[K][4];
-  if constexpr (fast_pipe(K)) {
+  if constexpr (fast_pipe(K, SHIFT, false)) {
     const uint64_t v = SHIFT ? vb + lane : vb;
     if (vb < a.nvec) fast_load<K>(a.src, a.head + (v < a.nvec ? v : a.nvec - 1) * 16u, wn);
   }
@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(fast_threads(K), 1) matrix_fast_kernel(const _
     const bool valid = !SHIFT || v < a.nvec;
     const uint64_t off = a.head + (valid ? v : a.nvec - 1) * 16u;
     uint32_t w[K][4];
-    if constexpr (fast_pipe(K)) {
+    if constexpr (fast_pipe(K, SHIFT, false)) {
 #pragma unroll
       for (int t = 0; t < K; ++t)
 #pragma unroll
@@ -73,10 +73,10 @@ cudaError_t launch_fast_k(const MatrixLaunch& a, cudaStream_t s) {
   cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(matrix_fast_kernel<K, OVR, SHIFT>),
                                    FastLayout<K>::smem);
   if (e != cudaSuccess) return e;
-  const uint64_t want = (a.nvec + fast_threads(K) - 1) / fast_threads(K);
+  const uint64_t want = (a.nvec + fast_threads(K, SHIFT, false) - 1) / fast_threads(K, SHIFT, false);
   const uint64_t cap = static_cast<uint64_t>(sm_count());
   const unsigned blocks = static_cast<unsigned>(want < cap ? want : cap);
-  matrix_fast_kernel<K, OVR, SHIFT><<<blocks, fast_threads(K), FastLayout<K>::smem, s>>>(a);
+  matrix_fast_kernel<K, OVR, SHIFT><<<blocks, fast_threads(K, SHIFT, false), FastLayout<K>::smem, s>>>(a);
   return cudaGetLastError();
 }
 
