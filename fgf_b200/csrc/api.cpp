@@ -189,10 +189,9 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
   for (size_t t = 0; t < k; ++t) same &= (reinterpret_cast<uintptr_t>(srcs[t]) & 15) == al;
   const uint64_t head = std::min<uint64_t>((16 - al) & 15, len);
 
-  static thread_local LutArgs a;  // large (inline images): keep off the stack
-  const bool byte_tables = same && len - head >= 16 && choose_kernel(field, k, m, len) == FGFC_KERNEL_BYTE;
-  if (byte_tables) {
+  if (same && len - head >= 16 && choose_kernel(field, k, m, len) == FGFC_KERNEL_BYTE) {
     static thread_local MatrixLaunch f;
+    f.len = len;
     f.head = head;
     f.nvec = (len - head) / 16;
     f.k = static_cast<uint32_t>(k);
@@ -205,10 +204,10 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
     if (!f.tables) build_compact_tables(field, cs.host, m, k, f.inline_tab);
     std::lock_guard<std::mutex> lk(g_launch_mu);
     cudaError_t e = launch_fast_matrix(overwrite, f, stream);
-    if (e != cudaSuccess) return cuda_fail(e, name);
-    if (!head && len % 16 == 0) return ok();
+    return e == cudaSuccess ? ok() : cuda_fail(e, name);
   }
 
+  static thread_local LutArgs a;  // large (inline images): keep off the stack
   size_t img_off = 0;
   for (size_t r0 = 0; r0 < m; r0 += lut_rows(E)) {
     const size_t nr = std::min(lut_rows(E), m - r0);
@@ -217,7 +216,6 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
     if (kc == 0) return fail(FGFC_ERR_LIMIT, "%s: internal tiling failed", name);
     bool off = !same;
     for (size_t j = 0; j < nr; ++j) off |= (reinterpret_cast<uintptr_t>(rows[r0 + j]) & 15) != al;
-    off &= !byte_tables;  // the byte-table kernel left a head and a tail
     const bool overlap = off && any_overlap(srcs, k, rows + r0, nr, len);
     const LutMode mode = !off ? kAligned : same && !overlap ? kRowsOff : kAnyOff;
     a.g.len = len;
@@ -240,7 +238,7 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
       cudaError_t e;
       {
         std::lock_guard<std::mutex> lk(g_launch_mu);
-        e = lut_launch(field, nr, a, mode, byte_tables, stream);
+        e = lut_launch(field, nr, a, mode, stream);
       }
       if (e != cudaSuccess) return cuda_fail(e, name);
     }

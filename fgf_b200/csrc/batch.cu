@@ -108,30 +108,11 @@ __global__ void __launch_bounds__(kFastThreads, 1)
             store_col4(acc, s_dst, J.nrows, off, ovr);
         }
       } else {
-        const uint64_t tail0 = J.head + J.nvec * 16u;
-        const uint64_t n0 = (J.head + 3) / 4, n1 = (J.len - tail0 + 3) / 4;
         const uint64_t gi = static_cast<uint64_t>(wi.y - J.nv_items) * kFastGroupsPerItem + threadIdx.x;
-        if (gi < n0 + n1) {
-          const uint64_t off = gi < n0 ? 4 * gi : tail0 + 4 * (gi - n0);
-          const uint64_t end = gi < n0 ? J.head : J.len;
-          const int nb = static_cast<int>(end - off < 4 ? end - off : 4);
-          uint32_t w[K][1];
-#pragma unroll
-          for (int t = 0; t < K; ++t) {
-            uint32_t x = 0;
-            for (int b = 0; b < nb; ++b) x |= static_cast<uint32_t>(s_src[t][off + b]) << (8 * b);
-            w[t][0] = x;
-          }
-          uint32_t acc[4] = {0, 0, 0, 0};
-          fast_fold<K, 1>(w, acc, lane4);
-          for (uint32_t rr = 0; rr < J.nrows; ++rr) {
-            const uint32_t o = row_word4(acc, static_cast<int>(rr));
-            uint8_t* d = s_dst[rr] + off;
-            for (int b = 0; b < nb; ++b) {
-              const uint8_t v = static_cast<uint8_t>(o >> (8 * b));
-              d[b] = ovr ? v : static_cast<uint8_t>(d[b] ^ v);
-            }
-          }
+        if (gi < fast_groups(J.len, J.head, J.nvec)) {
+          uint64_t off;
+          const int nb = fast_group(J.len, J.head, J.nvec, gi, &off);
+          fast_bytes<K>(s_src, s_dst, J.nrows, off, nb, ovr, lane4);
         }
       }
     }
@@ -324,29 +305,9 @@ __global__ void __launch_bounds__(fast_threads(K, SHIFT, true), 1)
   for (uint64_t u = tid; u < gtotal; u += stride) {
     while (u >= P.gprefix[j + 1]) ++j;
     const UJob& J = P.jobs[j];
-    const uint64_t gi = u - P.gprefix[j];
-    const uint64_t tail0 = J.head + J.nvec * 16u;
-    const uint64_t n0 = (J.head + 3) / 4;
-    const uint64_t off = gi < n0 ? 4 * gi : tail0 + 4 * (gi - n0);
-    const uint64_t end = gi < n0 ? J.head : J.len;
-    const int nb = static_cast<int>(end - off < 4 ? end - off : 4);
-    uint32_t w[K][1];
-#pragma unroll
-    for (int t = 0; t < K; ++t) {
-      uint32_t x = 0;
-      for (int bb = 0; bb < nb; ++bb) x |= static_cast<uint32_t>(J.src[t][off + bb]) << (8 * bb);
-      w[t][0] = x;
-    }
-    uint32_t acc[4] = {0, 0, 0, 0};
-    fast_fold<K, 1>(w, acc, lane4);
-    for (uint32_t rr = 0; rr < J.nrows; ++rr) {
-      const uint32_t o = row_word4(acc, static_cast<int>(rr));
-      uint8_t* d = J.dst[rr] + off;
-      for (int bb = 0; bb < nb; ++bb) {
-        const uint8_t v = static_cast<uint8_t>(o >> (8 * bb));
-        d[bb] = J.ovr ? v : static_cast<uint8_t>(d[bb] ^ v);
-      }
-    }
+    uint64_t off;
+    const int nb = fast_group(J.len, J.head, J.nvec, u - P.gprefix[j], &off);
+    fast_bytes<K>(J.src, J.dst, J.nrows, off, nb, J.ovr != 0, lane4);
   }
 }
 
@@ -654,8 +615,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     for (uint32_t i : c.jobs) {
       // vectors: the segmented launch; scalar heads and tails: work items
       BatchJob& J = dj[i].byte;
-      const uint64_t tail = J.len - J.head - 16 * J.nvec;
-      const uint64_t ngroups = (J.head + 3) / 4 + (tail + 3) / 4;
+      const uint64_t ngroups = fast_groups(J.len, J.head, J.nvec);
       const uint64_t ns_items = (ngroups + kFastGroupsPerItem - 1) / kFastGroupsPerItem;
       J.nv_items = static_cast<uint32_t>((J.nvec + kFastVecPerItem - 1) / kFastVecPerItem);
       if (J.nvec) {
@@ -843,9 +803,8 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
           U.nvec = J.nvec;
           U.nrows = static_cast<uint32_t>(LJ.nrows);
           U.ovr = LJ.ovr ? 1u : 0u;
-          const uint64_t tail = J.len - J.head - 16 * J.nvec;
           P.vprefix[q + 1] = P.vprefix[q] + J.nvec;
-          P.gprefix[q + 1] = P.gprefix[q] + (J.head + 3) / 4 + (tail + 3) / 4;
+          P.gprefix[q + 1] = P.gprefix[q] + fast_groups(J.len, J.head, J.nvec);
         }
         Launch U = L;
         U.threads = static_cast<unsigned>(fast_threads(c.K, c.shift, true));
@@ -1194,9 +1153,8 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
       J.ovr = S.overwrite ? 1u : 0u;
       J.src_idx = src_idx;
       J.dst_idx = dst_idx;
-      const uint64_t tail = J.len - J.head - 16 * J.nvec;
       J.nv_items = static_cast<uint32_t>((J.nvec + kFastVecPerItem - 1) / kFastVecPerItem);
-      nitems = J.nv_items + ((J.head + 3) / 4 + (tail + 3) / 4 + kFastGroupsPerItem - 1) / kFastGroupsPerItem;
+      nitems = J.nv_items + (fast_groups(J.len, J.head, J.nvec) + kFastGroupsPerItem - 1) / kFastGroupsPerItem;
       class_smem[cls][var] = fast_smem(cls);
     } else {
       build_lut_images(field, cm, S.nrows, 0, S.nsrcs, 0, S.nrows, ht + tn);

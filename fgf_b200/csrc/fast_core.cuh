@@ -214,6 +214,41 @@ __device__ __forceinline__ uint32_t row_word4(const uint32_t* acc, int rr) {
   return prmt(s01, s23, (rr & 1) ? 0x7632u : 0x5410u);
 }
 
+// Group gi of the 4-byte groups before (head) and after the 16-byte columns of a
+// job: nb bytes at *off.
+__device__ __forceinline__ int fast_group(uint64_t len, uint64_t head, uint64_t nvec, uint64_t gi, uint64_t* off) {
+  const uint64_t tail0 = head + nvec * 16u, n0 = (head + 3) / 4;
+  *off = gi < n0 ? 4 * gi : tail0 + 4 * (gi - n0);
+  const uint64_t end = gi < n0 ? head : len;
+  return static_cast<int>(end - *off < 4 ? end - *off : 4);
+}
+__host__ __device__ inline uint64_t fast_groups(uint64_t len, uint64_t head, uint64_t nvec) {
+  return (head + 3) / 4 + (len - head - 16 * nvec + 3) / 4;
+}
+
+// Bytes [off, off + nb) of the rows, one thread, bytewise.
+template <int K>
+__device__ __forceinline__ void fast_bytes(const uint8_t* const* src, uint8_t* const* dst, uint32_t nrows, uint64_t off,
+                                           int nb, bool ovr, uint32_t lane4) {
+  uint32_t w[K][1];
+#pragma unroll
+  for (int t = 0; t < K; ++t) {
+    uint32_t x = 0;
+    for (int b = 0; b < nb; ++b) x |= static_cast<uint32_t>(src[t][off + b]) << (8 * b);
+    w[t][0] = x;
+  }
+  uint32_t acc[4] = {0, 0, 0, 0};
+  fast_fold<K, 1>(w, acc, lane4);
+  for (uint32_t rr = 0; rr < nrows; ++rr) {
+    const uint32_t o = row_word4(acc, static_cast<int>(rr));
+    uint8_t* d = dst[rr] + off;
+    for (int b = 0; b < nb; ++b) {
+      const uint8_t v = static_cast<uint8_t>(o >> (8 * b));
+      d[b] = ovr ? v : static_cast<uint8_t>(d[b] ^ v);
+    }
+  }
+}
+
 // ---------------------------------------------------------------- row stores
 //
 // The vector paths compute 16-byte columns in the alignment of the sources.

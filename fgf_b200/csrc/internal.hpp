@@ -22,6 +22,7 @@ constexpr size_t kFastMaxSources = 14;   // byte-table kernels: sources per laun
 constexpr int kCompactWords = 32;
 
 struct MatrixLaunch {
+  uint64_t len;            // bytes per row
   uint64_t head;           // bytes before the vector body
   uint64_t nvec;           // 16-byte vectors in the body
   uint32_t k;              // sources
@@ -127,7 +128,7 @@ size_t lut_image_words(int E, size_t k, size_t m);
 void build_lut_images(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t r0, size_t nr,
                       uint32_t* out);
 // Launch one job (rows of one lut_shape).
-cudaError_t lut_launch(int field, size_t nr, LutArgs& a, int mode, bool edges_only, cudaStream_t s);
+cudaError_t lut_launch(int field, size_t nr, LutArgs& a, int mode, cudaStream_t s);
 // One descriptor of a batched submission: a byte-table sub-job (batch.cu) or a
 // table sub-job (lut_batch.cuh).
 struct BatchJob {
@@ -162,13 +163,12 @@ LutBatchKernel lut_batch_e1(int lev, int w, int mode);
 LutBatchKernel lut_batch_e2(int lev, int w, int mode);
 LutBatchKernel lut_batch_e4(int lev, int w, int mode);
 LutBatchKernel lut_batch_e8(int lev, int w, int mode);
-cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only);
-cudaError_t lut_launch_e2(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only);
-cudaError_t lut_launch_e4(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only);
-cudaError_t lut_launch_e8(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only);
+cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, int mode);
+cudaError_t lut_launch_e2(int lev, int w, LutArgs& a, cudaStream_t s, int mode);
+cudaError_t lut_launch_e4(int lev, int w, LutArgs& a, cudaStream_t s, int mode);
+cudaError_t lut_launch_e8(int lev, int w, LutArgs& a, cudaStream_t s, int mode);
 
-// The byte-table kernel (kernels.cu; Gf8, at most 4 rows, <= 14 sources) over
-// the vector body of a call; `overwrite` selects dot-product (overwrite) or
+// The byte-table kernel (kernels.cu; Gf8, at most 4 rows, <= 14 sources); `overwrite` selects dot-product (overwrite) or
 // mul_add (accumulate) semantics.
 cudaError_t launch_fast_matrix(bool overwrite, const MatrixLaunch& a, cudaStream_t s);
 // Fill `n` rows of `len` bytes with zero.

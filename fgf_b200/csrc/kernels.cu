@@ -31,7 +31,17 @@ __global__ void __launch_bounds__(fast_threads(K, SHIFT, false), 1) matrix_fast_
   const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   const uint32_t lane = threadIdx.x & 31u;
+  // Head and tail, at most 8 groups: the last warp, whose columns end first. In a
+  // launch of the table kernel of their own they cost 3 to 6 us a call (4 bytes
+  // past 16 MiB, k = 1 10.6 -> 7.9, RS(10,4) 49.4 -> 45.3).
+  const uint32_t last = gridDim.x * blockDim.x - 32u;
+  if (blockIdx.x * blockDim.x + threadIdx.x >= last && lane < fast_groups(a.len, a.head, a.nvec)) {
+    uint64_t off;
+    const int nb = fast_group(a.len, a.head, a.nvec, lane, &off);
+    fast_bytes<K>(a.src, a.dst, a.nrows, off, nb, OVR, lane4);
+  }
   // SHIFT: whole warps iterate together (the row stores shuffle between lanes)
+  __syncwarp();
   uint64_t vb = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x - (SHIFT ? lane : 0u);
   uint32_t wn[K][4];
   if constexpr (fast_pipe(K, SHIFT, false)) {

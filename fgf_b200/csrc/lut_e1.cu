@@ -3,11 +3,11 @@
 
 namespace fgfc {
 
-cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only) {
-  if (lev == 0 && w == 1) return lut_launch_lw<1, 0, 1>(a, s, mode, edges_only);
-  if (lev == 0 && w == 2) return lut_launch_lw<1, 0, 2>(a, s, mode, edges_only);
-  if (lev == 0 && w == 3) return lut_launch_lw<1, 0, 3>(a, s, mode, edges_only);
-  if (lev == 0 && w == 4) return lut_launch_lw<1, 0, 4>(a, s, mode, edges_only);
+cudaError_t lut_launch_e1(int lev, int w, LutArgs& a, cudaStream_t s, int mode) {
+  if (lev == 0 && w == 1) return lut_launch_lw<1, 0, 1>(a, s, mode);
+  if (lev == 0 && w == 2) return lut_launch_lw<1, 0, 2>(a, s, mode);
+  if (lev == 0 && w == 3) return lut_launch_lw<1, 0, 3>(a, s, mode);
+  if (lev == 0 && w == 4) return lut_launch_lw<1, 0, 4>(a, s, mode);
   return cudaErrorInvalidValue;
 }
 

@@ -3,10 +3,10 @@
 
 namespace fgfc {
 
-cudaError_t lut_launch_e2(int lev, int w, LutArgs& a, cudaStream_t s, int mode, bool edges_only) {
-  if (lev == 0 && w == 1) return lut_launch_lw<2, 0, 1>(a, s, mode, edges_only);
-  if (lev == 1 && w == 1) return lut_launch_lw<2, 1, 1>(a, s, mode, edges_only);
-  if (lev == 1 && w == 2) return lut_launch_lw<2, 1, 2>(a, s, mode, edges_only);
+cudaError_t lut_launch_e2(int lev, int w, LutArgs& a, cudaStream_t s, int mode) {
+  if (lev == 0 && w == 1) return lut_launch_lw<2, 0, 1>(a, s, mode);
+  if (lev == 1 && w == 1) return lut_launch_lw<2, 1, 1>(a, s, mode);
+  if (lev == 1 && w == 2) return lut_launch_lw<2, 1, 2>(a, s, mode);
   return cudaErrorInvalidValue;
 }
 

@@ -36,12 +36,12 @@ __global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, MODE>())
     lut_edges<L, LEV, W, MODE>(a.g, sh, stage, ovr, fp);
     return;
   }
-  if (a.ntiles) lut_run<L, LEV, W, MODE>(a.g, sh, blockIdx.x, nwork, ovr, fp);
+  lut_run<L, LEV, W, MODE>(a.g, sh, blockIdx.x, nwork, ovr, fp);
 }
 
 // Launch one job of this (LEV, W); `a` is complete but for its tiling.
 template <int E, int LEV, int W, int MODE>
-cudaError_t lut_launch_one(LutArgs& a, cudaStream_t s, bool edges_only) {
+cudaError_t lut_launch_one(LutArgs& a, cudaStream_t s) {
   using L = Lut<E, LEV>;
   using S = LutSmem<L::NV, W>;
   auto kern = lut_kernel<E, LEV, W, MODE>;
@@ -52,10 +52,10 @@ cudaError_t lut_launch_one(LutArgs& a, cudaStream_t s, bool edges_only) {
   const uint64_t sms = static_cast<uint64_t>(sm_count());
   // Small calls take narrower CTAs, so that every SM gets one.
   unsigned threads = kLutThreads;
-  const uint64_t cols = edges_only ? 0 : a.g.len / 16;
+  const uint64_t cols = a.g.len / 16;
   while (threads > 64 && cols < sms * threads) threads /= 2;
   a.edge_cta = edges ? 1u : 0u;
-  a.ntiles = edges_only ? 0 : lut_tiles(a.g, MODE, threads);
+  a.ntiles = lut_tiles(a.g, MODE, threads);
   const uint64_t cap = sms * lut_min_ctas<E, LEV, W, MODE>();
   const unsigned grid = static_cast<unsigned>(a.ntiles < cap ? a.ntiles : cap) + a.edge_cta;
   if (!grid) return cudaSuccess;
@@ -64,10 +64,10 @@ cudaError_t lut_launch_one(LutArgs& a, cudaStream_t s, bool edges_only) {
 }
 
 template <int E, int LEV, int W>
-cudaError_t lut_launch_lw(LutArgs& a, cudaStream_t s, int mode, bool edges_only) {
-  return mode == kAligned   ? lut_launch_one<E, LEV, W, kAligned>(a, s, edges_only)
-         : mode == kRowsOff ? lut_launch_one<E, LEV, W, kRowsOff>(a, s, edges_only)
-                            : lut_launch_one<E, LEV, W, kAnyOff>(a, s, edges_only);
+cudaError_t lut_launch_lw(LutArgs& a, cudaStream_t s, int mode) {
+  return mode == kAligned   ? lut_launch_one<E, LEV, W, kAligned>(a, s)
+         : mode == kRowsOff ? lut_launch_one<E, LEV, W, kRowsOff>(a, s)
+                            : lut_launch_one<E, LEV, W, kAnyOff>(a, s);
 }
 
 }  // namespace fgfc

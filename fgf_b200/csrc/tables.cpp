@@ -110,15 +110,15 @@ void build_lut_images(int field, const uint64_t* coeffs, size_t m, size_t t0, si
     }
 }
 
-cudaError_t lut_launch(int field, size_t nr, LutArgs& a, int mode, bool edges_only, cudaStream_t s) {
+cudaError_t lut_launch(int field, size_t nr, LutArgs& a, int mode, cudaStream_t s) {
   const int E = field_bytes(field);
   const LutShape sh = lut_shape(E, nr);
   a.fp = field == kFp16 || field == kFp32 || field == kFp64 ? 1u : 0u;
   switch (E) {
-    case 1: return lut_launch_e1(sh.lev, sh.w, a, s, mode, edges_only);
-    case 2: return lut_launch_e2(sh.lev, sh.w, a, s, mode, edges_only);
-    case 4: return lut_launch_e4(sh.lev, sh.w, a, s, mode, edges_only);
-    case 8: return lut_launch_e8(sh.lev, sh.w, a, s, mode, edges_only);
+    case 1: return lut_launch_e1(sh.lev, sh.w, a, s, mode);
+    case 2: return lut_launch_e2(sh.lev, sh.w, a, s, mode);
+    case 4: return lut_launch_e4(sh.lev, sh.w, a, s, mode);
+    case 8: return lut_launch_e8(sh.lev, sh.w, a, s, mode);
     default: return cudaErrorInvalidValue;
   }
 }
