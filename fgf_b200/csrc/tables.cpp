@@ -15,6 +15,21 @@ const Gf8Log& gf8d_tab() {
   return t;
 }
 
+Fp8Log::Fp8Log() {
+  uint8_t v = 1;
+  for (int i = 0; i < 255; ++i) {
+    exp[i] = exp[i + 255] = v;
+    log[v] = static_cast<uint8_t>(i);
+    v = static_cast<uint8_t>(fp_mul_bits(v, 0x2D, 8));
+  }
+  exp[510] = exp[511] = 1;
+  log[0] = 0;
+}
+const Fp8Log& fp8_tab() {
+  static const Fp8Log t;
+  return t;
+}
+
 void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t k, uint32_t* out) {
   for (size_t t = 0; t < k; ++t)
     for (int half = 0; half < 2; ++half)
