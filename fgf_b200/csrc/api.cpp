@@ -211,8 +211,9 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
   size_t img_off = 0;
   for (size_t r0 = 0; r0 < m; r0 += lut_rows(E)) {
     const size_t nr = std::min(lut_rows(E), m - r0);
-    const size_t kc = lut_sources(E, nr, cs.img == nullptr);
-    const size_t src_words = lut_shape(E, nr).src_words();
+    const LutShape shape = lut_shape(E, nr, k);
+    const size_t kc = lut_sources(shape, cs.img == nullptr);
+    const size_t src_words = shape.src_words();
     if (kc == 0) return fail(FGFC_ERR_LIMIT, "%s: internal tiling failed", name);
     bool off = !same;
     for (size_t j = 0; j < nr; ++j) off |= (reinterpret_cast<uintptr_t>(rows[r0 + j]) & 15) != al;
@@ -233,12 +234,12 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
         a.img = cs.img + img_off + t0 * src_words;
       } else {
         a.img = nullptr;
-        build_lut_images(field, cs.host, m, t0, kk, r0, nr, a.inl);
+        build_lut_images(field, shape, cs.host, m, t0, kk, r0, nr, a.inl);
       }
       cudaError_t e;
       {
         std::lock_guard<std::mutex> lk(g_launch_mu);
-        e = lut_launch(field, nr, a, mode, stream);
+        e = lut_launch(field, shape, a, mode, stream);
       }
       if (e != cudaSuccess) return cuda_fail(e, name);
     }
@@ -264,8 +265,9 @@ fgfc_status upload_plan_tables(fgfc_plan* p) {
     size_t off = at;
     for (size_t r0 = 0; r0 < m; r0 += lut_rows(E)) {
       const size_t nr = std::min(lut_rows(E), m - r0);
-      build_lut_images(p->field, p->values.data(), m, 0, k, r0, nr, host.data() + off);
-      off += k * lut_shape(E, nr).src_words();
+      const LutShape s = lut_shape(E, nr, k);
+      build_lut_images(p->field, s, p->values.data(), m, 0, k, r0, nr, host.data() + off);
+      off += k * s.src_words();
     }
     return at;
   };
@@ -967,7 +969,7 @@ void lower_tables(const fgfc_plan* plan, const std::vector<uint64_t>& srcs, cons
     L.srcs = srcs;
     L.dsts.assign(dsts.begin() + r0, dsts.begin() + r0 + nr);
     out.push_back(std::move(L));
-    img += srcs.size() * lut_shape(E, nr).src_words();
+    img += srcs.size() * lut_shape(E, nr, srcs.size()).src_words();
   }
 }
 

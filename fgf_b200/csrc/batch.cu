@@ -536,7 +536,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     const LoweredJob& L = jobs[i];
     const int E = field_bytes(L.field);
     const bool fast = L.byte_tab && al[i].sources && byte_cols[L.k] >= kByteClassCols;
-    const LutShape shape = lut_shape(E, L.nrows);
+    const LutShape shape = lut_shape(E, L.nrows, L.k);
     const int key = fast ? 1000 + 2 * static_cast<int>(L.k) + al[i].unal
                          : ((E * 4 + shape.lev) * 8 + shape.w) * 3 + al[i].mode;
     BatchClass& c = classes[key];
@@ -560,7 +560,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     } else {
       c.shape = shape;
       c.kern = lut_batch_kernel_for(E, shape, al[i].mode);
-      c.kc = lut_sources(E, L.nrows, false);
+      c.kc = lut_sources(shape, false);
       D.lut = lut_batch_job(L.field, L.img, al[i], L.len, L.k, L.nrows, L.ovr);
       D.lut.src_idx = idx[i].first;
       D.lut.dst_idx = idx[i].second;
@@ -1019,6 +1019,8 @@ int noalloc_class(int E, size_t nsrcs, size_t nrows) {
   if (E == 1 && G == 1 && nsrcs >= 1 && nsrcs <= static_cast<size_t>(kFastMaxK)) return static_cast<int>(nsrcs);
   return 100 + static_cast<int>(G);
 }
+// A class holds stripes of any number of sources.
+LutShape noalloc_shape(int E, size_t nr) { return lut_shape(E, nr, kMaxSrc); }
 constexpr uint32_t kNoallocCols = 4096;   // columns per item
 constexpr uint32_t kNoallocGroups = 512;  // 4-byte groups per item of the limit
 
@@ -1157,7 +1159,8 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
       nitems = J.nv_items + (fast_groups(J.len, J.head, J.nvec) + kFastGroupsPerItem - 1) / kFastGroupsPerItem;
       class_smem[cls][var] = fast_smem(cls);
     } else {
-      build_lut_images(field, cm, S.nrows, 0, S.nsrcs, 0, S.nrows, ht + tn);
+      const LutShape shape = noalloc_shape(E, S.nrows);
+      build_lut_images(field, shape, cm, S.nrows, 0, S.nsrcs, 0, S.nrows, ht + tn);
       LutBatchJob& J = hj[jn].lut;
       J = lut_batch_job(field, tables, al, S.row_len, S.nsrcs, S.nrows, S.overwrite != 0);
       J.src_idx = src_idx;
@@ -1166,8 +1169,7 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
       J.parts = static_cast<uint32_t>((lut_tiles(J.g, al.mode, kLutThreads) + per - 1) / per);
       nitems = J.parts + (lut_has_edges(J.g, al.mode) ? 1 : 0);
       class_smem[cls][var] = std::max(class_smem[cls][var],
-                                      lut_smem(lut_shape(E, S.nrows),
-                                               std::min(S.nsrcs, lut_sources(E, S.nrows, false))));
+                                      lut_smem(shape, std::min(S.nsrcs, lut_sources(shape, false))));
     }
     tn += S.nsrcs * E * G * kCompactWords;
     uint2* list = reinterpret_cast<uint2*>(g_noalloc_host + class_off[cls]);
@@ -1191,7 +1193,7 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
       if (!n) continue;
       const bool fast = c < 100 && var == 0;
       const KernelFn fn = fast ? fast_kernel_for(c, false) : nullptr;
-      const LutBatchKernel lut = fast ? LutBatchKernel{} : lut_batch_kernel_for(E, lut_shape(E, class_rows[c]), var ? kAnyOff : kAligned);
+      const LutBatchKernel lut = fast ? LutBatchKernel{} : lut_batch_kernel_for(E, noalloc_shape(E, class_rows[c]), var ? kAnyOff : kAligned);
       if (!fn && !lut.fn) {
         e = cudaErrorInvalidValue;
         break;
@@ -1212,7 +1214,7 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
       else
         lut.fn<<<static_cast<unsigned>(std::min<uint64_t>(n, sms * lut.ctas)), kLutThreads, smem, stream>>>(
             descs, ptrs, list, static_cast<uint32_t>(n), counter,
-            static_cast<uint32_t>(lut_sources(E, class_rows[c], false)));
+            static_cast<uint32_t>(lut_sources(noalloc_shape(E, class_rows[c]), false)));
       e = cudaGetLastError();
     }
   }

@@ -131,7 +131,7 @@ inline uint64_t fp_mul_alpha(uint64_t v, unsigned bits) {
 
 // The byte level's products by logarithms of its generator 0x2d. The recursion
 // below 8 bits takes 27 times as many steps, and a plan of an 8-byte field needs
-// tens of thousands of byte products (FP64, 10 x 4 coefficients: @PLAN@).
+// tens of thousands of byte products (FP64, 10 x 4 coefficients: 1240 -> 232 us).
 struct Fp8Log {
   uint8_t exp[512];
   uint8_t log[256];

@@ -104,7 +104,8 @@ struct LutArgs {
 };
 static_assert(sizeof(LutArgs) <= 4096, "launches with more than 4 KiB of parameters cost more");
 
-// Tower levels split and output words per leaf product of a launch of nr rows.
+// Tower levels split and output words per leaf product of a launch of nr rows
+// of a call of k sources.
 struct LutShape {
   int lev, w;
   size_t nv;  // leaf input bytes per element
@@ -118,17 +119,17 @@ inline uint32_t lut_smem(const LutShape& s, size_t k) {
   return static_cast<uint32_t>(k / 3 * s.smem3() + k % 3 * s.smem1() + (k + kLutRows) * kEdges * 16);
 }
 inline size_t lut_rows(int E) { return E == 1 ? 16 : E == 2 ? 8 : 4; }
-LutShape lut_shape(int E, size_t nr);
+LutShape lut_shape(int E, size_t nr, size_t k);
 // Sources per launch: table pages, pointers and (raw forms) inline images fit.
-size_t lut_sources(int E, size_t nr, bool inl);
+size_t lut_sources(const LutShape& s, bool inl);
 // Image words of k sources and m rows, launch by launch of lut_rows(E) rows.
 size_t lut_image_words(int E, size_t k, size_t m);
 // Images of sources [t0, t0 + k) and rows [r0, r0 + nr) of a term-major
 // coefficient matrix with m columns: [source][leaf byte][word][8].
-void build_lut_images(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t r0, size_t nr,
-                      uint32_t* out);
-// Launch one job (rows of one lut_shape).
-cudaError_t lut_launch(int field, size_t nr, LutArgs& a, int mode, cudaStream_t s);
+void build_lut_images(int field, const LutShape& s, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t r0,
+                      size_t nr, uint32_t* out);
+// Launch one job (rows of one shape).
+cudaError_t lut_launch(int field, const LutShape& sh, LutArgs& a, int mode, cudaStream_t s);
 // One descriptor of a batched submission: a byte-table sub-job (batch.cu) or a
 // table sub-job (lut_batch.cuh).
 struct BatchJob {

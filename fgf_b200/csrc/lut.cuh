@@ -58,6 +58,7 @@ struct Lut {
   // Index shifts on the multiply pipe: GF(2^64) RS(10,4), 16 MiB, 204 -> 173 us;
   // level or worse for the other widths.
   static constexpr bool kMulShift = E == 8;
+  static constexpr bool kDirect = LEV == 0 && E > 1;
 
   // element and leaf byte (product * H + byte) of byte b of packed word w;
   // elem() < 0: no byte there
@@ -129,6 +130,11 @@ struct LutSmem {
   static constexpr uint32_t block1 = (NV * W * 128u + 255u) / 256u * 256u;
 };
 
+// Direct shapes of several words per element (2- and 4-byte fields) serve calls of
+// one or two sources: no groups of three.
+template <class L, int W>
+constexpr bool kLutFewSources = L::kDirect && W > 1;
+
 // ---------------------------------------------------------------- table fill
 
 // Tables of k sources from their images (8 words per (source, leaf byte,
@@ -142,7 +148,7 @@ __device__ __forceinline__ void lut_fill(const uint32_t* img, uint32_t k) {
 #pragma unroll
   for (int b = 0; b < 5; ++b) m[b] = 0u - ((lane >> b) & 1u);
   const uint4* im = reinterpret_cast<const uint4*>(img);
-  const uint32_t nt = k / 3u, tasks = nt * NS;
+  const uint32_t nt = kLutFewSources<L, W> ? 0 : k / 3u, tasks = nt * NS;
 #pragma unroll 2
   for (uint32_t i = warp; i < tasks; i += nwarps) {
     const uint32_t tr = i / NS, s = i - tr * NS;
@@ -403,7 +409,7 @@ template <class L, int W, class Load, class Fix>
 __device__ __forceinline__ void lut_column(LutAcc<L, W>& A, uint32_t k, Load load, Fix fix) {
   using S = LutSmem<L::NV, W>;
   A.zero();
-  const uint32_t nt = k / 3u;
+  const uint32_t nt = kLutFewSources<L, W> ? 0 : k / 3u;
   uint4 c0 = load(0u), c1, c2;
   c1 = c2 = make_uint4(0, 0, 0, 0);
   if (k > 1) c1 = load(1u);
@@ -434,7 +440,7 @@ __device__ __forceinline__ void lut_column_ahead(LutAcc<L, W>& A, uint32_t k, Lu
                                                  Fix fix) {
   using S = LutSmem<L::NV, W>;
   A.zero();
-  const uint32_t nt = k / 3u, rest = k - 3u * nt;
+  const uint32_t nt = kLutFewSources<L, W> ? 0 : k / 3u, rest = k - 3u * nt;
   uint32_t base = 0;
   for (uint32_t i = 0; i < nt; ++i) {
     const uint32_t t = 3u * i;

@@ -16,7 +16,7 @@ namespace fgfc {
 template <int E, int LEV, int W, int MODE>
 constexpr int lut_min_ctas() {
   constexpr int n = pow3(LEV) * W * (16 / E);
-  return E == 2 && LEV == 0 && MODE != kAnyOff ? 4 : n <= 16 ? 3 : n <= 32 && MODE == kAligned ? 3 : 2;
+  return E == 2 && LEV == 0 && W == 1 && MODE != kAnyOff ? 4 : n <= 16 ? 3 : n <= 32 && MODE == kAligned ? 3 : 2;
 }
 
 template <int E, int LEV, int W, int MODE>

@@ -47,10 +47,17 @@ void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t k,
 //   2 bytes: direct 2 per 2 rows, halves 3 per 4 rows;
 //   4 bytes: direct 4 per row, 16-bit leaves 6 per 2 rows, byte leaves 9 per 4;
 //   8 bytes: 32-bit leaves 12 per row, 16-bit 18 per 2 rows, byte leaves 27 per 4.
-LutShape lut_shape(int E, size_t nr) {
+// The splits cost a fix-up per column whatever the number of sources, so the 2-
+// and 4-byte fields go direct, a word per 4 / E rows, with one source, and with
+// two unless the rows fill a split's words. 16 MiB, us, split -> direct: Gf32 k = 1,
+// m = 3 34.5 -> 19.8, m = 8 added 114 -> 78; k = 2, m = 3 43.0 -> 32.5, m = 4 44.6
+// -> 39.8 but 5.0 -> 6.1 at 64 KiB; Gf16 k = 1, m = 4 21.7 -> 16.2.
+LutShape lut_shape(int E, size_t nr, size_t k) {
   LutShape s{};
   if (E == 1) {
     s.w = static_cast<int>((nr + 3) / 4);
+  } else if (E <= 4 && (k == 1 || (k == 2 && nr * E < 16))) {
+    s.w = static_cast<int>((nr * E + 3) / 4);
   } else if (E == 2) {
     s.lev = nr > 2 ? 1 : 0;
     s.w = nr > 4 ? 2 : 1;
@@ -66,8 +73,7 @@ LutShape lut_shape(int E, size_t nr) {
   return s;
 }
 
-size_t lut_sources(int E, size_t nr, bool inl) {
-  const LutShape s = lut_shape(E, nr);
+size_t lut_sources(const LutShape& s, bool inl) {
   const size_t edge = kEdges * 16;  // staged edge columns per source and row
   size_t kc = std::min<size_t>(kMaxSrc, (kLutSmemMax - kLutRows * edge) / (s.smem3() + 3 * edge) * 3);
   if (inl) kc = std::min<size_t>(kc, kLutInlineWords / s.src_words());
@@ -76,7 +82,7 @@ size_t lut_sources(int E, size_t nr, bool inl) {
 
 size_t lut_image_words(int E, size_t k, size_t m) {
   size_t n = 0;
-  for (size_t r0 = 0; r0 < m; r0 += lut_rows(E)) n += k * lut_shape(E, std::min(lut_rows(E), m - r0)).src_words();
+  for (size_t r0 = 0; r0 < m; r0 += lut_rows(E)) n += k * lut_shape(E, std::min(lut_rows(E), m - r0), k).src_words();
   return n;
 }
 
@@ -92,10 +98,9 @@ int leaf_field(int field, int H) {
 
 }  // namespace
 
-void build_lut_images(int field, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t r0, size_t nr,
-                      uint32_t* out) {
+void build_lut_images(int field, const LutShape& s, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t r0,
+                      size_t nr, uint32_t* out) {
   const int E = field_bytes(field);
-  const LutShape s = lut_shape(E, nr);
   const int H = E >> s.lev, leaf = leaf_field(field, H);
   const size_t W = static_cast<size_t>(s.w);
   std::memset(out, 0, k * s.src_words() * sizeof(uint32_t));
@@ -125,9 +130,8 @@ void build_lut_images(int field, const uint64_t* coeffs, size_t m, size_t t0, si
     }
 }
 
-cudaError_t lut_launch(int field, size_t nr, LutArgs& a, int mode, cudaStream_t s) {
+cudaError_t lut_launch(int field, const LutShape& sh, LutArgs& a, int mode, cudaStream_t s) {
   const int E = field_bytes(field);
-  const LutShape sh = lut_shape(E, nr);
   a.fp = field == kFp16 || field == kFp32 || field == kFp64 ? 1u : 0u;
   switch (E) {
     case 1: return lut_launch_e1(sh.lev, sh.w, a, s, mode);
