@@ -100,6 +100,7 @@ struct CoeffSrc {
   const uint64_t* host = nullptr;      // term-major k x m
   const uint32_t* img = nullptr;       // table images (build_lut_images), launch by launch of rows
   const uint32_t* byte_tab = nullptr;  // compact tables [source][32] where the byte-table kernel covers the shape
+  const uint32_t* unit = nullptr;      // 8-byte plans: single-row images, coefficient by coefficient
   const uint32_t* bits = nullptr;  // GF(2) bit matrix (plans), or built from `host` when needed
 };
 
@@ -204,6 +205,12 @@ fgfc_status run_matrix(int field, const uint8_t* const* srcs, size_t k, uint8_t*
     if (!f.tables) build_compact_tables(field, cs.host, m, k, f.inline_tab);
     std::lock_guard<std::mutex> lk(g_launch_mu);
     cudaError_t e = launch_fast_matrix(overwrite, f, stream);
+    return e == cudaSuccess ? ok() : cuda_fail(e, name);
+  }
+
+  if (cs.unit && wide_chosen(field, k, m, len)) {
+    std::lock_guard<std::mutex> lk(g_launch_mu);
+    cudaError_t e = wide_launch(field, srcs, k, rows, m, cs.unit, len, overwrite, stream);
     return e == cudaSuccess ? ok() : cuda_fail(e, name);
   }
 
@@ -315,6 +322,7 @@ CoeffSrc plan_src(const fgfc_plan* p, int o, const std::vector<uint32_t>& bits) 
   CoeffSrc c;
   c.img = p->dev + p->off_img[o];
   c.byte_tab = p->off_byte[o] == SIZE_MAX ? nullptr : p->dev + p->off_byte[o];
+  if (field_bytes(p->field) == 8) c.unit = p->dev + p->off_img[2];  // gather: one row per coefficient
   c.bits = bits.empty() ? nullptr : bits.data();
   return c;
 }
@@ -1062,6 +1070,7 @@ fgfc_status fgfc_batch_run(fgfc_batch* batch, const fgfc_matrix_job* jobs, size_
   std::vector<LoweredJob> low;
   std::vector<Gf2Job> tc;
   low.reserve(njobs);
+  std::vector<size_t> own;  // long stripes of few sources of the 8-byte fields: a call each (wide.cu)
   for (size_t i = 0; i < njobs; ++i) {
     const fgfc_matrix_job& J = jobs[i];
     const char* name = J.row_starts ? (J.overwrite ? "dot_product_matrix_scattered_with"
@@ -1112,7 +1121,21 @@ fgfc_status fgfc_batch_run(fgfc_batch* batch, const fgfc_matrix_job* jobs, size_
       dsts[j] = reinterpret_cast<uint64_t>(J.dst + (J.row_starts ? J.row_starts[j] : j * J.row_len));
     std::vector<uint64_t> srcs(J.nsrcs);
     for (size_t t = 0; t < J.nsrcs; ++t) srcs[t] = reinterpret_cast<uint64_t>(J.srcs[t].ptr);
+    if (J.row_len >= kWideStripe && wide_chosen(field, J.nsrcs, J.nrows, J.row_len)) {
+      own.push_back(i);
+      continue;
+    }
     lower_matrix_job(plan, srcs, dsts, J.row_len, J.overwrite != 0, low, tc);
+  }
+  for (size_t i : own) {
+    const fgfc_matrix_job& J = jobs[i];
+    std::vector<const uint8_t*> sp(J.nsrcs);
+    std::vector<uint8_t*> rp(J.nrows);
+    for (size_t t = 0; t < J.nsrcs; ++t) sp[t] = J.srcs[t].ptr;
+    for (size_t j = 0; j < J.nrows; ++j) rp[j] = J.dst + (J.row_starts ? J.row_starts[j] : j * J.row_len);
+    fgfc_status st = run_matrix(J.plan->field, sp.data(), J.nsrcs, rp.data(), J.nrows, plan_mat(J.plan), J.row_len,
+                                J.overwrite != 0, stream, "batch");
+    if (st != FGFC_OK) return st;
   }
   cudaError_t e = batch_run(batch->state, low, tc, stream);
   return e == cudaSuccess ? ok() : cuda_fail(e, "batch");

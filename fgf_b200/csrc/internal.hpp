@@ -130,6 +130,16 @@ void build_lut_images(int field, const LutShape& s, const uint64_t* coeffs, size
                       size_t nr, uint32_t* out);
 // Launch one job (rows of one shape).
 cudaError_t lut_launch(int field, const LutShape& sh, LutArgs& a, int mode, cudaStream_t s);
+// The kernel of short rows and of few sources of the 8-byte fields (wide.cu) over
+// one call: `img` holds the single-row images (build_lut_images) of coefficient
+// (t, j) at (t * m + j).
+bool wide_chosen(int field, size_t k, size_t m, size_t len);
+// Stripes at least this long run there in batches too, a launch each; shorter ones
+// gain more from sharing the GPU. Two stripes of 8 MiB, k = 1, m = 3, table kernels
+// -> a launch each: 65.3 -> 39.2 us.
+constexpr size_t kWideStripe = 4u << 20;
+cudaError_t wide_launch(int field, const uint8_t* const* srcs, size_t k, uint8_t* const* rows, size_t m,
+                        const uint32_t* img, size_t len, bool overwrite, cudaStream_t stream);
 // One descriptor of a batched submission: a byte-table sub-job (batch.cu) or a
 // table sub-job (lut_batch.cuh).
 struct BatchJob {
