@@ -368,7 +368,10 @@ struct BatchClass {
   LutBatchKernel kern;
   size_t kc = 0;               // sources per fill
   std::vector<uint32_t> jobs;  // sub-job indices, plan order
-  std::vector<uint2> items;
+  std::vector<uint2> items;    // byte-table class: heads and tails
+  size_t nitems = 0;
+  uint32_t each = 0;           // table class: items of every job, if they are equal
+  size_t list_bytes() const { return each ? jobs.size() * sizeof(uint32_t) : nitems * sizeof(uint2); }
   std::vector<size_t> cuts;    // first item of each launch after the first
   std::vector<uint32_t> seg_jobs;   // byte-table class with own plans: sub-jobs with vectors, plan order
   std::vector<uint64_t> seg_prefix; // and the prefix of their vector counts (the segmented launch)
@@ -509,6 +512,9 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   std::vector<BatchDesc> dj(jobs.size());
   std::vector<JobAlign> al(jobs.size());
   std::vector<uint64_t> ptrs;
+  size_t nptr = 0;
+  for (const LoweredJob& L : jobs) nptr += L.k + L.nrows;
+  ptrs.reserve(nptr);
   std::vector<std::pair<uint32_t, uint32_t>> idx(jobs.size());  // first source and row pointer
   for (size_t i = 0; i < jobs.size(); ++i) {
     const LoweredJob& L = jobs[i];
@@ -520,7 +526,8 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   }
   std::vector<size_t> order(jobs.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t c) { return jobs[a].img < jobs[c].img; });
+  const auto before = [&](size_t a, size_t c) { return jobs[a].img < jobs[c].img; };
+  if (!std::is_sorted(order.begin(), order.end(), before)) std::stable_sort(order.begin(), order.end(), before);
   // Byte-table classes (a source count K) with fewer columns than this run the
   // table kernels instead, together with the other 1-byte sub-jobs: a 1024-thread
   // CTA with 227 KiB of tables waits for a whole SM to drain, which a mixed
@@ -539,13 +546,22 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     const LutShape shape = lut_shape(E, L.nrows, L.k);
     const int key = fast ? 1000 + 2 * static_cast<int>(L.k) + al[i].unal
                          : ((E * 4 + shape.lev) * 8 + shape.w) * 3 + al[i].mode;
-    BatchClass& c = classes[key];
-    c.E = E;
+    const auto at = classes.try_emplace(key);
+    BatchClass& c = at.first->second;
+    if (at.second) {  // what its jobs share
+      c.E = E;
+      if (fast) {
+        c.shift = al[i].unal;
+        c.K = static_cast<int>(L.k);
+      } else {
+        c.shape = shape;
+        c.kern = lut_batch_kernel_for(E, shape, al[i].mode);
+        c.kc = lut_sources(shape, false);
+      }
+    }
     c.jobs.push_back(static_cast<uint32_t>(i));
     BatchDesc& D = dj[i];
     if (fast) {
-      c.shift = al[i].unal;
-      c.K = static_cast<int>(L.k);
       BatchJob& J = D.byte;
       J.tables = L.byte_tab;
       J.len = L.len;
@@ -558,9 +574,6 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       J.dst_idx = idx[i].second;
       J.nv_items = 0;
     } else {
-      c.shape = shape;
-      c.kern = lut_batch_kernel_for(E, shape, al[i].mode);
-      c.kc = lut_sources(shape, false);
       D.lut = lut_batch_job(L.field, L.img, al[i], L.len, L.k, L.nrows, L.ovr);
       D.lut.src_idx = idx[i].first;
       D.lut.dst_idx = idx[i].second;
@@ -587,7 +600,8 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         return tile[G];
       };
       const int mode = kv.first % 3;
-      std::stable_sort(c.jobs.begin(), c.jobs.end(), [&](uint32_t p, uint32_t q) { return jobs[p].k > jobs[q].k; });
+      const auto more = [&](uint32_t p, uint32_t q) { return jobs[p].k > jobs[q].k; };
+      if (!std::is_sorted(c.jobs.begin(), c.jobs.end(), more)) std::stable_sort(c.jobs.begin(), c.jobs.end(), more);
       uint64_t total = 0;  // tiles times sources
       for (uint32_t i : c.jobs) total += lut_tiles(dj[i].lut.g, mode, kLutThreads) * jobs[i].k;
       c.cost = static_cast<double>(total) * c.shape.nv * c.shape.w * (16 / c.E);
@@ -599,12 +613,13 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       for (uint32_t i : c.jobs) one_plan = one_plan && jobs[i].byte_tab == jobs[c.jobs[0]].byte_tab;
       for (size_t q = 0; q < c.jobs.size(); ++q) {
         const uint32_t i = c.jobs[q];
-        if (one_plan && q && q % kUniformJobs == 0) c.cuts.push_back(c.items.size());
+        if (one_plan && q && q % kUniformJobs == 0) c.cuts.push_back(c.nitems);
         LutBatchJob& J = dj[i].lut;
         const uint64_t per = std::max<uint64_t>(1, std::min<uint64_t>(job_tile(i), total / (slots * jobs[i].k)));
         J.parts = static_cast<uint32_t>((lut_tiles(J.g, mode, kLutThreads) + per - 1) / per);
         const uint32_t n = J.parts + (lut_has_edges(J.g, mode) ? 1u : 0u);
-        for (uint32_t p = 0; p < n; ++p) c.items.push_back(make_uint2(i, p));
+        c.nitems += n;
+        c.each = q == 0 || n == c.each ? n : 0;
       }
       continue;
     }
@@ -626,6 +641,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       for (uint64_t p = J.nv_items; p < J.nv_items + ns_items; ++p)
         c.items.push_back(make_uint2(i, static_cast<unsigned>(p)));
     }
+    c.nitems = c.items.size();
   }
 
   // ---- blob: jobs | ptrs | per work-list class: items, counter
@@ -640,7 +656,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     std::pair<size_t, size_t> x{0, 0}, y{0, 0};
     if (!kv.second.uniform) {
       x.first = off;
-      off = align16(off + kv.second.items.size() * sizeof(uint2));
+      off = align16(off + kv.second.list_bytes());
       x.second = off;
       off = align16(off + std::max<size_t>(64, 4 * (kv.second.cuts.size() + 1)));
       if (!kv.second.seg_jobs.empty()) {
@@ -703,7 +719,18 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       const auto& y = sb[ci];
       const auto& x = cb[ci++];
       if (kv.second.uniform) continue;
-      std::memcpy(s.host + x.first, kv.second.items.data(), kv.second.items.size() * sizeof(uint2));
+      uint2* at = reinterpret_cast<uint2*>(s.host + x.first);
+      if (kv.second.K) {
+        std::memcpy(at, kv.second.items.data(), kv.second.list_bytes());
+      } else if (kv.second.each) {
+        std::memcpy(at, kv.second.jobs.data(), kv.second.list_bytes());
+      } else {
+        for (uint32_t i : kv.second.jobs) {
+          const LutBatchJob& J = dj[i].lut;
+          const uint32_t n = J.parts + (lut_has_edges(J.g, kv.first % 3) ? 1u : 0u);
+          for (uint32_t p = 0; p < n; ++p) *at++ = make_uint2(i, p);
+        }
+      }
       std::memset(s.host + x.second, 0, std::max<size_t>(64, 4 * (kv.second.cuts.size() + 1)));
       if (!kv.second.seg_jobs.empty()) {
         std::memcpy(s.host + y.first, kv.second.seg_jobs.data(), kv.second.seg_jobs.size() * sizeof(uint32_t));
@@ -734,7 +761,8 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     UniformFn ufn = nullptr;
     unsigned grid = 0, threads = 0;
     uint32_t smem = 0;
-    const uint2* items = nullptr;
+    const void* items = nullptr;
+    uint32_t each = 0;
     uint32_t n = 0;
     uint32_t* counter = nullptr;
     size_t uparam = 0;
@@ -773,8 +801,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       L.smem = fast_smem(c.K);
       L.threads = static_cast<unsigned>(kFastThreads);
     } else {
-      for (uint32_t i : c.jobs)
-        L.smem = std::max(L.smem, lut_smem(c.shape, std::min<size_t>(jobs[i].k, c.kc)));
+      L.smem = lut_smem(c.shape, std::min<size_t>(jobs[c.jobs[0]].k, c.kc));  // jobs with the most sources first
       L.threads = static_cast<unsigned>(kLutThreads);
       L.kc = static_cast<uint32_t>(c.kc);
     }
@@ -839,19 +866,20 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         S.key = "|s" + std::to_string(akey) + "," + std::to_string(S.n) + "," + std::to_string(S.grid);
         launches.push_back(S);
       }
-      if (!c.items.empty()) {
+      if (c.nitems) {
         for (size_t q = 0; q <= c.cuts.size(); ++q) {
-          const size_t i0 = q ? c.cuts[q - 1] : 0, i1 = q < c.cuts.size() ? c.cuts[q] : c.items.size();
+          const size_t i0 = q ? c.cuts[q - 1] : 0, i1 = q < c.cuts.size() ? c.cuts[q] : c.nitems;
           L.n = static_cast<uint32_t>(i1 - i0);
           L.grid = L.lfn ? static_cast<unsigned>(std::min<uint64_t>(L.n, static_cast<uint64_t>(sms) * c.kern.ctas))
                          : static_cast<unsigned>(std::min<uint64_t>((L.n + kClaim - 1) / kClaim, sms));
-          L.items = reinterpret_cast<const uint2*>(s.dev + x.first) + i0;
+          L.each = c.each;
+          L.items = s.dev + x.first + (c.each ? i0 / c.each * sizeof(uint32_t) : i0 * sizeof(uint2));
           L.counter = reinterpret_cast<uint32_t*>(s.dev + x.second) + q;
-          L.key = "|" + std::to_string(akey) + "," + std::to_string(L.n) + "," + std::to_string(L.grid) + "," +
-                 std::to_string(L.smem);
+          L.key = "|" + std::to_string(akey) + "," + std::to_string(L.n) + "," + std::to_string(L.each) + "," +
+                 std::to_string(L.grid) + "," + std::to_string(L.smem);
           launches.push_back(L);
         }
-        b->last_items += c.items.size();
+        b->last_items += c.nitems;
       }
     }
   }
@@ -929,10 +957,10 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
         L.sfn<<<L.grid, L.threads, L.smem, ls>>>(djobs, dptrs, L.seg_jobs, L.seg_prefix, L.n);
         err = cudaGetLastError();
       } else if (L.lfn) {
-        L.lfn<<<L.grid, L.threads, L.smem, ls>>>(djobs, dptrs, L.items, L.n, L.counter, L.kc);
+        L.lfn<<<L.grid, L.threads, L.smem, ls>>>(djobs, dptrs, L.items, L.each, L.n, L.counter, L.kc);
         err = cudaGetLastError();
       } else {
-        L.fn<<<L.grid, L.threads, L.smem, ls>>>(djobs, dptrs, L.items, L.n, L.counter);
+        L.fn<<<L.grid, L.threads, L.smem, ls>>>(djobs, dptrs, static_cast<const uint2*>(L.items), L.n, L.counter);
         err = cudaGetLastError();
       }
       if (err != cudaSuccess) return err;
@@ -1213,7 +1241,7 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
             descs, ptrs, list, static_cast<uint32_t>(n), counter);
       else
         lut.fn<<<static_cast<unsigned>(std::min<uint64_t>(n, sms * lut.ctas)), kLutThreads, smem, stream>>>(
-            descs, ptrs, list, static_cast<uint32_t>(n), counter,
+            descs, ptrs, list, 0u, static_cast<uint32_t>(n), counter,
             static_cast<uint32_t>(lut_sources(noalloc_shape(E, class_rows[c]), false)));
       e = cudaGetLastError();
     }

@@ -164,7 +164,7 @@ union BatchDesc {
   LutBatchJob lut;
 };
 static_assert(sizeof(BatchDesc) == 64, "the no-allocation scratch limit counts 64 bytes per stripe");
-using LutBatchFn = void (*)(const BatchDesc*, const uint64_t*, const uint2*, uint32_t, uint32_t*, uint32_t);
+using LutBatchFn = void (*)(const BatchDesc*, const uint64_t*, const void*, uint32_t, uint32_t, uint32_t*, uint32_t);
 struct LutBatchKernel {
   LutBatchFn fn = nullptr;
   int ctas = 1;  // resident per SM

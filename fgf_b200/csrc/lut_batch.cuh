@@ -5,7 +5,8 @@
 
 namespace fgfc {
 
-// Persistent CTAs claim items (job, part) from a counter; part p of a job's
+// Persistent CTAs claim items (job, part) from a counter: entries of a list, or,
+// where every job has `each` parts, positions in a list of jobs. Part p of a job's
 // `parts` takes its tiles p, p + parts, ..., part `parts` its edges. The next
 // item is claimed before the current one is worked on, and the tables are
 // refilled (a few KiB) only where the plan changes. Sources past kc (one fill's
@@ -13,7 +14,7 @@ namespace fgfc {
 template <int E, int LEV, int W, int MODE>
 __global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, MODE>())
     lut_batch_kernel(const BatchDesc* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
-                     const uint2* __restrict__ items, uint32_t nitems, uint32_t* counter, uint32_t kc) {
+                     const void* __restrict__ items, uint32_t each, uint32_t nitems, uint32_t* counter, uint32_t kc) {
   using L = Lut<E, LEV>;
   using S = LutSmem<L::NV, W>;
   __shared__ LutShared sh;
@@ -28,7 +29,11 @@ __global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, MODE>())
     const uint32_t it = s_item;
     if (it >= nitems) break;
     if (threadIdx.x == 0) next = atomicAdd(counter, 1u);
-    const uint2 wi = items[it];
+    uint2 wi;
+    if (each)
+      wi = make_uint2(static_cast<const uint32_t*>(items)[it / each], it % each);
+    else
+      wi = static_cast<const uint2*>(items)[it];
     const LutBatchJob* jp = &jobs[wi.x].lut;
     const uint32_t k = jp->g.k;
     for (uint32_t t0 = 0; t0 < k; t0 += kc) {

@@ -13,7 +13,9 @@ from fgf_b200.fields import Gf16, Gf32
 
 pytestmark = pytest.mark.gpu
 
-K, ROW = 2, 4 << 20  # long enough that the built-in split takes several columns per thread
+# Three sources (one or two go without a split, a class per group count), long
+# enough that the built-in split takes several columns per thread.
+K, ROW = 3, 4 << 20
 
 
 @pytest.fixture(autouse=True)
