@@ -532,17 +532,28 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // table kernels instead, together with the other 1-byte sub-jobs: a 1024-thread
   // CTA with 227 KiB of tables waits for a whole SM to drain, which a mixed
   // submission's dozens of small classes did one after the other (256 mixed
-  // stripes, with the order of items and launches below: 1505 -> 1463 us). One call crosses over between 4 MiB rows (K =
-  // 10: 17.3 us by table kernel, 19.1 by byte tables) and 16 MiB (54.7, 47.7).
+  // stripes, with the order of items and launches below: 1505 -> 1463 us). One call
+  // crosses over between 4 MiB rows (K = 10: 17.3 us by table kernel, 19.1 by byte
+  // tables) and 16 MiB (54.7, 47.7). A class that is alone, a plan per stripe and
+  // rows at the sources' offset, has nothing to wait for: up to 10 sources the byte
+  // tables are not slower at any size (32 stripes in 4 MiB of row length, 4 rows,
+  // table kernels / byte tables alone, us: K = 2 30.0 / 27.6, K = 6 38.3 / 35.0, K =
+  // 10 40.8 / 37.2, K = 14 45.1 / 46.3).
   constexpr uint64_t kByteClassCols = 8u << 16;
   std::map<size_t, uint64_t> byte_cols;
   for (size_t i = 0; i < jobs.size(); ++i)
     if (jobs[i].byte_tab && al[i].sources) byte_cols[jobs[i].k] += jobs[i].len / 16;
+  bool lone = tc.empty() && !jobs.empty() && jobs[0].k <= 10, own_plans = false;
+  for (size_t i = 0; i < jobs.size() && lone; ++i) {
+    lone = jobs[i].byte_tab && !al[i].unal && jobs[i].k == jobs[0].k;
+    own_plans = own_plans || jobs[i].byte_tab != jobs[0].byte_tab;
+  }
+  lone = lone && own_plans;
   std::map<int, BatchClass> classes;
   for (size_t i : order) {
     const LoweredJob& L = jobs[i];
     const int E = field_bytes(L.field);
-    const bool fast = L.byte_tab && al[i].sources && byte_cols[L.k] >= kByteClassCols;
+    const bool fast = L.byte_tab && al[i].sources && (lone || byte_cols[L.k] >= kByteClassCols);
     const LutShape shape = lut_shape(E, L.nrows, L.k);
     const int key = fast ? 1000 + 2 * static_cast<int>(L.k) + al[i].unal
                          : ((E * 4 + shape.lev) * 8 + shape.w) * 3 + al[i].mode;

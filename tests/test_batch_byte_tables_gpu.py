@@ -109,3 +109,34 @@ def test_more_stripes_than_one_parameter_block(cuda, shifted):
             want ^= products[t * m + j][host[:, t, :n]]
         bad = np.nonzero((got[:, j] != want).any(axis=1))[0]
         assert bad.size == 0, (j, bad[:8])
+
+
+@pytest.mark.parametrize("k,lone", [(3, True), (10, True), (11, False), (10, False)])
+def test_short_stripes_of_own_plans(cuda, k, lone):
+    """A class far below the threshold runs the byte tables where it is the
+    submission's only one (up to 10 sources, rows at the sources' offset)."""
+    m, n = 4, 4096 + 48
+    rng = np.random.default_rng(k + lone)
+    jobs, checks = [], []
+    for i in range(5):
+        coeffs = [int(c) for c in rng.integers(0, 256, size=k * m)]
+        plan = ops.Plan.matrix(Gf8D, k, m, coeffs)
+        srcs, dst, srcs_h, want, starts = _stripe(rng, k, m, n, 0, False)
+        jobs.append(fb.Job(plan, srcs, dst, n, m, True, starts))
+        products = _products(Gf8D, coeffs)
+        for j, s in enumerate(starts):
+            want[s:s + n] = 0
+            for t in range(k):
+                want[s:s + n] ^= products[t * m + j][srcs_h[t]]
+        checks.append((dst, want))
+    if k == 10 and not lone:  # another number of sources beside them
+        srcs, dst, srcs_h, want, starts = _stripe(rng, 2, 1, n, 0, False)
+        jobs.append(fb.Job(ops.Plan.matrix(Gf8D, 2, 1, [1, 1]), srcs, dst, n, 1, True, starts))
+        want[starts[0]:starts[0] + n] = srcs_h[0] ^ srcs_h[1]
+        checks.append((dst, want))
+    runner = fb.Batch()
+    runner.run(jobs)
+    torch.cuda.synchronize()
+    for i, (dst, want) in enumerate(checks):
+        assert np.array_equal(dst.cpu().numpy(), want), i
+    assert (runner.stats()["items"] == len(jobs)) == lone  # the table kernels take two tiles of a stripe
