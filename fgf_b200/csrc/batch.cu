@@ -925,19 +925,29 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
     if (e != cudaSuccess) return e;
   }
-  // The blob goes up on the stream that records graphs, under whatever the caller's stream
-  // still runs (the slot is free: its last submission finished), and the
-  // caller's stream waits for it: in line the copy and the gaps around it cost
-  // 10 us between two submissions (64 stripes of 1 MiB shards, RS(10,4): encode
-  // 192.5 -> 186.9 us, rebuild 203.5 -> 199.9). Launches that carry everything in
+  // The blob of a submission that the GPU takes longer on than the host goes up on
+  // the stream that records graphs, under whatever the caller's stream still runs
+  // (the slot is free: its last submission finished), and the caller's stream waits
+  // for it: as a node of the graph the copy and the gaps around it cost 10 us
+  // between two submissions (64 stripes of 1 MiB shards, RS(10,4): encode 192.5 ->
+  // 186.9 us, rebuild 203.5 -> 199.9). The host pays 5 us for it, so the others keep
+  // the node: per submission, one after another, beside / node, us: 100 Gf16 stripes
+  // of 2 x 2 rows of 4 KiB 33.8 / 27.2, Gf16 (10,4) of 16 KiB 30.6 / 31.4 and 64 / 55
+  // alone, 32 Gf8D (10,4) of 64 KiB 17.5 / 25.9. The line is where 8 us and 0.2 us a
+  // stripe pass the time of the bytes at 1.8 TB/s. Launches that carry everything in
   // their parameters need no blob.
   bool blob = false;
   for (const Launch& L : launches) blob = blob || !L.ufn;
+  uint64_t moved = 0;
+  for (const LoweredJob& L : jobs) moved += L.len * (L.k + L.nrows);
+  for (const Gf2Job& J : tc) moved += J.nblk * 512u * static_cast<uint64_t>(field_bytes(J.field)) * (J.k + J.m);
+  const bool beside = moved >= (8u << 20) + (384u << 10) * static_cast<uint64_t>(jobs.size());
+  if (!beside) key += "|copy";
   if (!b->capture) {
     e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking);
     if (e != cudaSuccess) return e;
   }
-  if (blob) {
+  if (blob && beside) {
     e = cudaMemcpyAsync(s.dev, s.host, bytes, cudaMemcpyHostToDevice, b->capture);
     if (e == cudaSuccess) e = cudaEventRecord(s.up, b->capture);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, s.up, 0);
@@ -947,6 +957,8 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // i % kSideStreams) and join back
   auto enqueue = [&](cudaStream_t st) -> cudaError_t {
     cudaError_t err = cudaSuccess;
+    if (blob && !beside) err = cudaMemcpyAsync(s.dev, s.host, bytes, cudaMemcpyHostToDevice, st);
+    if (err != cudaSuccess) return err;
     if (nside) {
       err = cudaEventRecord(b->fork, st);
       for (int i = 0; i < nside && err == cudaSuccess; ++i) err = cudaStreamWaitEvent(b->side[i], b->fork, 0);
