@@ -31,14 +31,20 @@ const Fp8Log& fp8_tab() {
 }
 
 void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t k, uint32_t* out) {
-  for (size_t t = 0; t < k; ++t)
-    for (int half = 0; half < 2; ++half)
-      for (uint32_t n = 0; n < 16; ++n) {
-        uint32_t word = 0;
-        for (size_t j = 0; j < m; ++j)
-          word |= static_cast<uint32_t>(gf_mul(field, coeffs[t * m + j] & 0xFF, half ? n << 4 : n)) << (8 * j);
-        out[t * kCompactWords + half * 16 + n] = word;
+  for (size_t t = 0; t < k; ++t) {
+    uint32_t bit[8] = {0};  // products by each input bit, byte j of row j
+    for (size_t j = 0; j < m; ++j)
+      for (int b = 0; b < 8; ++b)
+        bit[b] |= static_cast<uint32_t>(gf_mul(field, coeffs[t * m + j] & 0xFF, 1u << b)) << (8 * j);
+    uint32_t* w = out + t * kCompactWords;
+    for (int half = 0; half < 2; ++half, w += 16) {
+      w[0] = 0;
+      for (uint32_t n = 1; n < 16; ++n) {  // the lowest set bit and the rest
+        const int low = n & 1 ? 0 : n & 2 ? 1 : n & 4 ? 2 : 3;
+        w[n] = w[n & (n - 1)] ^ bit[4 * half + low];
       }
+    }
+  }
 }
 
 // Tower levels split per launch. A leaf product's table word holds the H-byte
@@ -98,34 +104,34 @@ int leaf_field(int field, int H) {
 
 }  // namespace
 
-void build_lut_images(int field, const LutShape& s, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t r0,
+void build_lut_images(int field, const LutShape& shape, const uint64_t* coeffs, size_t m, size_t t0, size_t k, size_t r0,
                       size_t nr, uint32_t* out) {
-  const int E = field_bytes(field);
-  const int H = E >> s.lev, leaf = leaf_field(field, H);
-  const size_t W = static_cast<size_t>(s.w);
-  std::memset(out, 0, k * s.src_words() * sizeof(uint32_t));
+  const int E = field_bytes(field), lev = shape.lev;
+  const int H = E >> lev, leaf = leaf_field(field, H);
+  const size_t W = static_cast<size_t>(shape.w), nv = shape.nv;
+  std::memset(out, 0, k * shape.src_words() * sizeof(uint32_t));
   for (size_t t = 0; t < k; ++t)
     for (size_t r = 0; r < nr; ++r) {
-      uint64_t c[27] = {coeffs[(t0 + t) * m + r0 + r] & field_mask(field)};
-      size_t n = 1;
-      for (int w = E / 2; w >= H; w /= 2) {  // split every product: low half, high half, their sum
-        for (size_t i = n; i-- > 0;) {
-          const uint64_t v = c[i], lo = v & ((1ull << (8 * w)) - 1), hi = v >> (8 * w);
-          c[3 * i] = lo;
-          c[3 * i + 1] = hi;
-          c[3 * i + 2] = lo ^ hi;
-        }
-        n *= 3;
+      // v[P][i]: product P by bit i. The element's leaves are multiplied; the
+      // products of sums of leaves are sums of theirs.
+      uint32_t v[27][32];
+      const uint64_t c = coeffs[(t0 + t) * m + r0 + r] & field_mask(field);
+      int at[8], n = 1 << lev;  // where each leaf's product stands in tree order
+      for (int l = 0; l < n; ++l) {
+        at[l] = 0;
+        for (int d = lev; d-- > 0;) at[l] = 3 * at[l] + (l >> d & 1);
+        for (int i = 0; i < 8 * H; ++i)
+          v[at[l]][i] = static_cast<uint32_t>(gf_mul(leaf, c >> (8 * H * l) & field_mask(leaf), 1ull << i));
       }
-      for (size_t P = 0; P < n; ++P)
-        for (int p = 0; p < H; ++p)
-          for (int b = 0; b < 8; ++b) {
-            const uint64_t v = gf_mul(leaf, c[P], 1ull << (8 * p + b));
-            for (int o = 0; o < H; ++o) {
-              const size_t f = r * H + o;  // output byte: word f / 4
-              out[((t * s.nv + P * H + p) * W + f / 4) * 8 + b] |= static_cast<uint32_t>((v >> (8 * o)) & 0xFF)
-                                                                  << (8 * (f % 4));
-            }
+      for (int sub = 1; sub < static_cast<int>(nv) / H; sub *= 3)  // products below a split: low, high, their sum
+        for (int P = 0; P < static_cast<int>(nv) / H; ++P)
+          if (P / sub % 3 == 2)
+            for (int i = 0; i < 8 * H; ++i) v[P][i] = v[P - 2 * sub][i] ^ v[P - sub][i];
+      for (size_t P = 0; P < nv / H; ++P)
+        for (int i = 0; i < 8 * H; ++i)
+          for (int o = 0; o < H; ++o) {
+            const size_t f = r * H + o;  // output byte: word f / 4
+            out[((t * nv + P * H + i / 8) * W + f / 4) * 8 + i % 8] |= (v[P][i] >> (8 * o) & 0xFFu) << (8 * (f % 4));
           }
     }
 }
