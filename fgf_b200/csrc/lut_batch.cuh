@@ -21,14 +21,13 @@ __global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, MODE>())
   __shared__ LutBatchJob s_job;
   __shared__ uint32_t s_item;
   const uint32_t* resident = nullptr;
-  uint32_t next = 0;
-  if (threadIdx.x == 0) next = atomicAdd(counter, 1u);
+  uint32_t next = blockIdx.x;
   for (;;) {
     if (threadIdx.x == 0) s_item = next;
     __syncthreads();
     const uint32_t it = s_item;
     if (it >= nitems) break;
-    if (threadIdx.x == 0) next = atomicAdd(counter, 1u);
+    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(counter, 1u);
     uint2 wi;
     if (each)
       wi = make_uint2(static_cast<const uint32_t*>(items)[it / each], it % each);
