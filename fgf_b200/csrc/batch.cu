@@ -536,10 +536,10 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // crosses over between 4 MiB rows (K = 10: 17.3 us by table kernel, 19.1 by byte
   // tables) and 16 MiB (54.7, 47.7). A class that is alone, a plan per stripe and
   // rows at the sources' offset, has nothing to wait for: up to 10 sources the byte
-  // tables are not slower at any size (32 stripes in 4 MiB of row length, 4 rows,
-  // table kernels / byte tables alone, us: K = 2 30.0 / 27.6, K = 6 38.3 / 35.0, K =
-  // 10 40.8 / 37.2, K = 14 45.1 / 46.3).
-  constexpr uint64_t kByteClassCols = 8u << 16;
+  // tables win from about 1 MiB of row length on (32 stripes, 4 rows, waited for,
+  // table kernels / byte tables, us: 4 MiB of K = 2 30.0 / 27.6, K = 6 38.3 / 35.0, K =
+  // 10 40.8 / 37.2, K = 14 45.1 / 46.3; 8 stripes of 4 KiB, K = 4, 20.1 / 29.1).
+  constexpr uint64_t kByteClassCols = 8u << 16, kLoneClassCols = 1u << 16;
   std::map<size_t, uint64_t> byte_cols;
   for (size_t i = 0; i < jobs.size(); ++i)
     if (jobs[i].byte_tab && al[i].sources) byte_cols[jobs[i].k] += jobs[i].len / 16;
@@ -548,7 +548,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
     lone = jobs[i].byte_tab && !al[i].unal && jobs[i].k == jobs[0].k;
     own_plans = own_plans || jobs[i].byte_tab != jobs[0].byte_tab;
   }
-  lone = lone && own_plans;
+  lone = lone && own_plans && byte_cols[jobs[0].k] >= kLoneClassCols;
   std::map<int, BatchClass> classes;
   for (size_t i : order) {
     const LoweredJob& L = jobs[i];
@@ -933,15 +933,16 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // 186.9 us, rebuild 203.5 -> 199.9). The host pays 5 us for it, so the others keep
   // the node: per submission, one after another, beside / node, us: 100 Gf16 stripes
   // of 2 x 2 rows of 4 KiB 33.8 / 27.2, Gf16 (10,4) of 16 KiB 30.6 / 31.4 and 64 / 55
-  // alone, 32 Gf8D (10,4) of 64 KiB 17.5 / 25.9. The line is where 8 us and 0.2 us a
-  // stripe pass the time of the bytes at 1.8 TB/s. Launches that carry everything in
+  // alone, 32 Gf8D (10,4) of 64 KiB 17.5 / 25.9, 7 Gf8B (11,3) of 44 KiB 12.3 / 16.9.
+  // The line is where 8 us and 0.2 us a sub-job pass 13 us and the time of the bytes
+  // at 1.8 TB/s. Launches that carry everything in
   // their parameters need no blob.
   bool blob = false;
   for (const Launch& L : launches) blob = blob || !L.ufn;
   uint64_t moved = 0;
   for (const LoweredJob& L : jobs) moved += L.len * (L.k + L.nrows);
   for (const Gf2Job& J : tc) moved += J.nblk * 512u * static_cast<uint64_t>(field_bytes(J.field)) * (J.k + J.m);
-  const bool beside = moved >= (8u << 20) + (384u << 10) * static_cast<uint64_t>(jobs.size());
+  const bool beside = jobs.size() <= 25 || moved >= (360u << 10) * static_cast<uint64_t>(jobs.size() - 25);
   if (!beside) key += "|copy";
   if (!b->capture) {
     e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking);

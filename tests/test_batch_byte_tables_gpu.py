@@ -111,11 +111,13 @@ def test_more_stripes_than_one_parameter_block(cuda, shifted):
         assert bad.size == 0, (j, bad[:8])
 
 
-@pytest.mark.parametrize("k,lone", [(3, True), (10, True), (11, False), (10, False)])
-def test_short_stripes_of_own_plans(cuda, k, lone):
-    """A class far below the threshold runs the byte tables where it is the
-    submission's only one (up to 10 sources, rows at the sources' offset)."""
-    m, n = 4, 4096 + 48
+@pytest.mark.parametrize("k,columns,lone", [(3, 13108, True), (10, 13108, True), (11, 13108, False), (10, 13108, False),
+                                            (10, 13107, False)])
+def test_short_stripes_of_own_plans(cuda, k, columns, lone):
+    """A class far below the threshold, of at least 65536 columns, runs the byte
+    tables where it is the submission's only one (up to 10 sources, rows at the
+    sources' offset)."""
+    m, n = 4, 16 * columns
     rng = np.random.default_rng(k + lone)
     jobs, checks = [], []
     for i in range(5):
@@ -129,7 +131,7 @@ def test_short_stripes_of_own_plans(cuda, k, lone):
             for t in range(k):
                 want[s:s + n] ^= products[t * m + j][srcs_h[t]]
         checks.append((dst, want))
-    if k == 10 and not lone:  # another number of sources beside them
+    if (k, columns, lone) == (10, 13108, False):  # another number of sources beside them
         srcs, dst, srcs_h, want, starts = _stripe(rng, 2, 1, n, 0, False)
         jobs.append(fb.Job(ops.Plan.matrix(Gf8D, 2, 1, [1, 1]), srcs, dst, n, 1, True, starts))
         want[starts[0]:starts[0] + n] = srcs_h[0] ^ srcs_h[1]
@@ -139,4 +141,4 @@ def test_short_stripes_of_own_plans(cuda, k, lone):
     torch.cuda.synchronize()
     for i, (dst, want) in enumerate(checks):
         assert np.array_equal(dst.cpu().numpy(), want), i
-    assert (runner.stats()["items"] == len(jobs)) == lone  # the table kernels take two tiles of a stripe
+    assert (runner.stats()["items"] == len(jobs)) == lone  # the table kernels take many items of a stripe
