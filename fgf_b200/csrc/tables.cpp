@@ -30,12 +30,27 @@ const Fp8Log& fp8_tab() {
   return t;
 }
 
+namespace {
+
+// Logarithm tables of a field of bytes.
+struct ByteLogs {
+  const uint8_t *exp, *log;
+};
+ByteLogs byte_logs(int field) {
+  if (field == kFp8) return {fp8_tab().exp, fp8_tab().log};
+  const Gf8Log& t = field == kGf8D ? gf8d_tab() : gf8b_tab();
+  return {t.exp, t.log};
+}
+
+}  // namespace
+
 void build_compact_tables(int field, const uint64_t* coeffs, size_t m, size_t k, uint32_t* out) {
+  const ByteLogs logs = byte_logs(field);
   for (size_t t = 0; t < k; ++t) {
     uint32_t bit[8] = {0};  // products by each input bit, byte j of row j
     for (size_t j = 0; j < m; ++j)
-      for (int b = 0; b < 8; ++b)
-        bit[b] |= static_cast<uint32_t>(gf_mul(field, coeffs[t * m + j] & 0xFF, 1u << b)) << (8 * j);
+      if (const uint8_t c = static_cast<uint8_t>(coeffs[t * m + j]))
+        for (int b = 0; b < 8; ++b) bit[b] |= static_cast<uint32_t>(logs.exp[logs.log[c] + logs.log[1 << b]]) << (8 * j);
     uint32_t* w = out + t * kCompactWords;
     for (int half = 0; half < 2; ++half, w += 16) {
       w[0] = 0;
@@ -108,11 +123,15 @@ void build_lut_images(int field, const LutShape& shape, const uint64_t* coeffs, 
                       size_t nr, uint32_t* out) {
   const int E = field_bytes(field), lev = shape.lev;
   const int H = E >> lev, leaf = leaf_field(field, H);
+  const ByteLogs byte = byte_logs(leaf_field(field, 1));
+  int two[8];  // logarithms of a byte's bits
+  for (int b = 0; b < 8; ++b) two[b] = byte.log[1 << b];
   const size_t W = static_cast<size_t>(shape.w), nv = shape.nv;
   std::memset(out, 0, k * shape.src_words() * sizeof(uint32_t));
   for (size_t t = 0; t < k; ++t)
     for (size_t r = 0; r < nr; ++r) {
-      // v[P][i]: product P by bit i. The element's leaves are multiplied; the
+      // v[P][i]: product P by bit i. The element's leaves are multiplied by each
+      // byte's 1, bytes scale the others (the byte level is a subfield), and the
       // products of sums of leaves are sums of theirs.
       uint32_t v[27][32];
       const uint64_t c = coeffs[(t0 + t) * m + r0 + r] & field_mask(field);
@@ -120,8 +139,15 @@ void build_lut_images(int field, const LutShape& shape, const uint64_t* coeffs, 
       for (int l = 0; l < n; ++l) {
         at[l] = 0;
         for (int d = lev; d-- > 0;) at[l] = 3 * at[l] + (l >> d & 1);
-        for (int i = 0; i < 8 * H; ++i)
-          v[at[l]][i] = static_cast<uint32_t>(gf_mul(leaf, c >> (8 * H * l) & field_mask(leaf), 1ull << i));
+        const uint64_t cl = c >> (8 * H * l) & field_mask(leaf);
+        for (int p = 0; p < H; ++p) {
+          const uint64_t one = p ? gf_mul(leaf, cl, 1ull << (8 * p)) : cl;
+          uint32_t* x = v[at[l]] + 8 * p;
+          for (int b = 0; b < 8; ++b) x[b] = 0;
+          for (int o = 0; o < H; ++o)
+            if (const uint8_t a = static_cast<uint8_t>(one >> (8 * o)))
+              for (int b = 0; b < 8; ++b) x[b] |= static_cast<uint32_t>(byte.exp[byte.log[a] + two[b]]) << (8 * o);
+        }
       }
       for (int sub = 1; sub < static_cast<int>(nv) / H; sub *= 3)  // products below a split: low, high, their sum
         for (int P = 0; P < static_cast<int>(nv) / H; ++P)
