@@ -7,10 +7,12 @@ namespace fgfc {
 
 // Persistent CTAs claim items (job, part) from a counter: entries of a list, or,
 // where every job has `each` parts, positions in a list of jobs. Part p of a job's
-// `parts` takes its tiles p, p + parts, ..., part `parts` its edges. The next
-// item is claimed before the current one is worked on, and the tables are
-// refilled (a few KiB) only where the plan changes. Sources past kc (one fill's
-// limit) accumulate in further rounds over the same tiles.
+// `parts` takes its tiles p, p + parts, ..., part `parts` its edges. The next item is
+// claimed before the current one is worked on; where there is no more than one for
+// every CTA they are taken by number, or the CTAs that start first would have the
+// late ones' too (four Gf32 stripes of 1 MiB, (10,4), 64 items: 73 or 138 us). The
+// tables are refilled (a few KiB) only where the plan changes. Sources past kc (one
+// fill's limit) accumulate in further rounds over the same tiles.
 template <int E, int LEV, int W, int MODE>
 __global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, MODE>())
     lut_batch_kernel(const BatchDesc* __restrict__ jobs, const uint64_t* __restrict__ ptrs,
@@ -19,20 +21,23 @@ __global__ void __launch_bounds__(kLutThreads, lut_min_ctas<E, LEV, W, MODE>())
   using S = LutSmem<L::NV, W>;
   __shared__ LutShared sh;
   __shared__ LutBatchJob s_job;
-  __shared__ uint32_t s_item;
+  __shared__ uint2 s_item;
   const uint32_t* resident = nullptr;
+  const bool one_each = nitems <= gridDim.x;
   uint32_t next = blockIdx.x;
+  if (!one_each && threadIdx.x == 0) next = atomicAdd(counter, 1u);
   for (;;) {
-    if (threadIdx.x == 0) s_item = next;
+    if (threadIdx.x == 0) {
+      uint2 item = make_uint2(~0u, 0u);
+      if (next < nitems)
+        item = each ? make_uint2(static_cast<const uint32_t*>(items)[next / each], next % each)
+                    : static_cast<const uint2*>(items)[next];
+      s_item = item;
+    }
     __syncthreads();
-    const uint32_t it = s_item;
-    if (it >= nitems) break;
-    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(counter, 1u);
-    uint2 wi;
-    if (each)
-      wi = make_uint2(static_cast<const uint32_t*>(items)[it / each], it % each);
-    else
-      wi = static_cast<const uint2*>(items)[it];
+    const uint2 wi = s_item;
+    if (wi.x == ~0u) break;
+    if (threadIdx.x == 0) next = one_each ? nitems : atomicAdd(counter, 1u);
     const LutBatchJob* jp = &jobs[wi.x].lut;
     const uint32_t k = jp->g.k;
     for (uint32_t t0 = 0; t0 < k; t0 += kc) {
