@@ -536,10 +536,11 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // crosses over between 4 MiB rows (K = 10: 17.3 us by table kernel, 19.1 by byte
   // tables) and 16 MiB (54.7, 47.7). A class that is alone, a plan per stripe and
   // rows at the sources' offset, has nothing to wait for: up to 10 sources the byte
-  // tables win from about 1 MiB of row length on (32 stripes, 4 rows, waited for,
+  // tables win from about 2 MiB of row length on (32 stripes, 4 rows, waited for,
   // table kernels / byte tables, us: 4 MiB of K = 2 30.0 / 27.6, K = 6 38.3 / 35.0, K =
-  // 10 40.8 / 37.2, K = 14 45.1 / 46.3; 8 stripes of 4 KiB, K = 4, 20.1 / 29.1).
-  constexpr uint64_t kByteClassCols = 8u << 16, kLoneClassCols = 1u << 16;
+  // 10 40.8 / 37.2, K = 14 45.1 / 46.3; 64 stripes of 16 KiB, K = 10, 37.1 / 41.3, 8
+  // of 4 KiB, K = 4, 20.1 / 29.1).
+  constexpr uint64_t kByteClassCols = 8u << 16, kLoneClassCols = 2u << 16;
   std::map<size_t, uint64_t> byte_cols;
   for (size_t i = 0; i < jobs.size(); ++i)
     if (jobs[i].byte_tab && al[i].sources) byte_cols[jobs[i].k] += jobs[i].len / 16;
@@ -940,9 +941,13 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   bool blob = false;
   for (const Launch& L : launches) blob = blob || !L.ufn;
   uint64_t moved = 0;
-  for (const LoweredJob& L : jobs) moved += L.len * (L.k + L.nrows);
+  bool wide = false;  // 8-byte fields: the GPU takes longer
+  for (const LoweredJob& L : jobs) {
+    moved += L.len * (L.k + L.nrows);
+    wide = wide || field_bytes(L.field) == 8;
+  }
   for (const Gf2Job& J : tc) moved += J.nblk * 512u * static_cast<uint64_t>(field_bytes(J.field)) * (J.k + J.m);
-  const bool beside = jobs.size() <= 25 || moved >= (360u << 10) * static_cast<uint64_t>(jobs.size() - 25);
+  const bool beside = wide || jobs.size() <= 25 || moved >= (360u << 10) * static_cast<uint64_t>(jobs.size() - 25);
   if (!beside) key += "|copy";
   if (!b->capture) {
     e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking);

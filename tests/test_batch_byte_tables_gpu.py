@@ -111,10 +111,10 @@ def test_more_stripes_than_one_parameter_block(cuda, shifted):
         assert bad.size == 0, (j, bad[:8])
 
 
-@pytest.mark.parametrize("k,columns,lone", [(3, 13108, True), (10, 13108, True), (11, 13108, False), (10, 13108, False),
-                                            (10, 13107, False)])
+@pytest.mark.parametrize("k,columns,lone", [(3, 26215, True), (10, 26215, True), (11, 26215, False), (10, 26215, False),
+                                            (10, 26214, False)])
 def test_short_stripes_of_own_plans(cuda, k, columns, lone):
-    """A class far below the threshold, of at least 65536 columns, runs the byte
+    """A class far below the threshold, of at least 131072 columns, runs the byte
     tables where it is the submission's only one (up to 10 sources, rows at the
     sources' offset)."""
     m, n = 4, 16 * columns
@@ -131,7 +131,7 @@ def test_short_stripes_of_own_plans(cuda, k, columns, lone):
             for t in range(k):
                 want[s:s + n] ^= products[t * m + j][srcs_h[t]]
         checks.append((dst, want))
-    if (k, columns, lone) == (10, 13108, False):  # another number of sources beside them
+    if (k, columns, lone) == (10, 26215, False):  # another number of sources beside them
         srcs, dst, srcs_h, want, starts = _stripe(rng, 2, 1, n, 0, False)
         jobs.append(fb.Job(ops.Plan.matrix(Gf8D, 2, 1, [1, 1]), srcs, dst, n, 1, True, starts))
         want[starts[0]:starts[0] + n] = srcs_h[0] ^ srcs_h[1]
