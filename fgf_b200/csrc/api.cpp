@@ -1121,7 +1121,7 @@ fgfc_status fgfc_batch_run(fgfc_batch* batch, const fgfc_matrix_job* jobs, size_
       dsts[j] = reinterpret_cast<uint64_t>(J.dst + (J.row_starts ? J.row_starts[j] : j * J.row_len));
     std::vector<uint64_t> srcs(J.nsrcs);
     for (size_t t = 0; t < J.nsrcs; ++t) srcs[t] = reinterpret_cast<uint64_t>(J.srcs[t].ptr);
-    if (J.row_len >= kWideStripe && wide_chosen(field, J.nsrcs, J.nrows, J.row_len)) {
+    if (wide_stripe(field, J.nsrcs, J.nrows, J.row_len)) {
       own.push_back(i);
       continue;
     }

@@ -134,10 +134,8 @@ cudaError_t lut_launch(int field, const LutShape& sh, LutArgs& a, int mode, cuda
 // one call: `img` holds the single-row images (build_lut_images) of coefficient
 // (t, j) at (t * m + j).
 bool wide_chosen(int field, size_t k, size_t m, size_t len);
-// Stripes at least this long run there in batches too, a launch each; shorter ones
-// gain more from sharing the GPU. Two stripes of 8 MiB, k = 1, m = 3, table kernels
-// -> a launch each: 65.3 -> 39.2 us.
-constexpr size_t kWideStripe = 4u << 20;
+// Does a batched stripe run there too, as a launch of its own?
+bool wide_stripe(int field, size_t k, size_t m, size_t len);
 cudaError_t wide_launch(int field, const uint8_t* const* srcs, size_t k, uint8_t* const* rows, size_t m,
                         const uint32_t* img, size_t len, bool overwrite, cudaStream_t stream);
 // One descriptor of a batched submission: a byte-table sub-job (batch.cu) or a

@@ -153,6 +153,16 @@ bool wide_chosen(int field, size_t k, size_t m, size_t len) {
   return k <= 2 && m >= 2;
 }
 
+// Long stripes of few sources gain more from this kernel than from sharing the
+// GPU. Table kernels' work list / a launch each, us: two of 8 MiB GF(2^64) k = 1, m
+// = 3 65 / 40, k = 2, m = 2 53 / 45, FP64 k = 1, m = 4 55 / 50, k = 2, m = 8 123 / 140;
+// four of 4 MiB GF(2^64) k = 1, m = 2 41 / 41, m = 3 65 / 50, k = 2, m = 4 82 / 94, FP64
+// k = 1, m = 4 55 / 60.
+bool wide_stripe(int field, size_t k, size_t m, size_t len) {
+  if (len < (4u << 20) || !wide_chosen(field, k, m, len)) return false;
+  return len >= (8u << 20) ? !(field == kFp64 && k == 2 && m > 4) : field == kGf64 && k == 1;
+}
+
 cudaError_t wide_launch(int field, const uint8_t* const* srcs, size_t k, uint8_t* const* rows, size_t m,
                         const uint32_t* img, size_t len, bool overwrite, cudaStream_t stream) {
   const uint64_t nelem = len / 8;

@@ -83,11 +83,11 @@ def test_scatter_and_gather(cuda, field):
 
 @pytest.mark.parametrize("field", WIDE, ids=lambda f: f.__name__)
 def test_long_stripes_in_a_batch(cuda, field):
-    """Stripes of few sources run as calls of their own from 4 MiB on; shorter and
-    wider ones beside them on the work list."""
+    """Long stripes of few sources run as calls of their own; shorter and wider ones
+    beside them on the work list."""
     rng = np.random.default_rng(field.ID + 5)
     jobs, checks = [], []
-    for k, m, n in ((1, 3, 4 << 20), (1, 3, (4 << 20) - 8), (3, 2, 8000), (2, 3, (4 << 20) + 8)):
+    for k, m, n in ((1, 3, 4 << 20), (1, 3, (4 << 20) - 8), (3, 2, 8000), (2, 3, (4 << 20) + 8), (1, 3, 8 << 20)):
         srcs = [rng.integers(0, 256, size=n, dtype=np.uint8) for _ in range(k)]
         coeffs = _coeffs(k * m, rng)
         ovr = k != 2
