@@ -533,9 +533,9 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // CTA with 227 KiB of tables waits for a whole SM to drain, which a mixed
   // submission's dozens of small classes did one after the other (256 mixed
   // stripes, with the order of items and launches below: 1505 -> 1463 us). One call
-  // crosses over between 4 MiB rows (K = 10: 17.3 us by table kernel, 19.1 by byte
-  // tables) and 16 MiB (54.7, 47.7). A class that is alone, a plan per stripe and
-  // rows at the sources' offset, has nothing to wait for: up to 10 sources the byte
+  // of K = 10 is level at 4 MiB rows and 16 % faster by byte tables at 8 MiB (tune.cpp).
+  // A class that is alone, a plan per stripe and rows at the sources' offset, has
+  // nothing to wait for: up to 10 sources the byte
   // tables win from about 2 MiB of row length on (32 stripes, 4 rows, waited for,
   // table kernels / byte tables, us: 4 MiB of K = 2 30.0 / 27.6, K = 6 38.3 / 35.0, K =
   // 10 40.8 / 37.2, K = 14 45.1 / 46.3; 64 stripes of 16 KiB, K = 10, 37.1 / 41.3, 8
@@ -619,8 +619,8 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
       c.cost = static_cast<double>(total) * c.shape.nv * c.shape.w * (16 / c.E);
       const uint64_t slots = 2 * static_cast<uint64_t>(sm_count() * c.kern.ctas);
       // Stripes of one plan and of the byte tables' shape: one launch per
-      // kUniformJobs stripes, so that such a submission counts the same launches
-      // whatever its size and alignment.
+      // kUniformJobs stripes, as the uniform kernel needs. The work list does not;
+      // such a submission counts the same launches whatever its size and alignment.
       bool one_plan = jobs[c.jobs[0]].byte_tab != nullptr;
       for (uint32_t i : c.jobs) one_plan = one_plan && jobs[i].byte_tab == jobs[c.jobs[0]].byte_tab;
       for (size_t q = 0; q < c.jobs.size(); ++q) {
@@ -1121,7 +1121,7 @@ int noalloc_run(int field, const fgfc_noalloc_job* jobs, size_t njobs, cudaStrea
   const int R = 4 / E;
 
   // ---- sizes: per class its items; every stripe's tables at its own G
-  constexpr int kClasses = 105;  // byte-table 1..14, nibble 101..104
+  constexpr int kClasses = 105;  // byte tables 1..14, table kernels 101..104
   size_t nptr = 0, ntab = 0, nlive = 0;
   size_t class_items[kClasses] = {0};
   for (size_t i = 0; i < njobs; ++i) {

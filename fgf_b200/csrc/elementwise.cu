@@ -9,8 +9,9 @@
 // to 16, transposes included. 1-byte fields run at HBM's rate, the others are
 // bound by the ALU pipe (HBM's time is worth about 8 operations per byte). us on B200, 64 MiB
 // vectors, shift-and-mask (Fan-Paar: log tables) -> planes:
-//   Gf8D 44.6 -> 33.6   Gf16 77.2 -> 40.6   Gf32 185 -> 56   Gf64 322 -> 86
-//   FP8  149 -> 35      FP16 129 -> 43      FP32 168 -> 65   FP64 246 -> 99
+//   Gf8D 44.6 -> 32.7   Gf16 77.2 -> 40.4   Gf32 185 -> 54   Gf64 322 -> 85
+//   FP8  149 -> 35      FP16 129 -> 44      FP32 168 -> 66   FP64 246 -> 97
+// (FP64 holds more planes than registers: 256 bytes a thread go through local memory.)
 //
 // The order of elements within a transposed block does not matter as long as
 // all three vectors use the same, so a thread's words are whichever 16-byte

@@ -222,8 +222,7 @@ inline uint64_t gf_inv(int f, uint64_t a) {
 // GF(2) in every field here. img[p][b] is c times the element whose only set
 // bit is bit b of byte p (an E-byte value), so that for an input element x,
 // byte o of c * x = XOR over the set bits (p, b) of x of byte o of img[p][b].
-// Every table the kernels use (nibble and byte tables, GF(2) bit matrices)
-// is derived from these images, for any field.
+// The GF(2) bit matrices are derived from these images, for any field.
 inline void coeff_images(int f, uint64_t c, uint64_t img[8][8]) {
   const int E = field_bytes(f);
   for (int p = 0; p < 8; ++p)

@@ -198,7 +198,7 @@ int sm_count();
 // Kernel families (fgfc_kernel values) and the choice per shape (tune.cpp).
 bool kernel_usable(int kernel, int field, size_t k, size_t m);
 int choose_kernel(int field, size_t k, size_t m, size_t len);
-// Tile shape of the batched nibble work lists (tune.cpp): element-vector
+// Tile shape of the batched table work lists (tune.cpp): element-vector
 // columns per thread per work item for the class of element width E and G
 // table groups; set_tile_cols(E, G, 0) restores the built-in value.
 constexpr int kTileColsDefault = 8;
@@ -266,7 +266,7 @@ struct Gf2Job {
 void* batch_state_create();
 void batch_state_destroy(void* state);
 void batch_state_graphs(void* state, bool on);
-// The nibble work-list classes (element width, table groups) of the state's
+// The table work-list classes (element width, table groups) of the state's
 // last submission.
 std::vector<std::pair<int, int>> batch_state_classes(const void* state);
 void batch_state_stats(const void* state, size_t* launches, size_t* items, int* replayed);

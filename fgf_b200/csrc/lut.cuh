@@ -8,8 +8,8 @@
 // served by one broadcast, so a warp's 32 lookups never conflict whatever the
 // data, with a single 128-byte copy of the table. Five index bits per lookup
 // is therefore the widest conflict-free table: one bit more doubles the
-// wavefronts, and copies per lane (32 x 128 bytes per nibble pair) were what
-// held the older kernels to one CTA per SM and a 1.5 us fill. Three sources
+// wavefronts, and copies per lane (32 x 128 bytes per nibble pair) hold a kernel
+// to one CTA per SM and a 1.5 us fill. Three sources
 // are folded together: 24 bits of one byte position of three sources take five
 // lookups (each byte's low 5 bits, then the 3 + 2 and 1 + 3 bits left over)
 // where nibble tables take six.
@@ -22,17 +22,18 @@
 //   Fan-Paar   (X^2 = alpha X + 1):   lo = A + B,      hi = A + C + B + alpha B.
 // With LEV levels the leaves are H = E >> LEV bytes wide and a table word holds
 // the leaf products of 4 / H rows. More levels mean fewer lookups per row but
-// need enough rows to fill the word, which is the rule of lut_shape().
+// need enough rows to fill the word and enough sources to carry the fix-up, which
+// is the rule of lut_shape(). Short rows of 8-byte elements run wide.cu.
 //
 // What bounds it: the lookups (one shared-memory wavefront each) and, with one
 // word per product, the issue slots of the operations around them (address dot
-// product, XOR, index masks). Measured on B200 against the kernels it replaced, with 32
-// table copies per lane (or unreplicated nibbles for 8-byte elements):
+// product, XOR, index masks). Measured on B200 against 16-word tables with 32 copies
+// per lane (or unreplicated for 8-byte elements):
 //   GF(2^64) RS(10,4), 16 MiB shards     308 -> 173 us (lookups per element 992 -> 459)
 //   256 stripes of Gf8D and Gf16, k 4..32, m 1..8, 4 KiB .. 4 MiB, one batch
 //                                        3240 -> 1320 us (more CTAs resident, no 216 KiB refills)
-//   Gf8D RS(12,4), consecutive shards of 1000003 bytes: 24.1 -> 7.7 us (single
-//   bytes before, 16-byte granules spliced now)
+//   Gf8D RS(12,4), consecutive shards of 1000003 bytes: 24.1 -> 7.7 us (by single
+//   bytes, by spliced 16-byte granules)
 #pragma once
 #include <cuda_runtime.h>
 
@@ -58,7 +59,7 @@ struct Lut {
   // Index shifts on the multiply pipe: GF(2^64) RS(10,4), 16 MiB, 204 -> 173 us;
   // level or worse for the other widths.
   static constexpr bool kMulShift = E == 8;
-  static constexpr bool kDirect = LEV == 0 && E > 1;
+  static constexpr bool kDirect = LEV == 0 && E > 1;  // no split
 
   // element and leaf byte (product * H + byte) of byte b of packed word w;
   // elem() < 0: no byte there
@@ -664,7 +665,7 @@ __device__ __forceinline__ uint64_t lut_edge(const LutGeom& g, int mode, uint32_
 
 // The edge columns of a job, by one CTA: a thread stages a source's column with
 // 16 independent byte loads, one thread folds a column, a thread writes a
-// row's column. `stage` holds (kMaxSrc + kLutRows) * kEdges * 16 bytes.
+// row's column. `stage` holds (g.k + kLutRows) * kEdges * 16 bytes.
 template <class L, int LEV, int W, int MODE>
 __device__ __forceinline__ void lut_edges(const LutGeom& g, const LutShared& sh, uint8_t* stage, bool ovr, bool fp) {
   constexpr int R = 4 / L::H;

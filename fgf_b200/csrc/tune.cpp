@@ -47,7 +47,7 @@ struct TuneVal {
 
 std::map<TuneKey, TuneVal> g_table;
 
-// Tile shape of the batched nibble work lists: element-vector columns per
+// Tile shape of the batched table work lists: element-vector columns per
 // thread per work item, by (element width, table groups); 0 = built-in.
 // FGFC_TILE_COLS=n in the environment (read once) overrides every class.
 struct TileVal {
@@ -100,12 +100,15 @@ int forced_locked() {
 }
 
 // Built-in rules. Byte tables for their shapes once a row is long enough to
-// amortise their 1.5 us fill. The tensor-core contraction is not chosen: at
+// amortise their 1.5 us fill: level with the table kernels at 4 MiB, ahead from
+// 8 MiB on (4 rows, us, table kernels / byte tables, 2, 4, 8, 16 MiB: K = 2 5.4 / 5.4,
+// 6.9 / 6.6, 11.0 / 9.7, 18.8 / 15.3; K = 10 10.2 / 10.2, 16.3 / 16.1, 29.7 / 24.9, 51.8
+// / 44.1; K = 14 12.1 / 12.3, 20.7 / 20.5, 38.6 / 40.2, 68.8 / 68.6). The tensor-core contraction is not chosen: at
 // the shapes that suit it best (16 output bytes per column, 64 input bytes)
 // the 32-word tables take, on B200 and device time,
-//   Gf16 RS(32,8), 16 MiB rows   361 us against 522
-//   Gf32 RS(16,4),  8 MiB rows    91 us against 149
-//   Gf8B RS(64,16), 4 MiB rows   249 us against 321
+//   Gf16 RS(32,8), 16 MiB rows   341 us against 522
+//   Gf32 RS(16,4),  8 MiB rows    81 us against 149
+//   Gf8B RS(64,16), 4 MiB rows   252 us against 321
 // and the gap widens as columns carry fewer bytes (Gf8D RS(20,8): 46 against
 // 176). It stays for callers that force it or measure their own shapes.
 int builtin_choice(int field, size_t k, size_t m, size_t len) {
