@@ -420,6 +420,7 @@ static cudaError_t ensure_slot(BatchSlot& s, size_t bytes) {
   if (s.dev) cudaFree(s.dev);
   s.host = nullptr;
   s.dev = nullptr;
+  s.cap = 0;  // until both are there
   if (s.graph) {
     cudaGraphExecDestroy(s.graph);
     s.graph = nullptr;
@@ -431,9 +432,12 @@ static cudaError_t ensure_slot(BatchSlot& s, size_t bytes) {
   if (e != cudaSuccess) return e;
   e = cudaMalloc(&s.dev, cap);
   if (e != cudaSuccess) return e;
+  if (!s.up) {
+    e = cudaEventCreateWithFlags(&s.up, cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+  }
   if (!s.done) {
     e = cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.up, cudaEventDisableTiming);
     if (e != cudaSuccess) return e;
   }
   s.cap = cap;
@@ -535,11 +539,10 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // stripes, with the order of items and launches below: 1505 -> 1463 us). One call
   // of K = 10 is level at 4 MiB rows and 16 % faster by byte tables at 8 MiB (tune.cpp).
   // A class that is alone, a plan per stripe and rows at the sources' offset, has
-  // nothing to wait for: up to 10 sources the byte
-  // tables win from about 2 MiB of row length on (32 stripes, 4 rows, waited for,
-  // table kernels / byte tables, us: 4 MiB of K = 2 30.0 / 27.6, K = 6 38.3 / 35.0, K =
-  // 10 40.8 / 37.2, K = 14 45.1 / 46.3; 64 stripes of 16 KiB, K = 10, 37.1 / 41.3, 8
-  // of 4 KiB, K = 4, 20.1 / 29.1).
+  // nothing to wait for: up to 10 sources the byte tables win from about 2 MiB of
+  // row length on (32 stripes, 4 rows, waited for, table kernels / byte tables, us:
+  // 4 MiB of K = 2 30.0 / 27.6, K = 6 38.3 / 35.0, K = 10 40.8 / 37.2, K = 14 45.1 /
+  // 46.3; 64 stripes of 16 KiB, K = 10, 37.1 / 41.3, 8 of 4 KiB, K = 4, 20.1 / 29.1).
   constexpr uint64_t kByteClassCols = 8u << 16, kLoneClassCols = 2u << 16;
   std::map<size_t, uint64_t> byte_cols;
   for (size_t i = 0; i < jobs.size(); ++i)
@@ -936,8 +939,7 @@ cudaError_t batch_run(void* state, const std::vector<LoweredJob>& jobs, const st
   // of 2 x 2 rows of 4 KiB 33.8 / 27.2, Gf16 (10,4) of 16 KiB 30.6 / 31.4 and 64 / 55
   // alone, 32 Gf8D (10,4) of 64 KiB 17.5 / 25.9, 7 Gf8B (11,3) of 44 KiB 12.3 / 16.9.
   // The line is where 8 us and 0.2 us a sub-job pass 13 us and the time of the bytes
-  // at 1.8 TB/s. Launches that carry everything in
-  // their parameters need no blob.
+  // at 1.8 TB/s. Launches that carry everything in their parameters need no blob.
   bool blob = false;
   for (const Launch& L : launches) blob = blob || !L.ufn;
   uint64_t moved = 0;

@@ -12,10 +12,10 @@
 // banks); the fix-up takes 8 more per row. A thread has one element, half of a
 // table kernel's column, up to 8 rows in one launch, and no more code than one
 // source's, so where a thread gets one column anyway (short rows) or the fix-up
-// outweighs the lookups (few sources) it ends first. Latency bounds the former,
-// the lookups the latter. us on B200, table kernels -> this one, GF(2^64): 64 KiB of k = 4, m = 3
-// 11.6 -> 7.8, m = 6 21.9 -> 10.4; 300000 bytes at odd addresses, k = 10, m = 4 28.7
-// -> 14.6; 16 MiB of k = 1, m = 4 59.1 -> 42.1.
+// outweighs the lookups (few sources) it ends first. Latency bounds the former, the
+// lookups the latter. us on B200, table kernels -> this one, GF(2^64): 64 KiB of
+// k = 4, m = 3 11.6 -> 7.8, m = 6 21.9 -> 10.4; 300000 bytes at odd addresses,
+// k = 10, m = 4 28.7 -> 14.6; 16 MiB of k = 1, m = 4 59.1 -> 42.1.
 #include <cuda_runtime.h>
 
 #include <algorithm>
